@@ -92,7 +92,8 @@ __device__ __forceinline__ float reduce_2pi_f(float x) {
 // Device copies of the interpolation kernels (tops_lut_dev).
 struct LutPtrs {
   const float *kaz, *krg;  // [2048][12]
-  const float4 *krg2;      // [2048][6]: range taps duplicated (w0,w0,w1,w1), ...
+  const float4 *kaz2;      // [2048][6]: azimuth taps duplicated (w0,w0,w1,w1), ...
+  const float4 *krgo;      // [2048][4]: range taps one sample later: 0, w0 .. w11, 0, 0, 0
   const float *sp1;        // [2048]: sum(krg row) - 1
 };
 

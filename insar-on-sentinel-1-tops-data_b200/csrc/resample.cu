@@ -13,59 +13,59 @@
 //             sum of the deramp phase phi.
 //
 // B200 design (no textures, no phase array in HBM).  A CTA of 128 threads
-// owns a strip of RS_TW = 112 output columns and a segment of up to 252
-// output rows (a work item), swept in groups of RS_GR = 12 rows.
+// owns two adjacent strips of RS_TW = 112 output columns, 64 threads and a
+// ring of 128 slave columns (two per thread) each, and a segment of up to 252
+// output rows (a work item).  The rows are prepared in chunks and computed in
+// halves of 6 rows:
 //
-// Item prologue (all threads): per-row statistics from the offset
-// polynomials -- along the strip y is a quadratic in the column, so a row
-// whose whole strip maps to one (azimuth line, LUT bin) key (nearly every
-// row of a TOPS pair) gets one shared azimuth pass -- with the row's FP64
-// phase terms; per output column the runs of its range key (p0, bin) over
-// the item, found by bisection of the exact per-pixel position (keys change
-// every ~100+ rows), each run with its range weights' phase moments.
+// Chunk prologue.  Row keys: per row and strip, the runs of equal azimuth key
+// (L0, bin) along the strip, found by bisection of the exact per-pixel key on
+// monotone pieces; each run is an "entry" (its columns, its reramp terms).
+// Nearly parallel orbits give one entry per row, crossing orbits a few.
+// Column keys: thread per column pair, the runs of the range key over the
+// chunk's rows, each with its residual phase terms.  A chunk is as many rows
+// (up to 120) as the entry and run tables hold.
 //
-// Per group:
-//   [A] azimuth pass, thread = ring column (RS_FW = 128 slave columns): the
-//       thread's raw slave lines were staged in shared memory with cp.async
-//       during the previous group; each new line is deramped in registers
-//       and pushed into a 12-line register window (the window's slots rotate
-//       with the row index, so a steady row costs one deramp and no moves);
-//       v = sum_j kAz[j] d(L0-5+j) is 12 packed FP32x2 FMAs, written to the
-//       group's 12 x 128 tile; then the next group's raw lines are staged,
-//       so their copies land while [B] runs.
-//   [B] range pass, thread = 2 adjacent output columns x 6 rows: the 14
-//       tile samples of the pair are 7 16-byte loads, the 12 range weights
-//       of each column stay in registers for its key run, and the reramp
-//       phase is a dot product of row terms and column-run terms (below).
-// A barrier separates [A] and [B]; the deferred passes [C1] (columns
-// without run tables), [C2] (the second bin of two-bin rows) and [C] (the
-// per-pixel path) follow [B] when the group has such pixels.
+// Half of 6 rows.
+//   [A] azimuth pass, thread = 2 adjacent ring columns: six new slave lines
+//       (staged with cp.async while earlier halves ran) are deramped in
+//       registers and pushed into a 12-line register window whose slots
+//       rotate statically; after each push the entries whose line is the
+//       window's are summed, v = sum_j kAz[j] d(L0-5+j), with FP32x2 FMAs
+//       over the two columns, into the tile: 16-byte units (re, re', im, im')
+//       of two columns.  An entry covers only the ring columns its output
+//       columns need, so a row of several entries costs little more than one.
+//   [B] range pass, thread = 2 adjacent output columns: 7 tile units; one
+//       column's 12 taps start at a unit boundary, the other's one sample
+//       later, so it takes 7 units with taps shifted by one (0, w0 .. w11, 0).
+//       An FP32x2 FMA multiplies two taps with the two samples of a unit.
+// Halves 2k and 2k + 1 share one tile and one [B] when their entries fit.
 //
 // The phase.  The reference reramps with the 144-tap FP64 sum
 // Phi = sum_j sum_i kAz[j] kRg[i] phi(y_j, x_i).  With phi = phi_ref(y) +
-// G(y, x), phi_ref the deramp phase of one reference column and G exactly
-// quadratic in the burst-local time tc (G = g2 tc^2 + g1 tc + g0 per
+// G(y, x), phi_ref the deramp phase of the strip's reference column and G
+// exactly quadratic in the burst-local time tc (G = g2 tc^2 + g1 tc + g0 per
 // column), Phi = (1 + sp) Psi + G2 R2 + G1 R1 + G0 R0, with
-//   Psi = sum_j kAz[j] phi_ref(y_j)                   (row, FP64, reduced)
+//   Psi = sum_j kAz[j] phi_ref(y_j)                   (entry, FP64, reduced)
 //   sp  = sum_i kRg[i] - 1, Gk = sum_i kRg[i] gk(x_i)  (column key run)
 //   R2 = M0 tc0^2 + 2 tc0 dt M1 + dt^2 M2, R1 = M0 tc0 + dt M1, R0 = M0
-//        (row; M0..M2 the azimuth taps' moments, tc0 = tc(L0)),
+//        (entry; M0..M2 the azimuth taps' moments, tc0 = tc(L0)),
 // equal to the reference's sum in exact arithmetic.
 //
-// Every row whose strip maps to one azimuth key takes the shared pass: from
-// the register window when its line is the window's, else (the row-to-line
-// map skipped a line inside a group) by the same 12-line sum over lines
-// deramped anew.  A row whose strip spans two adjacent bins of one line
-// takes it for the first bin; the second bin's sums follow the range pass
-// over the freed tile rows, and its columns (found by bisection in the
-// prologue) go through the keyed path.  A column with more than RS_MAXRUN
-// key runs in the item finds each pixel's key and run terms with the
-// functions that build the run tables.  Rows with more azimuth keys, and
-// pixels whose range support leaves the ring window, take a per-pixel path
-// that computes the reference's formula from the slave in HBM; edge and
-// outside pixels take the nearest sample and 0.  Which path a pixel takes depends on its row,
-// its column and its strip only, never on the work item, so a job that
-// produces a subset of the rows gives those rows bit for bit.
+// What bounds it: instruction issue with 12 warps per SM (168 registers and 72
+// KB of shared memory per CTA allow 3 CTAs).  Two columns per thread share a
+// line's terms, a row's taps and the bookkeeping, and fill the FP32x2 lanes:
+// 105 instead of 158 thread instructions per pixel on a burst of 1500 x 21000
+// (one entry per row, nearly no key changes), 0.463 -> 0.351 ms (816 -> 1077
+// GB/s of 12 bytes per pixel).  Rows whose strip spans several azimuth keys
+// took a per-pixel path from HBM before, columns with many range keys a keyed
+// one: a burst of 1539 x 10867 of crossing orbits 3.92 -> 0.87 ms.
+//
+// Which path a pixel takes, and the order of its sums, depend on its row, its
+// column and its strip only, never on the work item, so a job that produces a
+// subset of the rows gives those rows bit for bit.  Rows with more than
+// RS_MAXKEY azimuth runs in the strip and pixels whose range support leaves
+// the ring take the per-pixel path from HBM.
 //
 // Precision modes: TOPS_PREC_SPLIT (default) forms each sample's deramp
 // phase in FP32 as rho(y) + G(y, x), rho the FP64 reference phase reduced
@@ -76,8 +76,10 @@
 // formed in turns in both modes.  Positions, LUT bins and Psi are FP64 in
 // both.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -86,27 +88,33 @@
 namespace tops {
 
 constexpr int RS_NT = 128;                 // threads per CTA
+constexpr int RS_NS = 2;                   // strips per CTA
+constexpr int RS_ST = RS_NT / RS_NS;       // threads per strip
 constexpr int RS_TW = 112;                 // output columns per strip
 constexpr int RS_FW = 128;                 // ring (slave) columns of a strip
-constexpr int RS_GR = 12;                  // rows per group (= azimuth taps)
-constexpr int RS_HR = RS_GR / 2;           // rows per range-pass thread
-constexpr int RS_SEG = 252;                // default rows per work item
-constexpr int RS_MAXSEG = 252;             // per-item tables are sized for this
-constexpr int RS_NGRP = (RS_MAXSEG + RS_GR - 1) / RS_GR;
-constexpr int RS_SR = 32;                  // staged slave lines (power of two)
-constexpr int RS_NSR = RS_MAXSEG + 44;     // slave-line phase table
-constexpr int RS_MAXRUN = 6;               // range-key runs per column and item
-constexpr int RS_MAXBIN = 16;              // distinct azimuth bins per item
-constexpr int RS_NOSLOT = 0x7fff;          // azimuth bin outside the bin table
+constexpr int RS_UN = RS_FW / 2;           // 2-column units of a ring
+constexpr int RS_DT = RS_TW / 2;           // range-pass threads per strip
+constexpr int RS_H = 6;                    // rows (and pushed lines) per half
+constexpr int RS_MAXSEG = 252;             // longest work item
+constexpr int RS_CH = 120;                 // rows per chunk
+constexpr int RS_NH = RS_CH / RS_H;        // halves per chunk
+constexpr int RS_ECAP = 136;               // entries per chunk and strip
+constexpr int RS_TU = 2 * RS_H * RS_UN;    // tile units per strip
+constexpr int RS_ROWU = RS_TU / RS_H;      // most tile units of a row
+constexpr int RS_MAXKEY = 16;              // most entries of a row
 constexpr int RS_MAXJOBS = 32;
-constexpr int RS_DP = RS_TW / 2;           // column pairs of the range pass
-constexpr int RS_DT = 2 * RS_DP;           // range-pass threads
-static_assert(RS_FW == RS_NT, "one ring column per thread in the azimuth pass");
-static_assert(RS_DT <= RS_NT && RS_GR == 12 && RS_HR * 2 == RS_GR,
-              "thread mappings assume these sizes");
+static_assert(RS_UN == RS_ST, "one unit per thread in the azimuth pass");
+static_assert(RS_DT <= RS_ST && RS_CH <= 2 * RS_ST && RS_CH % (2 * RS_H) == 0 &&
+                  RS_MAXKEY <= RS_ECAP && RS_TW < 128 && RS_NH <= RS_ST,
+              "thread mappings and table fields assume these sizes");
 
 enum : int { REG_OUT = 0, REG_EDGE = 1, REG_IN = 2 };
-enum : int { RM_PIXEL = 0, RM_SHARED = 1, RM_TWO = 2 };
+// A half: has interior entries; fills its window anew; has entries off its
+// window; shares its tile with the next half; has per-pixel rows; every row is
+// one interior entry; and, besides, 6 rows with the window's lines and one bin.
+enum : int { HG_ON = 1, HG_FILL = 2, HG_DIRECT = 4, HG_JOIN = 8, HG_PIX = 16, HG_ONE = 32,
+             HG_PLAIN = 64 };
+constexpr int E_DIRECT = 4;                // entry flag beside its region
 
 using RsLut = LutPtrs;
 
@@ -117,20 +125,17 @@ struct RsBatch {
   ResampleJob jobs[RS_MAXJOBS];
 };
 
-// One output row of a work item.
-struct __align__(16) RsRow {
-  float rho, psif, R2, R1;   // Psi mod 2 pi, Psi as float, residual-phase row terms
-  float R0;
-  int L0;                    // azimuth line of the shared azimuth pass
-  int bin;                   // its LUT bin | bin-table slot << 16
-  int mode;                  // RM_SHARED: the row takes the shared azimuth pass;
-                             // RM_TWO | lo << 8 | hi << 16: the same, but columns
-                             // [lo, hi) have the next LUT bin of the same line;
-                             // RM_PIXEL: its pixels take the per-pixel path
+// One half of a strip: 6 rows and the 6 lines its window pushes.
+struct __align__(16) RsHalf {
+  int lb;                  // line of the first row's window
+  int flags;
+  int tbase;               // first tile unit
+  int units;
+  short pos[8];            // entries of window position q - 1: [pos[q], pos[q + 1])
 };
 
 // Deramp terms of one slave line: the burst-local azimuth time (FP64
-// mode), or the reference-column phase mod 2 pi and ta - tm (split mode).
+// mode), or the reference-column phase in turns and ta - tm (split mode).
 union RsSlaveRow {
   double ta;
   struct {
@@ -138,48 +143,67 @@ union RsSlaveRow {
   } f;
 };
 
-struct __align__(16) RsShared {
-  float2 vd[RS_GR][RS_FW];            // azimuth-interpolated rows of the group
-  short2 stage[RS_SR][RS_FW];         // raw slave lines, ring indexed by line & 31
-  RsRow rows[RS_MAXSEG];
-  RsSlaveRow srow[RS_NSR];            // slave lines ys0 .. ys0 + RS_NSR - 1
-  float4 run_g[RS_TW][RS_MAXRUN];     // per range-key run: (sp, G2, G1, G0)
-  int2 run_rk[RS_TW][RS_MAXRUN];      // (first item row, key = p0 * 4096 + bin)
-  int run_n[RS_TW];                   // runs of the column (-1: more than RS_MAXRUN)
+// FP64 deramp quadratics of the ring columns (FP64 mode).
+template <bool kSplit>
+struct RsRing {
+  double2 a21[RS_FW];
+  double a0[RS_FW];
+};
+template <>
+struct RsRing<true> {};
+
+template <bool kSplit>
+struct __align__(16) RsStrip {
+  static constexpr int kRuns = kSplit ? 3 : 2;   // range-key runs per column and chunk
+  float4 tile[RS_TU];                 // azimuth-interpolated units
+  float4 run_g[kRuns][RS_TW];         // per run: (sp, G2, G1, G0)
+  int2 run_rk[kRuns][RS_TW];          // (first chunk row, key = p0 * 4096 + bin)
   float4 ring_gc[RS_FW];              // per ring column (g2, g1, g0, 0)
-  float4 bin_w[RS_MAXBIN][6];         // azimuth taps as (w0,w0,w1,w1), ...
-  int bin_id[RS_MAXBIN];
-  alignas(16) double col_phat[RS_TW];
-  double col_qaz[RS_TW], col_qrg[RS_TW];
-  int4 gplan[RS_NGRP];                // per group: lines to stage before it, staged window
-  int4 gwin[RS_NGRP];                 // per group: window on, filled at its start, line of row 0,
-                                      // rows without a shared azimuth pass (bit mask)
-  int2 grange[RS_NGRP];               // per group: lines its window pushes need
-  RsRow r2[RS_GR];                    // row terms of the second bin of the group's two-bin rows
-  int gen_n[RS_NGRP];                 // per group: pixels deferred to the per-pixel pass
-  int gen_d[RS_NGRP];                 // per group: pixels of columns without a run table
-  unsigned short gen[RS_GR * RS_TW];  // their (row in group) * 128 + column: the first
-                                      // from the bottom, the second from the top
-  int scan[RS_NT / 32];               // per-warp totals of the bin-change scan
-  double caz[6], crg[6], shift;
-  double ref_a0, ref_a1, ref_a2, tm;
-  int xw, ys0, nbins, ngrp, next_item;
+  float4 eA[RS_ECAP];                 // entries: reramp terms (rho, psif, R2, R1)
+  int4 eM[RS_ECAP];                   // (L0, bin | region << 12 | c_lo << 16 | c_hi << 24, R0,
+                                      //  (tile offset & 0xffff) | first unit << 16 | last unit << 24)
+  RsHalf half[RS_NH];
+  RsSlaveRow srow[RS_NH * RS_H];      // the lines the halves push
+  int rowe[RS_CH];                    // first entry | entries << 16 (0 entries: per-pixel row)
+  unsigned gen[2 * RS_H][4];          // pixels of the tile's rows left to the per-pixel path
+  unsigned missb[RS_ST / 32];         // pairs with rows the pair path left, and the rows
+  unsigned short miss[RS_ST];
+  unsigned char run_n[RS_TW];
+  int scan[RS_ST / 32];
+  RsRing<kSplit> ring;
+  double ref_a0, ref_a1, ref_a2, tm;  // reference column's phase, burst centre time
+  int xo, dlo, dhi;                   // ring origin, bounds of (ring column - strip column)
+  int nfit, cov, gen_any, prev_line;
 };
 
-// Asynchronous 4-byte global -> shared copy; src_bytes 0 fills zeros.
+template <bool kSplit>
+struct __align__(16) RsShared {
+  RsStrip<kSplit> strip[RS_NS];
+  uint2 stage[2 * RS_H][RS_NT];       // raw slave lines of the next two halves
+  double caz[6], crg[6], shift;
+  int next_item;
+};
+
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return static_cast<unsigned>(__cvta_generic_to_shared(p));
 }
-__device__ __forceinline__ void cp_async_4s(unsigned d, const void *src, int src_bytes) {
+// Asynchronous global -> shared copies; src_bytes 0 fills zeros.
+__device__ __forceinline__ void cp_async_4(unsigned d, const void *src, int src_bytes) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(src),
+               "r"(src_bytes)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_8(unsigned d, const void *src, int src_bytes) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(d), "l"(src),
                "r"(src_bytes)
                : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() {
   asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 // Deramp + demodulation phase (DerampAndResample.cu:151-158), FP64, as the
@@ -213,11 +237,24 @@ __device__ __forceinline__ float to_turns(double phi) {
   const double u = phi * kInvTwoPi;
   return (float)(u - rint(u));
 }
+// Two phases in turns as reduced phases in radians; t - rint(t) by packed
+// adds of 3 2^22, which rounds |t| < 2^22 to the nearest integer as rint does.
+__device__ __forceinline__ float2 turns_to_rad2(float2 t) {
+  const float2 big = make_float2(12582912.f, 12582912.f);
+  const float2 nbig = make_float2(-12582912.f, -12582912.f);
+  const float2 m1 = make_float2(-1.f, -1.f);
+  const float2 r = __fadd2_rn(__fadd2_rn(t, big), nbig);
+  return __fmul2_rn(__ffma2_rn(r, m1, t), make_float2(kTwoPiF, kTwoPiF));
+}
+// a exp(-i f)
+__device__ __forceinline__ float2 cmul_conj(float2 a, float f) {
+  float s, c;
+  __sincosf(f, &s, &c);
+  return make_float2(a.x * c + a.y * s, a.y * c - a.x * s);
+}
 // a * exp(-i 2 pi t), t in turns
 __device__ __forceinline__ float2 cmul_conj_turns(float2 a, float t) {
-  float s, c;
-  __sincosf(turns_reduce(t) * kTwoPiF, &s, &c);
-  return make_float2(a.x * c + a.y * s, a.y * c - a.x * s);
+  return cmul_conj(a, turns_reduce(t) * kTwoPiF);
 }
 
 // Integer index and LUT bin of a position (GetIndexes, DerampAndResample.cu:
@@ -229,10 +266,9 @@ __device__ __forceinline__ void split_pos(double v, int &i0, int &bin) {
   bin = min(max(b, 0), kLutBins - 1);
 }
 
-__device__ __forceinline__ int region_of(const ResampleJob &J, int l0, int p0) {
-  if (l0 > J.sy1 || l0 < J.sy0 || p0 > J.sx1 || p0 < J.sx0) return REG_OUT;
-  if (l0 > J.sy1 - 7 || l0 < J.sy0 + 5 || p0 > J.sx1 - 7 || p0 < J.sx0 + 5) return REG_EDGE;
-  return REG_IN;
+__device__ __forceinline__ int region_1d(int v, int lo, int hi) {
+  if (v > hi || v < lo) return REG_OUT;
+  return (v > hi - 7 || v < lo + 5) ? REG_EDGE : REG_IN;
 }
 
 // my_polyval grouped by row: position = fma(B(row), P^, A(row) + c5 P^2)
@@ -241,28 +277,29 @@ __device__ __forceinline__ int region_of(const ResampleJob &J, int l0, int p0) {
 __device__ __forceinline__ double row_L(const ResampleJob &J, int r) {
   return ((double)(r + J.my0) - J.midL) * J.invL;
 }
+__device__ __forceinline__ double col_P(const ResampleJob &J, int c) {
+  return ((double)c - J.midP) * J.invP;
+}
 __device__ __forceinline__ double row_a(const double *c, double L) {
   return fma(fma(c[3], L, c[1]), L, c[0]);
 }
 __device__ __forceinline__ double row_b(const double *c, double L) { return fma(c[4], L, c[2]); }
-__device__ __forceinline__ double pix_pos(double A, double B, double P, double Q) {
-  return fma(B, P, A + Q);
+__device__ __forceinline__ double pix_pos(double A, double B, double c5, double P) {
+  return fma(B, P, __dadd_rn(A, __dmul_rn(__dmul_rn(c5, P), P)));
 }
 
-// Range [lo, hi] of f(p) = fma(b, p, a + c p^2) -- the per-pixel form -- over
-// p in [p0, p1]: the ends and, when inside, the vertex.  Widened by 1e-9 so
-// that rounding of the per-pixel evaluation cannot leave it.
+// Range [lo, hi] of the position over P in [p0, p1]: the ends and, when
+// inside, the vertex.  Widened by 1e-9 so that rounding of the per-pixel
+// evaluation cannot leave it.
 __device__ __forceinline__ void quad_span(double a, double b, double c, double p0, double p1,
                                           double &lo, double &hi) {
-  const double f0 = fma(b, p0, a + c * p0 * p0);
-  const double f1 = fma(b, p1, a + c * p1 * p1);
+  const double f0 = pix_pos(a, b, c, p0), f1 = pix_pos(a, b, c, p1);
   lo = fmin(f0, f1);
   hi = fmax(f0, f1);
   // the vertex lies inside only if the slope changes sign over [p0, p1]
   const double s0 = fma(2.0 * c, p0, b), s1 = fma(2.0 * c, p1, b);
   if ((s0 < 0.0) != (s1 < 0.0)) {
-    const double pv = -b / (2.0 * c);
-    const double fv = fma(b, pv, a + c * pv * pv);
+    const double fv = pix_pos(a, b, c, -b / (2.0 * c));
     lo = fmin(lo, fv);
     hi = fmax(hi, fv);
   }
@@ -270,22 +307,21 @@ __device__ __forceinline__ void quad_span(double a, double b, double c, double p
   hi += 1e-9;
 }
 
-// Range key (p0 * 4096 + bin) of pixel (box row r, strip column c).
-__device__ __forceinline__ int rg_key(const RsShared &S, const ResampleJob &J, int r, int c) {
+// Range key (p0 * 4096 + bin) of pixel (box row r, box column c).
+__device__ __forceinline__ int rg_key(const double *crg, const ResampleJob &J, int r, double P) {
   const double L = row_L(J, r);
-  const double x = pix_pos(row_a(S.crg, L), row_b(S.crg, L), S.col_phat[c], S.col_qrg[c]);
   int p0, b;
-  split_pos(x, p0, b);
-  return p0 * 4096 + b;
+  split_pos(pix_pos(row_a(crg, L), row_b(crg, L), crg[5], P), p0, b);
+  return min(max(p0, -(1 << 19)), (1 << 19) - 1) * 4096 + b;
 }
 
 // ---------------------------------------------------- HBM slow path
 // Per-pixel interior resample straight from the CInt16 slave in HBM (rows
 // and pixels the shared passes do not cover).
-__device__ float2 interior_from_global(const ResampleJob &J, const RsLut &lut, int L0, int bL,
-                                       int P0, int bP) {
-  const float *kl = lut.kaz + bL * kTaps;
-  const float *kp = lut.krg + bP * kTaps;
+__device__ __forceinline__ float2 interior_from_global(const ResampleJob &J, int L0, int bL, int P0,
+                                                    int bP) {
+  const float *kl = J.lut.kaz + bL * kTaps;
+  const float *kp = J.lut.krg + bP * kTaps;
   float sre = 0.f, sim = 0.f;
   double ph = 0.0;
 #pragma unroll 1
@@ -316,226 +352,569 @@ __device__ float2 interior_from_global(const ResampleJob &J, const RsLut &lut, i
   return make_float2(sre * c + sim * s, sim * c - sre * s);
 }
 
-// Any pixel (box row r, strip column c) by the per-pixel definition.
-__device__ __forceinline__ float2 pixel_generic(const RsShared &S, const ResampleJob &J, int r,
-                                             int c) {
-  const double L = row_L(J, r);
-  const double P = S.col_phat[c];
-  const double y = pix_pos(row_a(S.caz, L) + S.shift, row_b(S.caz, L), P, S.col_qaz[c]);
-  const double x = pix_pos(row_a(S.crg, L), row_b(S.crg, L), P, S.col_qrg[c]);
+// Any pixel (box row r, box column c) by the per-pixel definition.
+template <bool kSplit>
+__device__ __forceinline__ float2 pixel_generic(const RsShared<kSplit> &S, const ResampleJob &J,
+                                                int r, int c) {
+  const double L = row_L(J, r), P = col_P(J, c);
   int l0, bl, p0, bp;
-  split_pos(y, l0, bl);
-  split_pos(x, p0, bp);
-  const int reg = region_of(J, l0, p0);
+  split_pos(pix_pos(row_a(S.caz, L) + S.shift, row_b(S.caz, L), S.caz[5], P), l0, bl);
+  split_pos(pix_pos(row_a(S.crg, L), row_b(S.crg, L), S.crg[5], P), p0, bp);
+  const int reg = min(region_1d(l0, J.sy0, J.sy1), region_1d(p0, J.sx0, J.sx1));
   if (reg == REG_OUT) return make_float2(0.f, 0.f);
   if (reg == REG_EDGE) {
     const short2 sv = J.slave[(long)(l0 - J.sy0) * J.slave_pitch + (p0 - J.sx0)];
     return make_float2((float)sv.x, (float)sv.y);
   }
-  return interior_from_global(J, J.lut, l0, bl, p0, bp);
+  return interior_from_global(J, l0, bl, p0, bp);
 }
 
-// Range weights and phase terms of one output column's current key run.
-struct ColRun {
-  float4 w[6];    // (w0,w0,w1,w1), (w2,w2,w3,w3), ...
-  float sp, G2, G1, G0;
-  int key;        // p0 * 4096 + bin
-  int next;       // first item row of the next run
-  int m;          // run index
-  bool ok;        // range-interior and inside the ring window: fast range pass
+// The per-pixel rows and the listed pixels of nrows tile rows (chunk rows from
+// cr0, box rows from r0 on), all threads of a strip.
+template <bool kSplit>
+__device__ __forceinline__ void pixel_pass(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
+                                           const ResampleJob &J, int u, int cr0, int r0, int nrows,
+                                           int c0, int cN) {
+  for (int k = 0; k < nrows; k++) {
+    const bool whole = (Q.rowe[cr0 + k] >> 16) == 0;
+    const int r = r0 + k;
+    for (int c = u; c < cN; c += RS_ST)
+      if (whole || ((Q.gen[k][c >> 5] >> (c & 31)) & 1u))
+        J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] = pixel_generic(S, J, r, c0 + c);
+  }
+}
+
+// ---------------------------------------------------- azimuth pass
+// Deramp coefficients of a thread's two ring columns.
+template <bool kSplit>
+struct RingPhase;
+template <>
+struct RingPhase<true> {
+  float2 g2, g1, g0;
+};
+template <>
+struct RingPhase<false> {
+  DerampQuad x, y;
+};
+template <bool kSplit>
+__device__ __forceinline__ RingPhase<kSplit> ring_load(const RsStrip<kSplit> &Q, int u) {
+  if constexpr (kSplit) {
+    const float4 a = Q.ring_gc[2 * u], b = Q.ring_gc[2 * u + 1];
+    return {make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z)};
+  } else {
+    const double2 a = Q.ring.a21[2 * u], b = Q.ring.a21[2 * u + 1];
+    return {DerampQuad{Q.ring.a0[2 * u], a.y, a.x}, DerampQuad{Q.ring.a0[2 * u + 1], b.y, b.x}};
+  }
+}
+// Deramp terms of line y.
+template <bool kSplit>
+__device__ __forceinline__ RsSlaveRow line_terms(const RsStrip<kSplit> &Q, const ResampleJob &J,
+                                                 int y) {
+  const double ta = (double)(y - J.s_first_line) * J.dt;
+  RsSlaveRow sr;
+  if (kSplit) {
+    const DerampQuad refq = {Q.ref_a0, Q.ref_a1, Q.ref_a2};
+    sr.f.rho = to_turns(quad_eval(refq, ta));
+    sr.f.tc = (float)(ta - Q.tm);
+  } else {
+    sr.ta = ta;
+  }
+  return sr;
+}
+
+// Two deramped samples: (re, re') and (im, im').
+struct Dpair {
+  float2 re, im;
+};
+template <bool kSplit>
+__device__ __forceinline__ Dpair deramp_pair(uint2 raw, RsSlaveRow sr,
+                                             const RingPhase<kSplit> &R) {
+  const short2 a = *reinterpret_cast<const short2 *>(&raw.x);
+  const short2 b = *reinterpret_cast<const short2 *>(&raw.y);
+  const float2 sx = make_float2((float)a.x, (float)b.x), sy = make_float2((float)a.y, (float)b.y);
+  float2 f;
+  if constexpr (kSplit) {
+    const float2 tc = make_float2(sr.f.tc, sr.f.tc);
+    const float2 G = __ffma2_rn(__ffma2_rn(R.g2, tc, R.g1), tc, R.g0);
+    f = turns_to_rad2(__fadd2_rn(make_float2(sr.f.rho, sr.f.rho), G));
+  } else {
+    f.x = reduce_2pi(quad_eval(R.x, sr.ta));
+    f.y = reduce_2pi(quad_eval(R.y, sr.ta));
+  }
+  float2 sn, cs;
+  __sincosf(f.x, &sn.x, &cs.x);
+  __sincosf(f.y, &sn.y, &cs.y);
+  Dpair d;
+  d.re = __ffma2_rn(sx, cs, __fmul2_rn(sy, make_float2(-sn.x, -sn.y)));
+  d.im = __ffma2_rn(sx, sn, __fmul2_rn(sy, cs));
+  return d;
+}
+
+// Raw samples of line y in the ring columns xa, xa + 1 (zeros outside the box).
+__device__ __forceinline__ uint2 raw_pair(const ResampleJob &J, int xa, int y) {
+  uint2 v = make_uint2(0u, 0u);
+  if (y < J.sy0 || y > J.sy1) return v;
+  const short2 *p = J.slave + (long)(y - J.sy0) * J.slave_pitch + (xa - J.sx0);
+  if (xa >= J.sx0 && xa <= J.sx1) v.x = *reinterpret_cast<const unsigned *>(p);
+  if (xa + 1 >= J.sx0 && xa + 1 <= J.sx1) v.y = *reinterpret_cast<const unsigned *>(p + 1);
+  return v;
+}
+
+// Stages lines y0 .. y0 + 5 into `slot` .. `slot + 5` (zeros outside the box).
+template <bool kSplit>
+__device__ __forceinline__ void stage_half(RsShared<kSplit> &S, const ResampleJob &J, int t,
+                                           int xa, int slot, int y0) {
+  const unsigned d = smem_u32(&S.stage[slot][t]);
+  constexpr unsigned kRow = RS_NT * sizeof(uint2);
+  const bool in0 = xa >= J.sx0 && xa <= J.sx1, in1 = xa + 1 >= J.sx0 && xa + 1 <= J.sx1;
+  const long off = (long)(y0 - J.sy0) * J.slave_pitch + (xa - J.sx0);
+  if (J.slave_al8 && in0 && in1 && y0 >= J.sy0 && y0 + RS_H - 1 <= J.sy1) {
+    const short2 *src = J.slave + off;
+#pragma unroll
+    for (int k = 0; k < RS_H; k++, src += J.slave_pitch) cp_async_8(d + k * kRow, src, 8);
+  } else {
+#pragma unroll 1
+    for (int k = 0; k < RS_H; k++) {
+      const bool yin = y0 + k >= J.sy0 && y0 + k <= J.sy1;
+      const long o = off + (long)k * J.slave_pitch;
+      const bool i0 = yin && in0, i1 = yin && in1;
+      cp_async_4(d + k * kRow, J.slave + (i0 ? o : 0), i0 ? 4 : 0);
+      cp_async_4(d + k * kRow + 4, J.slave + (i1 ? o + 1 : 0), i1 ? 4 : 0);
+    }
+  }
+}
+
+// v = sum_j w[j] d[j] of both columns over the window slots (rot + j) % 12;
+// even and odd taps in two partial sums.
+template <int ROT>
+__device__ __forceinline__ float4 az_sum(const float4 (&wz)[6], const Dpair (&w)[12]) {
+  float2 ar = make_float2(0.f, 0.f), ai = ar, br = ar, bi = ar;
+#pragma unroll
+  for (int j = 0; j < kTaps; j += 2) {
+    const float2 w0 = make_float2(wz[j >> 1].x, wz[j >> 1].y);
+    const float2 w1 = make_float2(wz[j >> 1].z, wz[j >> 1].w);
+    const Dpair &d0 = w[(ROT + j) % 12], &d1 = w[(ROT + j + 1) % 12];
+    ar = __ffma2_rn(w0, d0.re, ar);
+    ai = __ffma2_rn(w0, d0.im, ai);
+    br = __ffma2_rn(w1, d1.re, br);
+    bi = __ffma2_rn(w1, d1.im, bi);
+  }
+  const float2 r = __fadd2_rn(ar, br), i = __fadd2_rn(ai, bi);
+  return make_float4(r.x, r.y, i.x, i.y);
+}
+
+__device__ __forceinline__ void az_taps(float4 (&w)[6], const RsLut &lut, int bin) {
+  const float4 *p = lut.kaz2 + bin * (kTaps / 2);
+#pragma unroll
+  for (int q = 0; q < kTaps / 2; q++) w[q] = __ldg(p + q);
+}
+
+// The entries [e0, e1) of one window position.
+template <int ROT, bool kSplit>
+__device__ __forceinline__ void az_entries(RsStrip<kSplit> &Q, const RsLut &lut, int u, int e0,
+                                           int e1, int tbase, const Dpair (&w)[12]) {
+#pragma unroll 1
+  for (int e = e0; e < e1; e++) {
+    const int4 M = Q.eM[e];
+    if (((M.y >> 12) & 15) != REG_IN) continue;   // edge, outside, or summed directly
+    const int off = (short)(M.w & 0xffff), ulo = (M.w >> 16) & 0xff, uhi = (M.w >> 24) & 0xff;
+    if (uhi < (u & ~31) || ulo > (u | 31)) continue;   // none of the warp's columns
+    float4 wz[6];
+    az_taps(wz, lut, M.y & 0xfff);
+    if (u >= ulo && u <= uhi) Q.tile[tbase + off + u] = az_sum<ROT>(wz, w);
+  }
+}
+
+// The window before the first push of a half anew: lines lb - 6 .. lb + 5.
+template <int HALF, bool kSplit>
+__device__ __forceinline__ void az_fill(const RsStrip<kSplit> &Q, const ResampleJob &J, int xa,
+                                        int lb, const RingPhase<kSplit> &R, Dpair (&w)[12]) {
+  uint2 raw[12];
+#pragma unroll
+  for (int j = 0; j < 12; j++) raw[j] = raw_pair(J, xa, lb - 6 + j);
+#pragma unroll
+  for (int j = 0; j < 12; j++)
+    w[(RS_H * HALF + j + 11) % 12] =
+        deramp_pair<kSplit>(raw[j], line_terms<kSplit>(Q, J, lb - 6 + j), R);
+}
+
+// One half (number h of the chunk): the window of row k is slots
+// (6 HALF + k + j) % 12.  A plain half takes its taps once and one sum per push.
+template <int HALF, bool kSplit>
+__device__ __forceinline__ void az_half(RsShared<kSplit> &S, RsStrip<kSplit> &Q,
+                                        const ResampleJob &J, int t, int u, int xa, int h,
+                                        const RsHalf &H, Dpair (&w)[12]) {
+  constexpr int R0 = RS_H * HALF;
+  const RingPhase<kSplit> R = ring_load<kSplit>(Q, u);
+  const RsLut &lut = J.lut;
+  const RsSlaveRow *sr = &Q.srow[h * RS_H];
+  if (H.flags & HG_FILL) az_fill<HALF, kSplit>(Q, J, xa, H.lb, R, w);
+  if (H.flags & HG_PLAIN) {
+    float4 wz[6];
+    az_taps(wz, lut, Q.eM[H.pos[0]].y & 0xfff);
+    float4 *o = &Q.tile[H.tbase + u];
+#define RS_PUSH(k)                                                              \
+  w[(R0 + (k) + 11) % 12] = deramp_pair<kSplit>(S.stage[R0 + (k)][t], sr[k], R); \
+  o[(k) * RS_UN] = az_sum<(R0 + (k)) % 12>(wz, w);
+    RS_PUSH(0)
+    RS_PUSH(1)
+    RS_PUSH(2)
+    RS_PUSH(3)
+    RS_PUSH(4)
+    RS_PUSH(5)
+#undef RS_PUSH
+    return;
+  }
+  az_entries<(R0 + 11) % 12, kSplit>(Q, lut, u, H.pos[0], H.pos[1], H.tbase, w);
+#define RS_PUSH(k)                                                              \
+  w[(R0 + (k) + 11) % 12] = deramp_pair<kSplit>(S.stage[R0 + (k)][t], sr[k], R); \
+  az_entries<(R0 + (k)) % 12, kSplit>(Q, lut, u, H.pos[(k) + 1], H.pos[(k) + 2], H.tbase, w);
+  RS_PUSH(0)
+  RS_PUSH(1)
+  RS_PUSH(2)
+  RS_PUSH(3)
+  RS_PUSH(4)
+  RS_PUSH(5)
+#undef RS_PUSH
+}
+
+// Entries whose line is no window position of their half (the row-to-line
+// map skipped or repeated a line): the same sum, in the same order, over
+// lines deramped anew.
+template <bool kSplit>
+__device__ __forceinline__ void az_direct(RsStrip<kSplit> &Q, const ResampleJob &J, int u, int xa,
+                                          int tbase, int e0, int e1) {
+  const RingPhase<kSplit> R = ring_load<kSplit>(Q, u);
+#pragma unroll 1
+  for (int e = e0; e < e1; e++) {
+    const int4 M = Q.eM[e];
+    if (((M.y >> 12) & 15) != (REG_IN | E_DIRECT)) continue;
+    const int off = (short)(M.w & 0xffff), ulo = (M.w >> 16) & 0xff, uhi = (M.w >> 24) & 0xff;
+    if (u < ulo || u > uhi) continue;
+    const float4 *p = J.lut.kaz2 + (M.y & 0xfff) * (kTaps / 2);
+    float2 ar = make_float2(0.f, 0.f), ai = ar, br = ar, bi = ar;
+#pragma unroll 1
+    for (int j = 0; j < kTaps; j += 2) {
+      const float4 q = __ldg(p + (j >> 1));
+      const int y = M.x - 5 + j;
+      const Dpair d0 = deramp_pair<kSplit>(raw_pair(J, xa, y), line_terms<kSplit>(Q, J, y), R);
+      const Dpair d1 =
+          deramp_pair<kSplit>(raw_pair(J, xa, y + 1), line_terms<kSplit>(Q, J, y + 1), R);
+      ar = __ffma2_rn(make_float2(q.x, q.y), d0.re, ar);
+      ai = __ffma2_rn(make_float2(q.x, q.y), d0.im, ai);
+      br = __ffma2_rn(make_float2(q.z, q.w), d1.re, br);
+      bi = __ffma2_rn(make_float2(q.z, q.w), d1.im, bi);
+    }
+    const float2 r = __fadd2_rn(ar, br), i = __fadd2_rn(ai, bi);
+    Q.tile[tbase + off + u] = make_float4(r.x, r.y, i.x, i.y);
+  }
+}
+
+// ---------------------------------------------------- range pass
+// Taps from unit boundaries: samples of units U[0..5], weights w[0..11].
+template <int N>
+__device__ __forceinline__ float2 rg_sum(const float4 (&w)[(N + 1) / 2], const float4 *U) {
+  float2 re = make_float2(0.f, 0.f), im = re;
+#pragma unroll
+  for (int m = 0; m < N; m++) {
+    const float2 ww = (m & 1) ? make_float2(w[m >> 1].z, w[m >> 1].w)
+                              : make_float2(w[m >> 1].x, w[m >> 1].y);
+    re = __ffma2_rn(ww, make_float2(U[m].x, U[m].y), re);
+    im = __ffma2_rn(ww, make_float2(U[m].z, U[m].w), im);
+  }
+  return make_float2(re.x + re.y, im.x + im.y);
+}
+
+__device__ __forceinline__ void taps_even(float4 (&w)[3], const RsLut &lut, int bin) {
+  const float4 *p = reinterpret_cast<const float4 *>(lut.krg) + bin * 3;
+#pragma unroll
+  for (int q = 0; q < 3; q++) w[q] = __ldg(p + q);
+}
+__device__ __forceinline__ void taps_odd(float4 (&w)[4], const RsLut &lut, int bin) {
+  const float4 *p = lut.krgo + bin * 4;
+#pragma unroll
+  for (int q = 0; q < 4; q++) w[q] = __ldg(p + q);
+}
+
+// Reramp phase of a pixel in turns: (1 + sp) Psi + G2 R2 + G1 R1 + G0 R0, with
+// Psi as its reduced value plus sp times its float value.  A: (rho, psif, R2,
+// R1), g: (sp, G2, G1, G0).
+__device__ __forceinline__ float run_phase(float4 A, float R0, float4 g) {
+  return fmaf(g.x, A.y, A.x) + fmaf(g.y, A.z, fmaf(g.z, A.w, g.w * R0));
+}
+
+// The current runs of a thread's two output columns.
+struct PairRuns {
+  float4 gx, gy;
+  float4 we[3], wo[4];   // pair: taps of the even-aligned and of the odd column
+  int next;              // chunk row of the next change
+  int unit;              // pair: first tile unit of its 14 samples
+  bool pair, odd;        // pair: both columns in the ring, adjacent samples;
+                         // odd: the first column is the odd-aligned one
 };
 
-__device__ __forceinline__ void run_load(ColRun &cr, const RsShared &S, const ResampleJob &J,
-                                         int c, int m) {
-  const int n = S.run_n[c];
-  const int2 rk = S.run_rk[c][m];
-  const float4 g = S.run_g[c][m];
-  cr.m = m;
-  cr.key = rk.y;
-  cr.next = (m + 1 < n) ? S.run_rk[c][m + 1].x : INT32_MAX;
-  cr.sp = g.x;
-  cr.G2 = g.y;
-  cr.G1 = g.z;
-  cr.G0 = g.w;
-  const int p0 = rk.y >> 12;
-  const int xb = p0 - 5 - S.xw;
-  cr.ok = p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7 && xb >= 0 && xb + 13 < RS_FW;
+// Ring column of a key's first tap when the column is range-interior and
+// inside the ring, else -1.
+__device__ __forceinline__ int ring_col(int xo, const ResampleJob &J, int key) {
+  const int p0 = key >> 12, xb = p0 - 5 - xo;
+  return (p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7 && xb >= 0 && xb + 13 < RS_FW) ? xb : -1;
 }
 
-// The range weights of the column's current run (fast runs only).  They are
-// loaded at the start of each group's range pass and after a run change, so
-// they hold no registers during the azimuth pass.
-__device__ __forceinline__ void run_weights(ColRun &cr, const ResampleJob &J) {
-  if (cr.ok) {
-    const float4 *kp4 = J.lut.krg2 + (cr.key & 4095) * (kTaps / 2);
-#pragma unroll
-    for (int q = 0; q < kTaps / 2; q++) cr.w[q] = __ldg(kp4 + q);
-  }
-}
-
-__device__ __forceinline__ float2 wtap(const ColRun &cr, int i) {
-  const float4 q = cr.w[i >> 1];
-  return (i & 1) ? make_float2(q.z, q.w) : make_float2(q.x, q.y);
-}
-
-// 12-tap range pass of two adjacent columns over the 14 samples V (the first
-// column's taps start at V[odd], the second's at V[odd + 1]); two partial
-// sums per column shorten the FMA chains.
-__device__ __forceinline__ void range_pair(const ColRun &c0, const ColRun &c1,
-                                           const float2 (&V)[14], bool odd, float2 &s0,
-                                           float2 &s1) {
-  float2 a0 = make_float2(0.f, 0.f), b0 = a0, a1 = a0, b1 = a0;
-  if (odd) {
-#pragma unroll
-    for (int i = 0; i < kTaps; i += 2) {
-      a0 = __ffma2_rn(wtap(c0, i), V[i + 1], a0);
-      b0 = __ffma2_rn(wtap(c0, i + 1), V[i + 2], b0);
-      a1 = __ffma2_rn(wtap(c1, i), V[i + 2], a1);
-      b1 = __ffma2_rn(wtap(c1, i + 1), V[i + 3], b1);
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < kTaps; i += 2) {
-      a0 = __ffma2_rn(wtap(c0, i), V[i], a0);
-      b0 = __ffma2_rn(wtap(c0, i + 1), V[i + 1], b0);
-      a1 = __ffma2_rn(wtap(c1, i), V[i + 1], a1);
-      b1 = __ffma2_rn(wtap(c1, i + 1), V[i + 2], b1);
-    }
-  }
-  s0 = __fadd2_rn(a0, b0);
-  s1 = __fadd2_rn(a1, b1);
-}
-
-// 12-tap range pass of one column from a tile row (8-byte loads).
-__device__ __forceinline__ float2 range_single(const float2 *row, int xb, const ColRun &cr) {
-  float2 a = make_float2(0.f, 0.f), b = a;
-#pragma unroll
-  for (int i = 0; i < kTaps; i += 2) {
-    a = __ffma2_rn(wtap(cr, i), row[xb + i], a);
-    b = __ffma2_rn(wtap(cr, i + 1), row[xb + i + 1], b);
-  }
-  return __fadd2_rn(a, b);
-}
-
-// Reramp phase of a pixel: (1 + sp) Psi + G2 R2 + G1 R1 + G0 R0, with Psi
-// as its reduced value plus sp times its float value.
-__device__ __forceinline__ float run_phase(const RsRow &R, const ColRun &cr) {
-  return fmaf(cr.sp, R.psif, R.rho) + fmaf(cr.G2, R.R2, fmaf(cr.G1, R.R1, cr.G0 * R.R0));
-}
-
-// Deramped slave sample (line y, this thread's ring column) for the
-// azimuth-pass window: from the staged lines when the line is staged, else
-// from HBM.
 template <bool kSplit>
-__device__ __forceinline__ float2 deramp_at(const RsShared &S, const ResampleJob &J, int x,
-                                            int xa, bool xin, int y, int win_lo, int win_hi,
-                                            float g2c, float g1c, float g0c,
-                                            const DerampQuad &cq) {
-  float sx, sy;
-  if (y >= win_lo && y <= win_hi) {
-    const short2 v = S.stage[y & (RS_SR - 1)][x];
-    sx = (float)v.x;
-    sy = (float)v.y;
-  } else {
-    if (!xin || y < J.sy0 || y > J.sy1) return make_float2(0.f, 0.f);
-    const short2 v = J.slave[(long)(y - J.sy0) * J.slave_pitch + (xa - J.sx0)];
-    sx = (float)v.x;
-    sy = (float)v.y;
-  }
-  const int iy = y - S.ys0;
-  float r;
-  if (kSplit) {
-    float rho, tc;
-    if ((unsigned)iy < (unsigned)RS_NSR) {
-      rho = S.srow[iy].f.rho;
-      tc = S.srow[iy].f.tc;
-    } else {
-      const DerampQuad refq = {S.ref_a0, S.ref_a1, S.ref_a2};
-      const double ta = (double)(y - J.s_first_line) * J.dt;
-      rho = to_turns(quad_eval(refq, ta));
-      tc = (float)(ta - S.tm);
+__device__ __forceinline__ void load_runs(PairRuns &P, const RsStrip<kSplit> &Q,
+                                          const ResampleJob &J, int c, bool two, int row) {
+  int next = INT32_MAX, n = Q.run_n[c], m = 0;
+  while (m + 1 < n && Q.run_rk[m + 1][c].x <= row) m++;
+  if (m + 1 < n) next = Q.run_rk[m + 1][c].x;
+  P.gx = Q.run_g[m][c];
+  const int keyx = Q.run_rk[m][c].y;
+  P.pair = false;
+  if (two) {
+    n = Q.run_n[c + 1];
+    m = 0;
+    while (m + 1 < n && Q.run_rk[m + 1][c + 1].x <= row) m++;
+    if (m + 1 < n) next = min(next, Q.run_rk[m + 1][c + 1].x);
+    P.gy = Q.run_g[m][c + 1];
+    const int keyy = Q.run_rk[m][c + 1].y;
+    const int xb = ring_col(Q.xo, J, keyx);
+    if (xb >= 0 && ring_col(Q.xo, J, keyy) == xb + 1) {
+      P.pair = true;
+      P.odd = (xb & 1) != 0;
+      P.unit = xb >> 1;
+      taps_even(P.we, J.lut, (P.odd ? keyy : keyx) & 4095);
+      taps_odd(P.wo, J.lut, (P.odd ? keyx : keyy) & 4095);
     }
-    const float G = fmaf(fmaf(g2c, tc, g1c), tc, g0c);
-    r = turns_reduce(rho + G) * kTwoPiF;
-  } else {
-    const double ta = ((unsigned)iy < (unsigned)RS_NSR) ? S.srow[iy].ta
-                                                         : (double)(y - J.s_first_line) * J.dt;
-    r = reduce_2pi(quad_eval(cq, ta));
   }
-  float sn, cs;
-  __sincosf(r, &sn, &cs);
-  return make_float2(sx * cs - sy * sn, sx * sn + sy * cs);
+  P.next = next;
 }
 
-// deramp_at for a line known to be staged and in the slave-line table.
+// One pixel (chunk row k, strip column c) of a shared row outside the pair path.
 template <bool kSplit>
-__device__ __forceinline__ float2 deramp_staged(const RsShared &S, int x, int y, int ys0,
-                                                float g2c, float g1c, float g0c,
-                                                const DerampQuad &cq) {
-  const short2 v = S.stage[y & (RS_SR - 1)][x];
-  const float sx = (float)v.x, sy = (float)v.y;
-  const RsSlaveRow sr = S.srow[y - ys0];
-  float r;
-  if (kSplit) {
-    const float G = fmaf(fmaf(g2c, sr.f.tc, g1c), sr.f.tc, g0c);
-    r = turns_reduce(sr.f.rho + G) * kTwoPiF;
-  } else {
-    r = reduce_2pi(quad_eval(cq, sr.ta));
+__device__ __forceinline__ void pixel_shared(RsStrip<kSplit> &Q, const ResampleJob &J, int k,
+                                             int tbase, int kt, int c, float2 *out) {
+  const int re = Q.rowe[k], ne = re >> 16;
+  int e = re & 0xffff;
+  for (int q = 1; q < ne; q++, e++) {
+    const int z = Q.eM[e].y;
+    if (c >= ((z >> 16) & 0xff) && c < ((z >> 24) & 0xff)) break;
   }
-  float sn, cs;
-  __sincosf(r, &sn, &cs);
-  return make_float2(sx * cs - sy * sn, sx * sn + sy * cs);
+  int m = 0;
+  while (m + 1 < Q.run_n[c] && Q.run_rk[m + 1][c].x <= k) m++;
+  const int key = Q.run_rk[m][c].y;
+  const int4 M = Q.eM[e];
+  const int p0 = key >> 12;
+  const int reg = min((M.y >> 12) & 3, region_1d(p0, J.sx0, J.sx1));
+  if (reg == REG_OUT) {
+    *out = make_float2(0.f, 0.f);
+    return;
+  }
+  if (reg == REG_EDGE) {
+    const short2 sv = J.slave[(long)(M.x - J.sy0) * J.slave_pitch + (p0 - J.sx0)];
+    *out = make_float2((float)sv.x, (float)sv.y);
+    return;
+  }
+  const int xb = ring_col(Q.xo, J, key);
+  const int ulo = (M.w >> 16) & 0xff, uhi = (M.w >> 24) & 0xff;
+  if (xb < 0 || (xb >> 1) < ulo || ((xb + 12) >> 1) > uhi) {
+    atomicOr(&Q.gen[kt][c >> 5], 1u << (c & 31));
+    Q.gen_any = 1;
+    return;
+  }
+  const float4 *U = &Q.tile[tbase + (short)(M.w & 0xffff) + (xb >> 1)];
+  float2 v;
+  if (xb & 1) {
+    float4 w[4];
+    taps_odd(w, J.lut, key & 4095);
+    v = rg_sum<7>(w, U);
+  } else {
+    float4 w[3];
+    taps_even(w, J.lut, key & 4095);
+    v = rg_sum<6>(w, U);
+  }
+  *out = cmul_conj_turns(v, run_phase(Q.eA[e], __int_as_float(M.z), Q.run_g[m][c]));
 }
 
-// Azimuth taps of a row (bin | slot << 16) as (w, w) pairs.
-__device__ __forceinline__ void load_az_taps(const RsShared &S, const RsLut &lut, int bin,
-                                             float4 (&wz)[6]) {
-  const int slot = bin >> 16;
-  if (slot < RS_MAXBIN) {
-#pragma unroll
-    for (int q = 0; q < 6; q++) wz[q] = S.bin_w[slot][q];
-  } else {
-    const float *kl = lut.kaz + (bin & 0xffff) * kTaps;
-#pragma unroll
-    for (int q = 0; q < 6; q++) {
-      const float a = __ldg(kl + 2 * q), b = __ldg(kl + 2 * q + 1);
-      wz[q] = make_float4(a, a, b, b);
+// The pixels the pair path left, all threads of a strip: pairs with a row in
+// Q.miss, nrows tile rows from chunk row k0 on; from row ks on the entries'
+// tile starts at tb1.  obase: the output at chunk row k0, strip column 0.
+template <bool kSplit>
+__device__ __forceinline__ void slow_pixels(RsStrip<kSplit> &Q, const ResampleJob &J, int u0,
+                                            int k0, int nrows, int ks, int tb1, int cN,
+                                            float2 *obase) {
+  const int n0 = __popc(Q.missb[0]), np = n0 + __popc(Q.missb[1]);
+  const int per = 2 * nrows;
+  for (int v = u0; v < np * per; v += RS_ST) {
+    int i = v / per;
+    const int w = v - i * per, q = w >> 1;
+    const int wq = i >= n0 ? 1 : 0;
+    if (wq) i -= n0;
+    unsigned m = Q.missb[wq];
+    while (i-- > 0) m &= m - 1;
+    const int uu = wq * 32 + __ffs(m) - 1;   // the pair's thread
+    const int c = 2 * uu + (w & 1);
+    if (c < cN && ((Q.miss[uu] >> q) & 1))
+      pixel_shared(Q, J, k0 + q, k0 + q >= ks ? tb1 : 0, q, c, obase + (long)q * J.out_pitch + c);
+  }
+}
+
+// ---------------------------------------------------- chunk prologue
+// Walks the azimuth-key runs of a row along the strip's columns, in the
+// direction of ascending lines: emit(region, line, bin, c_lo, c_hi), until it
+// returns false.
+template <bool kSplit, class Emit>
+__device__ __forceinline__ void walk_row(const RsShared<kSplit> &S, const ResampleJob &J, int r,
+                                         int c0, int cN, Emit emit) {
+  const double L = row_L(J, r);
+  const double A = row_a(S.caz, L) + S.shift, B = row_b(S.caz, L), C = S.caz[5];
+  const double pa = col_P(J, c0), pb = col_P(J, c0 + cN - 1);
+  {
+    // the whole strip in one run?
+    double ylo, yhi;
+    quad_span(A, B, C, pa, pb, ylo, yhi);
+    int l0, b0, l1, b1;
+    split_pos(ylo, l0, b0);
+    split_pos(yhi, l1, b1);
+    const int g0 = region_1d(l0, J.sy0, J.sy1), g1 = region_1d(l1, J.sy0, J.sy1);
+    if (g0 == g1 && ((l0 == l1 && (b0 == b1 || g0 == REG_EDGE)) ||
+                     (g0 == REG_OUT && (l0 > J.sy1 || l1 < J.sy0)))) {
+      emit(g0, l0, b0, 0, cN);
+      return;
     }
   }
-}
-
-// Stage this thread's ring column of slave lines [lo, hi] (zeros outside
-// the slave box) into the line ring.
-__device__ __forceinline__ void stage_rows(RsShared &S, const ResampleJob &J, int x, int xa,
-                                           bool xin, int lo, int hi) {
-  const short2 *const sl = J.slave;
-  const long pitch = J.slave_pitch;
-  const unsigned base = smem_u32(&S.stage[0][x]);
-  constexpr unsigned kRow = RS_FW * sizeof(short2);
-  if (xin && lo >= J.sy0 && hi <= J.sy1) {
-    // every line inside the slave box (the usual case): no per-line checks
-    const short2 *src = sl + (long)(lo - J.sy0) * pitch + (xa - J.sx0);
-#pragma unroll 4
-    for (int y = lo; y <= hi; y++, src += pitch)
-      cp_async_4s(base + (unsigned)(y & (RS_SR - 1)) * kRow, src, 4);
-  } else {
-    const unsigned rows_in = (unsigned)(J.sy1 - J.sy0);
-    long off = (long)(lo - J.sy0) * pitch + (xa - J.sx0);
+  // key of column c, ascending with the position: before the box -1, edge
+  // (line, 4095), interior (line, bin), past the box INT32_MAX; lines relative
+  // to the box
+  auto key = [&](int c) -> int {
+    int l, b;
+    split_pos(pix_pos(A, B, C, col_P(J, c0 + c)), l, b);
+    const int g = region_1d(l, J.sy0, J.sy1);
+    if (g == REG_OUT) return l < J.sy0 ? -1 : INT32_MAX;
+    return (l - J.sy0) * 4096 + (g == REG_EDGE ? 4095 : b);
+  };
+  // monotone pieces: split at the vertex
+  const double s0 = fma(2.0 * C, pa, B), s1 = fma(2.0 * C, pb, B);
+  int vert = cN - 1;
+  if ((s0 < 0.0) != (s1 < 0.0)) {
+    const double v = (-B / (2.0 * C)) / J.invP + J.midP - (double)c0;
+    if (v >= 0.0 && v < (double)(cN - 1)) vert = (int)v;
+  }
+  const bool rev = pix_pos(A, B, C, pb) < pix_pos(A, B, C, pa);
+  auto at = [&](int i) { return key(rev ? cN - 1 - i : i); };
+  int cur = -2, from = 0;
+  auto put = [&](int k, int i0, int i1) -> bool {   // run [i0, i1) of key k
+    const int c_lo = rev ? cN - i1 : i0, c_hi = rev ? cN - i0 : i1;
+    if (k == -1 || k == INT32_MAX) return emit(REG_OUT, 0, 0, c_lo, c_hi);
+    return emit((k & 4095) == 4095 ? REG_EDGE : REG_IN, J.sy0 + (k >> 12), k & 4095, c_lo, c_hi);
+  };
+  const int split = rev ? cN - 2 - vert : vert;   // last index of the first piece
+  int i = 0;
 #pragma unroll 1
-    for (int y = lo; y <= hi; y++, off += pitch) {
-      const bool in = xin && (unsigned)(y - J.sy0) <= rows_in;
-      cp_async_4s(base + (unsigned)(y & (RS_SR - 1)) * kRow, sl + (in ? off : 0), in ? 4 : 0);
+  for (int piece = 0; piece < 2; piece++) {
+    const int end = (piece == 0 && split >= 0) ? split : cN - 1;
+    if (i > end) continue;
+    int k = at(i);
+    const int kb = at(end);
+    for (;;) {
+      if (k != cur) {
+        if (cur != -2 && !put(cur, from, i)) return;
+        cur = k;
+        from = i;
+      }
+      if (k == kb) break;   // monotone: the rest of the piece has this key
+      int lo = i, hi = end, khi = kb;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        const int km = at(mid);
+        if (km == k) {
+          lo = mid;
+        } else {
+          hi = mid;
+          khi = km;
+        }
+      }
+      i = hi;
+      k = khi;
     }
+    i = end + 1;
   }
-  cp_async_commit();
+  put(cur, from, cN);
+}
+
+// Ring units of output columns [c_lo, c_hi), from the strip's bounds of
+// (ring column - strip column).
+template <bool kSplit>
+__device__ __forceinline__ void entry_units(const RsStrip<kSplit> &Q, int c_lo, int c_hi, int &ulo,
+                                            int &uhi) {
+  ulo = min(max(c_lo + Q.dlo, 0), RS_FW - 1) >> 1;
+  uhi = min(max(c_hi - 1 + Q.dhi + 13, 0), RS_FW - 1) >> 1;
+}
+
+// [P4] Counts the entries of a row (0: a per-pixel row).
+template <bool kSplit>
+__device__ __forceinline__ int count_entries(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
+                                             const ResampleJob &J, int r, int c0, int cN) {
+  int m = 0, units = 0;
+  walk_row(S, J, r, c0, cN, [&](int reg, int, int, int c_lo, int c_hi) -> bool {
+    m++;
+    if (reg == REG_IN) {
+      int ulo, uhi;
+      entry_units(Q, c_lo, c_hi, ulo, uhi);
+      units += uhi - ulo + 1;
+    }
+    return m <= RS_MAXKEY;
+  });
+  return (m > RS_MAXKEY || (m > 1 && units > RS_ROWU)) ? 0 : m;
+}
+
+// Reramp terms of the azimuth key (L0, bin): Psi = sum_j kAz[j]
+// phi_ref(L0 - 5 + j) (FP64) and the taps' moments about the burst centre
+// time, as (rho, psif, R2, R1) and R0.
+template <bool kSplit>
+__device__ __forceinline__ float4 row_terms(const RsStrip<kSplit> &Q, const ResampleJob &J, int L0,
+                                            int bin, float &R0) {
+  const DerampQuad refq = {Q.ref_a0, Q.ref_a1, Q.ref_a2};
+  const float *kl = J.lut.kaz + bin * kTaps;
+  double psi = 0.0, m0 = 0.0, m1 = 0.0, m2 = 0.0;
+#pragma unroll 4
+  for (int j = 0; j < kTaps; j++) {
+    const double w = (double)__ldg(kl + j), u = (double)(j - 5);
+    const double ta = (double)(L0 - 5 + j - J.s_first_line) * J.dt;
+    psi = fma(w, quad_eval(refq, ta), psi);
+    m0 += w;
+    m1 = fma(w, u, m1);
+    m2 = fma(w, u * u, m2);
+  }
+  const double tc0 = (double)(L0 - J.s_first_line) * J.dt - Q.tm;
+  const double dt = J.dt;
+  R0 = (float)m0;
+  return make_float4(to_turns(psi), (float)(psi * kInvTwoPi),
+                     (float)(m0 * tc0 * tc0 + 2.0 * tc0 * dt * m1 + dt * dt * m2),
+                     (float)(m0 * tc0 + dt * m1));
+}
+
+// [P5] Writes a row's entries from entry e on, with the reramp terms of their
+// keys.
+template <bool kSplit>
+__device__ __forceinline__ void write_entries(const RsShared<kSplit> &S, RsStrip<kSplit> &Q,
+                                              const ResampleJob &J, int r, int c0, int cN, int e) {
+  walk_row(S, J, r, c0, cN, [&](int reg, int L0, int bin, int c_lo, int c_hi) -> bool {
+    int ulo = 0, uhi = RS_UN - 1;
+    if (c_hi - c_lo < cN) entry_units(Q, c_lo, c_hi, ulo, uhi);
+    float R0 = 0.f;
+    if (reg == REG_IN) Q.eA[e] = row_terms(Q, J, L0, bin, R0);
+    Q.eM[e] = make_int4(L0, bin | reg << 12 | c_lo << 16 | c_hi << 24, __float_as_int(R0),
+                        ulo << 16 | uhi << 24);
+    e++;
+    return true;
+  });
 }
 
 // Phase terms of a range-key run: (sp, G2, G1, G0) with Gk = sum_i kRg[i]
 // gk(x_i) over the ring columns of its taps (0 when they leave the window).
-__device__ __forceinline__ float4 run_terms(const RsShared &S, const RsLut &lut, int xw,
-                                            int key) {
+template <bool kSplit>
+__device__ __forceinline__ float4 run_terms(const RsStrip<kSplit> &Q, const RsLut &lut, int key) {
   const int p0 = key >> 12, bp = key & 4095;
-  const int xb = p0 - 5 - xw;
+  const int xb = p0 - 5 - Q.xo;
   float4 gg = make_float4(__ldg(lut.sp1 + bp), 0.f, 0.f, 0.f);
   if (xb >= 0 && xb + kTaps <= RS_FW) {
     const float *kp = lut.krg + bp * kTaps;
@@ -543,7 +922,7 @@ __device__ __forceinline__ float4 run_terms(const RsShared &S, const RsLut &lut,
 #pragma unroll
     for (int i = 0; i < kTaps; i++) {
       const float w = __ldg(kp + i);
-      const float4 gc = S.ring_gc[xb + i];
+      const float4 gc = Q.ring_gc[xb + i];
       G2 = fmaf(w, gc.x, G2);
       G1 = fmaf(w, gc.y, G1);
       G0 = fmaf(w, gc.z, G0);
@@ -555,113 +934,147 @@ __device__ __forceinline__ float4 run_terms(const RsShared &S, const RsLut &lut,
   return gg;
 }
 
-// A pixel of a shared row (its azimuth-interpolated row in vrow) whose
-// column has no run table: its range key and the key's run terms are found
-// here, by the same functions the run tables are built with, so the result
-// is the one the run path gives.
-__device__ __forceinline__ float2 pixel_keyed(const RsShared &S, const ResampleJob &J,
-                                           const RsRow &R, const float2 *vrow, int r, int c) {
-  ColRun cr;
-  cr.key = rg_key(S, J, r, c);
-  const float4 g = run_terms(S, J.lut, S.xw, cr.key);
-  cr.sp = g.x;
-  cr.G2 = g.y;
-  cr.G1 = g.z;
-  cr.G0 = g.w;
-  const int p0 = cr.key >> 12;
-  const int xb = p0 - 5 - S.xw;
-  cr.ok = p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7 && xb >= 0 && xb + 13 < RS_FW;
-  if (cr.ok) {
-    run_weights(cr, J);
-    return cmul_conj_turns(range_single(vrow, xb, cr), run_phase(R, cr));
-  }
-  if (p0 < J.sx0 || p0 > J.sx1) return make_float2(0.f, 0.f);
-  if (p0 < J.sx0 + 5 || p0 > J.sx1 - 7) {
-    const short2 sv = J.slave[(long)(R.L0 - J.sy0) * J.slave_pitch + (p0 - J.sx0)];
-    return make_float2((float)sv.x, (float)sv.y);
-  }
-  return pixel_generic(S, J, r, c);
-}
-
-// Azimuth sum of this thread's ring column for the key (L0, bin) over
-// lines deramped anew (staged lines in [win_lo, win_hi] from shared memory,
-// others from HBM), in the order of the register-window sum.
+// [P6] The runs of column c's range key over chunk rows [0, n) (box rows rb
+// ...), by bisection of the exact per-pixel key on the pieces where the
+// position is monotone in the row; rows from the first change that does not
+// fit the table on are left to the next chunk (Q.cov).
 template <bool kSplit>
-__device__ __forceinline__ float2 az_direct(const RsShared &S, const ResampleJob &J,
-                                            const RsLut &lut, int x, int xa, bool xin, int L0,
-                                            int bin, int win_lo, int win_hi, float g2c,
-                                            float g1c, float g0c, const DerampQuad &cq) {
-  const float *kl = lut.kaz + bin * kTaps;
-  float2 a = make_float2(0.f, 0.f), b = a;
-#pragma unroll 1
-  for (int j = 0; j < RS_GR; j += 2) {
-    const float wa = __ldg(kl + j), wb = __ldg(kl + j + 1);
-    const float2 d0 =
-        deramp_at<kSplit>(S, J, x, xa, xin, L0 - 5 + j, win_lo, win_hi, g2c, g1c, g0c, cq);
-    const float2 d1 =
-        deramp_at<kSplit>(S, J, x, xa, xin, L0 - 4 + j, win_lo, win_hi, g2c, g1c, g0c, cq);
-    a = __ffma2_rn(make_float2(wa, wa), d0, a);
-    b = __ffma2_rn(make_float2(wb, wb), d1, b);
+__device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kSplit> &Q,
+                                           const ResampleJob &J, int rb, int n, int c0, int c) {
+  const double P = col_P(J, c0 + c);
+  auto keyat = [&](int ri) { return rg_key(S.crg, J, rb + ri, P); };
+  int ends[2] = {n - 1, n - 1};
+  int np = 1;
+  {
+    // x(L) = g0 + g2 P + g5 P^2 + (g1 + g4 P) L + g3 L^2: vertex in L
+    const double *g = S.crg;
+    if (g[3] != 0.0) {
+      const double Lv = -(g[1] + g[4] * P) / (2.0 * g[3]);
+      const double rv = Lv / J.invL + J.midL - (double)J.my0 - (double)rb;
+      if (rv > 0.0 && rv < (double)(n - 1)) {
+        ends[0] = (int)rv;
+        np = 2;
+      }
+    }
   }
-  return __fadd2_rn(a, b);
+  int m = 0, last_key = 0, a = 0;
+  bool full = false;
+  for (int pc = 0; pc < np && !full; pc++) {
+    const int bend = ends[pc];
+    if (a > bend) continue;
+    int r = a, k = keyat(a);
+    const int kb = keyat(bend);
+    for (;;) {
+      if (m == 0 || k != last_key) {
+        if (m == RsStrip<kSplit>::kRuns) {
+          atomicMin(&Q.cov, r);
+          full = true;
+          break;
+        }
+        Q.run_rk[m][c] = make_int2(r, k);
+        Q.run_g[m][c] = run_terms(Q, J.lut, k);
+        m++;
+        last_key = k;
+      }
+      if (k == kb) break;   // monotone: the rest of the piece has this key
+      int lo = r, hi = bend, khi = kb;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        const int km = keyat(mid);
+        if (km == k) {
+          lo = mid;
+        } else {
+          hi = mid;
+          khi = km;
+        }
+      }
+      r = hi;
+      k = khi;
+    }
+    a = bend + 1;
+  }
+  Q.run_n[c] = (unsigned char)m;
 }
 
-// Reramp row terms of the azimuth key (L0, bin): Psi = sum_j kAz[j]
-// phi_ref(L0 - 5 + j) (FP64) and the taps' moments about the burst centre
-// time.
-__device__ __forceinline__ void row_terms(const RsShared &S, const ResampleJob &J,
-                                          const RsLut &lut, int L0, int bin, RsRow &R) {
-  const DerampQuad refq = {S.ref_a0, S.ref_a1, S.ref_a2};
-  const float *kl = lut.kaz + bin * kTaps;
-  double psi = 0.0, m0 = 0.0, m1 = 0.0, m2 = 0.0;
-#pragma unroll 4
-  for (int j = 0; j < kTaps; j++) {
-    const double w = (double)__ldg(kl + j), u = (double)(j - 5);
-    const double ta = (double)(L0 - 5 + j - J.s_first_line) * J.dt;
-    psi = fma(w, quad_eval(refq, ta), psi);
-    m0 += w;
-    m1 = fma(w, u, m1);
-    m2 = fma(w, u * u, m2);
-  }
-  const double tc0 = (double)(L0 - J.s_first_line) * J.dt - S.tm;
-  const double dt = J.dt;
-  R.rho = to_turns(psi);
-  R.psif = (float)(psi * kInvTwoPi);
-  R.R2 = (float)(m0 * tc0 * tc0 + 2.0 * tc0 * dt * m1 + dt * dt * m2);
-  R.R1 = (float)(m0 * tc0 + dt * m1);
-  R.R0 = (float)m0;
-}
-
-// One work item (strip x segment of one job); all threads of the CTA call it
-// with the same item.
+// [P7] Half h of a chunk of n rows: its window's lines, the entries of each
+// window position, tile offsets.
 template <bool kSplit>
-__device__ __forceinline__ void resample_item(RsShared &S, const RsBatch &B, int item) {
-  const int tid = threadIdx.x;
+__device__ __forceinline__ void plan_half(RsStrip<kSplit> &Q, int h, int n) {
+  RsHalf H;
+  H.flags = 0;
+  H.lb = 0;
+  H.tbase = 0;
+  H.units = 0;
+  const int r0 = h * RS_H, r1 = min(r0 + RS_H, n);
+  for (int r = r0; r < r1 && !(H.flags & HG_ON); r++) {
+    const int re = Q.rowe[r], e0 = re & 0xffff, ne = re >> 16;
+    for (int e = e0; e < e0 + ne; e++)
+      if (((Q.eM[e].y >> 12) & 15) == REG_IN) {
+        H.flags |= HG_ON;
+        H.lb = Q.eM[e].x - (r - r0);   // the row's last (highest) line
+      }
+  }
+  int cur = -1, end = Q.rowe[r0] & 0xffff, bin0 = -1;
+  bool one = true, plain = r1 - r0 == RS_H;
+  H.pos[0] = (short)end;
+  for (int r = r0; r < r1; r++) {
+    const int re = Q.rowe[r], e0 = re & 0xffff, ne = re >> 16;
+    if (ne == 0) H.flags |= HG_PIX;
+    one = one && ne == 1 && ((Q.eM[e0].y >> 12) & 15) == REG_IN;
+    for (int e = e0; e < e0 + ne; e++) {
+      int4 M = Q.eM[e];
+      if (((M.y >> 12) & 15) == REG_IN) {
+        const int ulo = (M.w >> 16) & 0xff, uhi = (M.w >> 24) & 0xff;
+        const int p = M.x - H.lb;
+        plain = plain && p == r - r0 && (bin0 < 0 || (M.y & 0xfff) == bin0);
+        bin0 = M.y & 0xfff;
+        if (p < cur || p >= RS_H) {
+          M.y |= E_DIRECT << 12;
+          H.flags |= HG_DIRECT;
+        } else {
+          for (; cur < p; cur++) H.pos[cur + 2] = (short)e;
+        }
+        M.w = (M.w & ~0xffff) | ((H.units - ulo) & 0xffff);
+        H.units += uhi - ulo + 1;
+        Q.eM[e] = M;
+      }
+      end = e + 1;
+    }
+  }
+  for (; cur < RS_H; cur++) H.pos[cur + 2] = (short)end;
+  if (one) H.flags |= HG_ONE | (plain ? HG_PLAIN : 0);
+  Q.half[h] = H;
+}
 
-  // ---- locate the work item (job, strip, segment)
+// One work item (strip pair x segment of one job); all threads of the CTA call
+// it with the same item.  Threads 0..63 work on the first strip, the others on
+// the second; only the barriers and the row loop are common.
+template <bool kSplit>
+__device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch &B, int item) {
+  const int t = threadIdx.x, side = t / RS_ST, u = t % RS_ST;
+  RsStrip<kSplit> &Q = S.strip[side];
+
+  // ---- locate the work item (job, strip pair, segment)
   int jb = 0;
   while (jb + 1 < B.njobs && B.jobs[jb + 1].item_begin <= item) jb++;
   const ResampleJob &J = B.jobs[jb];
-  const RsLut &lut = J.lut;
   const int local = item - J.item_begin;
-  const int strip = local % J.strips;
   const int seg = local / J.strips;
-  const int mpix = J.mx1 - J.mx0 + 1;
-  const int c0 = strip * RS_TW;
-  const int cN = min(RS_TW, mpix - c0);
+  const int c0 = ((local - seg * J.strips) * RS_NS + side) * RS_TW;
+  const int cN = min(RS_TW, J.mx1 - J.mx0 + 1 - c0);   // <= 0: no such strip
+  const bool live = cN > 0;
   const int r_begin = J.row0 + seg * J.seg_rows;
-  const int r_end = min(r_begin + J.seg_rows, J.row0 + J.nrows);
-  const int nr = r_end - r_begin;
+  const int nr = min(J.seg_rows, J.row0 + J.nrows - r_begin);
 
   // ---- [P1] polynomials and shift
-  if (tid < 12) {
-    const double v = J.cpm_dev ? J.cpm_dev[tid] : (tid < 6 ? J.caz[tid] : J.crg[tid - 6]);
-    if (tid < 6)
-      S.caz[tid] = v;
+  if (t < 12) {
+    const double v = J.cpm_dev ? J.cpm_dev[t] : (t < 6 ? J.caz[t] : J.crg[t - 6]);
+    if (t < 6)
+      S.caz[t] = v;
     else
-      S.crg[tid - 6] = v;
+      S.crg[t - 6] = v;
   }
-  if (tid == 12) {
+  if (t == 12) {
     double sh = J.az_shift;
     if (J.az_shift_dev) {
       // a device-provided ESD shift above 100 px is invalid and reset to 0,
@@ -671,666 +1084,292 @@ __device__ __forceinline__ void resample_item(RsShared &S, const RsBatch &B, int
     }
     S.shift = sh;
   }
+  if (u < 2 * RS_H * 4) (&Q.gen[0][0])[u] = 0u;
   __syncthreads();
 
-  // ---- [P2] column terms; the ring window and the reference column
-  if (tid < RS_TW) {
-    const double P = ((double)(c0 + min(tid, cN - 1)) - J.midP) * J.invP;
-    S.col_phat[tid] = P;
-    S.col_qaz[tid] = S.caz[5] * P * P;
-    S.col_qrg[tid] = S.crg[5] * P * P;
-  }
-  if (tid == RS_NT - 1) {
-    // range position at the corners and edge midpoints of the strip over
-    // the whole master box -> window.  The window, and with it the reference
-    // column of the phase split, depends on the strip only, so a job that
-    // produces a subset of the rows gives those rows bit for bit as the
-    // whole job does.
-    double pmin = 1e300;
+  // ---- [P2] the ring's origin, the bounds of (ring column - strip column)
+  // and the reference column, from the range position at the corners and edge
+  // midpoints of the strip over the whole master box: they depend on the strip
+  // only, so a job that produces a subset of the rows gives those rows bit for
+  // bit as the whole job does.
+  if (u == 0) {
+    double pmin = 1e300, dmin = 1e300, dmax = -1e300;
     const int box_rows = J.my1 - J.my0 + 1;
     for (int a = 0; a < 3; a++) {
       const int rr = (a == 0) ? 0 : (a == 1 ? (box_rows - 1) / 2 : box_rows - 1);
       const double L = row_L(J, rr);
       for (int b = 0; b < 3; b++) {
-        const int cc = (b == 0) ? c0 : (b == 1 ? c0 + (cN - 1) / 2 : c0 + cN - 1);
-        const double P = ((double)cc - J.midP) * J.invP;
+        const int cc = (b == 0) ? 0 : (b == 1 ? (cN - 1) / 2 : cN - 1);
+        const double P = col_P(J, c0 + cc);
         const double *c = S.crg;
         const double x = c[0] + c[1] * L + c[2] * P + c[3] * L * L + c[4] * L * P + c[5] * P * P;
         pmin = fmin(pmin, x);
+        dmin = fmin(dmin, x - (double)cc);
+        dmax = fmax(dmax, x - (double)cc);
       }
     }
-    // the range pass reads ring columns [p0 - 5, p0 + 8] of a column pair;
-    // one column of margin for the position's variation inside the strip
+    // the range pass reads ring columns [p0 - 5, p0 + 8] of a column pair; one
+    // column of margin for the position's variation inside the strip, and the
+    // ring starts on a sample pair of the slave box's rows
     const int xw = (int)floor(pmin) - 6;
-    S.xw = xw;
-    S.ys0 = INT32_MAX;   // first slave line used: minimum taken in [P6a]
     const int xr = min(max(xw + RS_FW / 2, J.sx0), J.sx1);
     const DerampQuad q = deramp_quad(J.kt[xr], J.tref[xr], J.fdc[xr]);
-    S.ref_a0 = q.a0;
-    S.ref_a1 = q.a1;
-    S.ref_a2 = q.a2;
-    S.tm = 0.5 * (double)(J.sy0 + J.sy1 - 2 * J.s_first_line) * J.dt;
+    Q.ref_a0 = q.a0;
+    Q.ref_a1 = q.a1;
+    Q.ref_a2 = q.a2;
+    Q.tm = 0.5 * (double)(J.sy0 + J.sy1 - 2 * J.s_first_line) * J.dt;
+    const int xo = xw - ((xw - J.sx0) & 1);
+    Q.xo = xo;
+    Q.dlo = max((int)floor(dmin) - 6 - xo, -RS_FW);
+    Q.dhi = min((int)floor(dmax) - 4 - xo, RS_FW);
+    Q.gen_any = 0;
+    Q.prev_line = INT32_MIN;
+    Q.missb[0] = Q.missb[1] = 0u;
   }
   __syncthreads();
 
-  // ---- [P3] this thread's ring column: deramp coefficients
-  const int xw = S.xw;
-  const int x = tid;                     // ring column
-  const int xa = xw + x;                 // absolute slave column
-  const bool xin = xa >= J.sx0 && xa <= J.sx1;
-  const double tm = S.tm;
-  DerampQuad cq;
-  float g2c, g1c, g0c;   // G = phi - phi_ref about tm: g2 tc^2 + g1 tc + g0
+  // ---- [P3] this thread's two ring columns: G = phi - phi_ref about tm
+  // (g2 tc^2 + g1 tc + g0)
+  const int xa = Q.xo + 2 * u;           // absolute slave column
   {
-    const DerampQuad refq = {S.ref_a0, S.ref_a1, S.ref_a2};
-    cq = refq;
-    if (xin) cq = deramp_quad(J.kt[xa], J.tref[xa], J.fdc[xa]);
-    const double d2 = cq.a2 - refq.a2, d1 = cq.a1 - refq.a1, d0 = cq.a0 - refq.a0;
-    g2c = (float)(d2 * kInvTwoPi);   // in turns
-    g1c = (float)((2.0 * d2 * tm + d1) * kInvTwoPi);
-    g0c = (float)(((d2 * tm + d1) * tm + d0) * kInvTwoPi);
-  }
-  S.ring_gc[x] = make_float4(g2c, g1c, g0c, 0.f);
-
-  // ---- [P4] per-row statistics: one shared azimuth pass where the whole
-  // strip maps to one (line, bin) key inside the slave box's interior; where
-  // it maps to two adjacent bins of one line and the position is monotone
-  // along the strip, the columns of the second bin are found by bisection of
-  // the exact per-pixel key
-  for (int ri = tid; ri < nr; ri += RS_NT) {
-    const double L = row_L(J, r_begin + ri);
-    const double Aaz = row_a(S.caz, L) + S.shift, Baz = row_b(S.caz, L);
-    double ylo, yhi;
-    quad_span(Aaz, Baz, S.caz[5], S.col_phat[0], S.col_phat[cN - 1], ylo, yhi);
-    int l0lo, blo, l0hi, bhi;
-    split_pos(ylo, l0lo, blo);
-    split_pos(yhi, l0hi, bhi);
-    const bool inter = l0lo >= J.sy0 + 5 && l0hi <= J.sy1 - 7;
-    const bool fast = (l0lo == l0hi) && (blo == bhi) && inter;
-    int mode = fast ? RM_SHARED : RM_PIXEL;
-    if (!fast && inter && l0lo == l0hi && bhi == blo + 1) {
-      const double c2 = 2.0 * S.caz[5];
-      const double s0 = fma(c2, S.col_phat[0], Baz), s1 = fma(c2, S.col_phat[cN - 1], Baz);
-      if ((s0 < 0.0) == (s1 < 0.0)) {
-        auto is_hi = [&](int c) {
-          int l, b;
-          split_pos(pix_pos(Aaz, Baz, S.col_phat[c], S.col_qaz[c]), l, b);
-          return b == bhi;
-        };
-        const bool f0 = is_hi(0);
-        int t = cN;   // first column whose bin differs from column 0's
-        if (is_hi(cN - 1) != f0) {
-          int lo = 0, hi = cN - 1;
-          while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (is_hi(mid) == f0)
-              lo = mid;
-            else
-              hi = mid;
-          }
-          t = hi;
-        }
-        const int c_lo = f0 ? 0 : t, c_hi = f0 ? t : cN;
-        mode = RM_TWO | (c_lo << 8) | (c_hi << 16);
-      }
-    }
-    RsRow R;
-    R.L0 = l0lo;
-    R.bin = blo | (RS_NOSLOT << 16);
-    R.rho = R.psif = R.R2 = R.R1 = R.R0 = 0.f;
-    if (mode != RM_PIXEL) row_terms(S, J, lut, l0lo, blo, R);
-    R.mode = mode;
-    S.rows[ri] = R;
-  }
-  __syncthreads();
-
-  // ---- [P5] the window of the azimuth pass over the groups.  The window
-  // advances one line per row; a group whose first row with a single key
-  // finds another line than the window expects (or no window yet) fills it
-  // anew at the group's start, with the line of that row extrapolated back
-  // one line per row.  A row takes the shared pass when it has a single key
-  // and its line is the window's.  Thread g finds group g's first
-  // single-key row; thread 0 then chains the groups.
-  {
-    const int ngrp = (nr + RS_GR - 1) / RS_GR;
-    if (tid < ngrp) {
-      int k1 = -1, l1 = 0;
-      for (int k = 0; k < RS_GR && tid * RS_GR + k < nr; k++) {
-        const RsRow &R = S.rows[tid * RS_GR + k];
-        if (R.mode) {
-          k1 = k;
-          l1 = R.L0;
-          break;
-        }
-      }
-      S.grange[tid] = make_int2(k1, l1);
-    }
-  }
-  __syncthreads();
-  if (tid == 0) {
-    const int ngrp = (nr + RS_GR - 1) / RS_GR;
-    bool on = false;
-    int base_row = 0, base_L0 = 0;
-    for (int g = 0; g < ngrp; g++) {
-      const int p = g * RS_GR;
-      const int2 f = S.grange[g];   // first single-key row of the group, its line
-      bool fill = false;
-      if (f.x >= 0 && (!on || f.y != base_L0 + (p + f.x - base_row))) {
-        fill = true;
-        on = true;
-        base_row = p + f.x;
-        base_L0 = f.y;
-      }
-      // (window on, bit 0: filled here | bit 1: check-free loop, line of
-      // row 0, per-pixel rows)
-      S.gwin[g] = make_int4(on ? 1 : 0, fill ? 1 : 0, on ? base_L0 + (p - base_row) : 0, 0);
-      S.gen_n[g] = 0;
-      S.gen_d[g] = 0;
-    }
-    S.ngrp = ngrp;
-  }
-  __syncthreads();
-
-  // ---- [P6a] row modes; azimuth-bin table (a slot per change of the bin
-  // between consecutive shared rows, ranked by a block-wide scan); each
-  // group's line range and per-pixel rows; the first slave line used.
-  // Thread t takes rows 2t and 2t + 1.
-  {
-    const int lane = tid & 31, warp = tid >> 5;
-    const int r0 = 2 * tid, r1 = r0 + 1;
-    auto shared_row = [&](int ri) -> bool { return ri < nr && S.rows[ri].mode; };
-    const bool h0 = shared_row(r0), h1 = shared_row(r1);
-    const bool p0 = r0 > 0 && shared_row(r0 - 1);
-    auto bin_of = [&](int ri) { return S.rows[ri].bin & 0xffff; };
-    const int f0 = h0 && (!p0 || bin_of(r0 - 1) != bin_of(r0)) ? 1 : 0;
-    const int f1 = h1 && (!h0 || bin_of(r0) != bin_of(r1)) ? 1 : 0;
-    int v = f0 + f1;
+    const DerampQuad refq = {Q.ref_a0, Q.ref_a1, Q.ref_a2};
+    const double tm = Q.tm;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += t;
-    }
-    if (lane == 31) S.scan[warp] = v;
-    int ymin = INT32_MAX;
-    const int ngrp = S.ngrp;
-    if (tid < ngrp) {
-      const int4 gw = S.gwin[tid];
-      const int gr = min(RS_GR, nr - tid * RS_GR);
-      if (gw.x) ymin = gw.z - (gw.y ? 5 : -6);
-      // rows without a shared pass (bits 0..11) and shared rows whose line
-      // is not the window's, summed directly (bits 16..27)
-      int mask = 0, two = 0;
-      for (int k = 0; k < gr; k++) {
-        const int ri = tid * RS_GR + k;
-        if (!shared_row(ri))
-          mask |= 1 << k;
-        else if (!gw.x || S.rows[ri].L0 != gw.z + k)
-          mask |= 1 << (16 + k);
-        if (shared_row(ri) && (S.rows[ri].mode & 0xff) == RM_TWO) two |= 1 << k;
+    for (int q = 0; q < 2; q++) {
+      const int x = xa + q;
+      DerampQuad cq = refq;
+      if (x >= J.sx0 && x <= J.sx1) cq = deramp_quad(J.kt[x], J.tref[x], J.fdc[x]);
+      const double d2 = cq.a2 - refq.a2, d1 = cq.a1 - refq.a1, d0 = cq.a0 - refq.a0;
+      Q.ring_gc[2 * u + q] = make_float4((float)(d2 * kInvTwoPi),   // in turns
+                                         (float)((2.0 * d2 * tm + d1) * kInvTwoPi),
+                                         (float)(((d2 * tm + d1) * tm + d0) * kInvTwoPi), 0.f);
+      if constexpr (!kSplit) {
+        Q.ring.a21[2 * u + q] = make_double2(cq.a2, cq.a1);
+        Q.ring.a0[2 * u + q] = cq.a0;
       }
-      // rows with a second bin (bits 4..15 of the flags)
-      S.gwin[tid].y = gw.y | (two << 4);
-      S.grange[tid] = gw.x ? make_int2(gw.y ? gw.z - 5 : gw.z + 6, gw.z + gr - 1 + 6)
-                           : make_int2(1, 0);
-      S.gwin[tid].w = mask;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ymin = min(ymin, __shfl_xor_sync(0xffffffffu, ymin, o));
-    if (lane == 0 && ymin != INT32_MAX) atomicMin(&S.ys0, ymin);
-    __syncthreads();
-    int off = 0, total = 0;
-#pragma unroll
-    for (int q = 0; q < RS_NT / 32; q++) {
-      const int t = S.scan[q];
-      off += q < warp ? t : 0;
-      total += t;
-    }
-    const int incl0 = off + v - f1, incl1 = incl0 + f1;   // inclusive ranks
-    auto set_row = [&](int ri, bool h, int incl, int f) {
-      if (ri >= nr) return;
-      RsRow &R = S.rows[ri];
-      if (!h) {
-        R.mode = RM_PIXEL;
-        return;
-      }
-      const int b = R.bin & 0xffff;
-      const int slot = incl - 1 < RS_MAXBIN ? incl - 1 : RS_NOSLOT;
-      R.bin = b | (slot << 16);
-      if (f && slot < RS_MAXBIN) S.bin_id[slot] = b;
-    };
-    set_row(r0, h0, incl0, f0);
-    set_row(r1, h1, incl1, f1);
-    if (tid == 0) S.nbins = min(total, RS_MAXBIN);
   }
-  __syncthreads();
 
-  // ---- [P6b] thread 0: the staging plan (a short chain over the groups);
-  // threads 16..127: range-key runs of the columns
-  if (tid == 0) {
-    if (S.ys0 == INT32_MAX) S.ys0 = 0;
-    // the lines each group's window pushes need, copied before the group
-    // (at most RS_SR lines kept)
-    int st_lo = 1, st_hi = 0;
-    for (int g = 0; g < S.ngrp; g++) {
-      int lo = S.grange[g].x;
-      const int hi = S.grange[g].y;
-      int c_lo = 1, c_hi = 0;
-      if (lo <= hi) {
-        lo = max(lo, hi - (RS_SR - 1));
-        if (st_lo <= st_hi && lo >= st_lo && lo <= st_hi + 1) {
-          c_lo = st_hi + 1;   // extend the staged window
-          c_hi = hi;
-          st_hi = max(st_hi, hi);
-          st_lo = max(st_lo, st_hi - (RS_SR - 1));
-        } else {
-          c_lo = lo;          // restart it
-          c_hi = hi;
-          st_lo = lo;
-          st_hi = hi;
-        }
-      }
-      S.gplan[g] = make_int4(c_lo, c_hi, st_lo, st_hi);
-      // a full group whose rows all take the shared pass and whose lines are
-      // all staged and in the slave-line table takes the check-free loop
-      const int4 gw = S.gwin[g];
-      const int lo_need = (gw.y & 1) ? gw.z - 5 : gw.z + 6;
-      const bool simple = gw.x && g * RS_GR + RS_GR <= nr && gw.w == 0 && lo_need >= st_lo &&
-                          hi <= st_hi && lo_need >= S.ys0 && hi < S.ys0 + RS_NSR;
-      if (simple) S.gwin[g].y = gw.y | 2;
-    }
-  } else if (tid >= RS_NT - RS_TW) {
-    const int c = tid - (RS_NT - RS_TW);
-    if (c < cN) {
-      // runs of the range key over the item rows, by bisection of the exact
-      // per-pixel key on the pieces where the position is monotone in the
-      // row; a piece that starts with the key the previous one ended with
-      // continues its run
-      auto keyat = [&](int ri) { return rg_key(S, J, r_begin + ri, c); };
-      int ends[2] = {nr - 1, nr - 1};
-      int np = 1;
-      {
-        // x(L) = g0 + g2 P + g5 P^2 + (g1 + g4 P) L + g3 L^2: vertex in L
-        const double *g = S.crg;
-        const double P = S.col_phat[c];
-        if (g[3] != 0.0) {
-          const double Lv = -(g[1] + g[4] * P) / (2.0 * g[3]);
-          const double rv = Lv / J.invL + J.midL - (double)J.my0 - (double)r_begin;
-          if (rv > 0.0 && rv < (double)(nr - 1)) {
-            ends[0] = (int)rv;
-            np = 2;
-          }
-        }
-      }
-      int n = 0, last_key = INT32_MIN;
-      bool dense = false;
-      int a = 0;
-      for (int pc = 0; pc < np && !dense; pc++) {
-        const int bend = ends[pc];
-        int r = a, k = keyat(a);
-        const int kb = keyat(bend);
-        for (;;) {
-          if (k != last_key) {
-            if (n == RS_MAXRUN) {
-              dense = true;
-              break;
-            }
-            S.run_rk[c][n] = make_int2(r, k);
-            S.run_g[c][n] = run_terms(S, lut, xw, k);
-            n++;
-            last_key = k;
-          }
-          if (k == kb) break;   // monotone: the rest of the piece has this key
-          int lo = r, hi = bend, khi = kb;
-          while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            const int km = keyat(mid);
-            if (km == k) {
-              lo = mid;
-            } else {
-              hi = mid;
-              khi = km;
-            }
-          }
-          r = hi;
-          k = khi;
-        }
-        a = bend + 1;
-      }
-      S.run_n[c] = dense ? -1 : n;
-    }
-  }
-  __syncthreads();
-
-  // ---- [P7] stage the first group's lines; slave-line phase table; the
-  // azimuth taps of the bin table
-  {
-    const int4 p = S.gplan[0];
-    if (p.x <= p.y) stage_rows(S, J, x, xa, xin, p.x, p.y);
-  }
-  {
-    const DerampQuad refq = {S.ref_a0, S.ref_a1, S.ref_a2};
-    for (int i = tid; i < RS_NSR; i += RS_NT) {
-      const int y = S.ys0 + i;
-      const double ta = (double)(y - J.s_first_line) * J.dt;
-      RsSlaveRow sr;
-      if (kSplit) {
-        sr.f.rho = to_turns(quad_eval(refq, ta));
-        sr.f.tc = (float)(ta - tm);
-      } else {
-        sr.ta = ta;
-      }
-      S.srow[i] = sr;
-    }
-  }
-  for (int e = tid; e < S.nbins * 6; e += RS_NT) {
-    const int slot = e / 6, q = e - slot * 6;
-    const float *kl = lut.kaz + S.bin_id[slot] * kTaps + 2 * q;
-    const float a = __ldg(kl), b = __ldg(kl + 1);
-    S.bin_w[slot][q] = make_float4(a, a, b, b);
-  }
-  __syncthreads();
-
-  // ---- range-pass thread: column pair (dc, dc + 1), rows 6h .. 6h + 5 of a group
-  const int dp = tid % RS_DP, dh = tid / RS_DP;
-  const bool dthread = tid < RS_DT;
-  const int dc = 2 * dp;
-  const bool dval0 = dthread && dc < cN, dval1 = dthread && dc + 1 < cN;
-  const bool dense0 = dval0 && S.run_n[dc] < 0, dense1 = dval1 && S.run_n[dc + 1] < 0;
-  ColRun cr0, cr1;
-  cr0.ok = cr1.ok = false;
-  cr0.next = cr1.next = INT32_MAX;
-  cr0.key = cr1.key = 0;
-  cr0.m = cr1.m = 0;
-  if (dval0 && !dense0) run_load(cr0, S, J, dc, 0);
-  if (dval1 && !dense1) run_load(cr1, S, J, dc + 1, 0);
+  // range-pass columns
+  const int dc = 2 * u;
+  const bool dval = u < RS_DT && dc < cN, dtwo = dval && dc + 1 < cN;
   const bool out16 = J.out_al16 != 0;
 
-  // azimuth-pass state: the 12-line window of this ring column (line
-  // wl0 + k - 5 + j of group row k in slot (k + j) % 12) and the taps
-  float2 w[RS_GR];
+  // the 12-line window of the two ring columns
+  Dpair w[12];
 #pragma unroll
-  for (int j = 0; j < RS_GR; j++) w[j] = make_float2(0.f, 0.f);
-  float4 wz[6];
-#pragma unroll
-  for (int q = 0; q < 6; q++) wz[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-  int wz_bin = -1;
+  for (int j = 0; j < 12; j++) w[j].re = w[j].im = make_float2(0.f, 0.f);
 
-  const int ngrp = S.ngrp;
-  for (int g = 0; g < ngrp; g++) {
-    const int rg0 = g * RS_GR;            // first item row of the group
-    const int gr = min(RS_GR, nr - rg0);
-    const int4 plan = S.gplan[g];
-    const int4 gw = S.gwin[g];
-    const int pixmask = gw.w & 0xfff;     // rows without a shared pass ([A] only)
-    const int dirmask = gw.w >> 16;       // shared rows off the window's line
-    cp_async_wait_all();                  // this thread's staged lines of the group
-    // ---- [A] azimuth pass of the group's rows (the taps are loaded anew per
-    // group, so they hold no registers during [B] and [C])
-    wz_bin = -1;
-    if (gw.y & 2) {
-      // every row takes the shared pass, every line is staged
-      const int wl0 = gw.z;
-      const int ys0 = S.ys0;
-      if (gw.y & 1) {
-#pragma unroll
-        for (int j = 0; j < RS_GR - 1; j++)
-          w[j] = deramp_staged<kSplit>(S, x, wl0 - 5 + j, ys0, g2c, g1c, g0c, cq);
-      }
-#pragma unroll
-      for (int k = 0; k < RS_GR; k++) {
-        w[(k + 11) % RS_GR] = deramp_staged<kSplit>(S, x, wl0 + k + 6, ys0, g2c, g1c, g0c, cq);
-        const int bin = S.rows[rg0 + k].bin;
-        if (bin != wz_bin) {
-          load_az_taps(S, lut, bin, wz);
-          wz_bin = bin;
-        }
-        float2 a = make_float2(0.f, 0.f), b = a;
-#pragma unroll
-        for (int j = 0; j < RS_GR; j += 2) {
-          const float4 q = wz[j >> 1];
-          a = __ffma2_rn(make_float2(q.x, q.y), w[(k + j) % RS_GR], a);
-          b = __ffma2_rn(make_float2(q.z, q.w), w[(k + j + 1) % RS_GR], b);
-        }
-        S.vd[k][x] = __fadd2_rn(a, b);
-      }
-    } else if (gw.x) {
-      const int wl0 = gw.z;
-      if (gw.y & 1) {
-        // fill the window of row 0 (slots 0..10; row 0 pushes slot 11)
-#pragma unroll
-        for (int j = 0; j < RS_GR - 1; j++)
-          w[j] = deramp_at<kSplit>(S, J, x, xa, xin, wl0 - 5 + j, plan.z, plan.w, g2c, g1c,
-                                   g0c, cq);
-      }
-#pragma unroll
-      for (int k = 0; k < RS_GR; k++) {
-        if (k < gr) {
-          w[(k + 11) % RS_GR] = deramp_at<kSplit>(S, J, x, xa, xin, wl0 + k + 6, plan.z, plan.w,
-                                                  g2c, g1c, g0c, cq);
-          if (!(((pixmask | dirmask) >> k) & 1)) {
-            const int bin = S.rows[rg0 + k].bin;
-            if (bin != wz_bin) {
-              load_az_taps(S, lut, bin, wz);
-              wz_bin = bin;
-            }
-            float2 a = make_float2(0.f, 0.f), b = a;
-#pragma unroll
-            for (int j = 0; j < RS_GR; j += 2) {
-              const float4 q = wz[j >> 1];
-              a = __ffma2_rn(make_float2(q.x, q.y), w[(k + j) % RS_GR], a);
-              b = __ffma2_rn(make_float2(q.z, q.w), w[(k + j + 1) % RS_GR], b);
-            }
-            S.vd[k][x] = __fadd2_rn(a, b);
-          }
-        }
-      }
+  int want = RS_CH;                      // rows to try for a chunk
+  for (int ch0 = 0; ch0 < nr;) {
+    // ---- [P4] the azimuth entries of the chunk's rows (thread u: rows u and
+    // u + 64): counts, and a scan of both packed in one word
+    const int nrc = min(min(want, RS_CH), nr - ch0);
+    const int rb = r_begin + ch0;        // box row of the chunk's first row
+    if (u == 0) {
+      Q.nfit = nrc;
+      Q.cov = nrc;
     }
-    if (dirmask) {
-      // shared rows whose line is not the window's (the row-to-line map
-      // skipped a line inside the group): the same sum, in the same order,
-      // over lines deramped anew
+    __syncthreads();                     // also: ring_gc is written
+    {
+      int mm = 0;
 #pragma unroll 1
-      for (int m = dirmask; m; m &= m - 1) {
-        const int k = __ffs(m) - 1;
-        const RsRow &R = S.rows[rg0 + k];
-        S.vd[k][x] = az_direct<kSplit>(S, J, lut, x, xa, xin, R.L0, R.bin & 0xffff, plan.z,
-                                       plan.w, g2c, g1c, g0c, cq);
+      for (int i = 0; i < 2; i++) {
+        const int r = u + RS_ST * i;
+        if (live && r < nrc) mm |= count_entries(S, Q, J, rb + r, c0, cN) << (16 * i);
       }
-    }
-    // stage the next group's new lines; they land while [B] runs
-    if (g + 1 < ngrp) {
-      const int4 pn = S.gplan[g + 1];
-      if (pn.x <= pn.y) stage_rows(S, J, x, xa, xin, pn.x, pn.y);
+      int v = mm;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, v, o);
+        if ((t & 31) >= o) v += x;
+      }
+      if ((t & 31) == 31) Q.scan[u >> 5] = v;
+      __syncthreads();
+      if (u >= 32) v += Q.scan[0];
+      const int total0 = (Q.scan[0] + Q.scan[1]) & 0xffff;
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int r = u + RS_ST * i, m = (mm >> (16 * i)) & 0xffff;
+        const int end = ((v >> (16 * i)) & 0xffff) + (i ? total0 : 0);
+        if (r < nrc) {
+          Q.rowe[r] = (end - m) | m << 16;
+          if (end > RS_ECAP) atomicMin(&Q.nfit, r);
+        }
+      }
     }
     __syncthreads();
-
-    // ---- [B] range pass, reramp, store: 2 columns x 6 rows per thread;
-    // pixels the shared passes do not cover are listed for [C]
-    // rows without a shared pass and two-bin rows (read again here, so the
-    // group's flags hold no registers during [B])
-    const int bskip = (S.gwin[g].w & 0xfff) | ((S.gwin[g].y >> 4) & 0xfff);
-    if (dval0) {
-      run_weights(cr0, J);
-      run_weights(cr1, J);
+    const int nfit = min(S.strip[0].nfit, S.strip[1].nfit);
+    // ---- [P5] the entries, [P6] the range-key runs
 #pragma unroll 1
-      for (int kk = 0; kk < RS_HR; kk++) {
-        const int k = dh * RS_HR + kk;
-        if (k >= gr) break;
-        if ((bskip >> k) & 1) continue;     // the whole row is done in [C2] or [C]
-        const int ri = rg0 + k;
-        if (ri >= cr0.next) {
-          while (ri >= cr0.next) run_load(cr0, S, J, dc, cr0.m + 1);
-          run_weights(cr0, J);
-        }
-        if (ri >= cr1.next) {
-          while (ri >= cr1.next) run_load(cr1, S, J, dc + 1, cr1.m + 1);
-          run_weights(cr1, J);
-        }
-        const int r = r_begin + ri;       // box row
-        float2 *orow = J.out + (long)(r - J.row0) * J.out_pitch + c0 + dc;
-        const float2 *vrow = &S.vd[k][0];
-        const int xb0 = (cr0.key >> 12) - 5 - xw;
-        if (cr0.ok && cr1.ok && dval1 && (cr1.key >> 12) == (cr0.key >> 12) + 1) {
-          const RsRow R = S.rows[ri];
-          const int base = xb0 & ~1;
-          const bool odd = (xb0 & 1) != 0;
-          float2 V[14];
-          const float4 *p = reinterpret_cast<const float4 *>(vrow + base);
+    for (int r = u; r < nfit; r += RS_ST) {
+      const int re = Q.rowe[r];
+      if (re >> 16) write_entries(S, Q, J, rb + r, c0, cN, re & 0xffff);
+    }
+    if (dval) {
+#pragma unroll 1
+      for (int c = dc; c < min(dc + 2, cN); c++) build_runs(S, Q, J, rb, nfit, c0, c);
+    }
+    __syncthreads();
+    // ---- [P7] the halves; a chunk that does not end the item ends with a
+    // pair of halves, so that the window carries over
+    int n = min(nfit, min(S.strip[0].cov, S.strip[1].cov));
+    if (n < nr - ch0 && n >= 2 * RS_H) n -= n % (2 * RS_H);
+    const int nh = (n + RS_H - 1) / RS_H;
+    if (u < nh) {
+      if (live) {
+        plan_half(Q, u, n);
+      } else {
+        Q.half[u].flags = 0;
+        Q.half[u].units = 0;
+        Q.half[u].lb = 0;
+      }
+    }
+    __syncthreads();
+    int fl = 0, tb = 0;
+    if (u < nh) {
+      const RsHalf &H = Q.half[u];
+      fl = H.flags;
+      const int expect = u == 0 ? Q.prev_line
+                         : (Q.half[u - 1].flags & HG_ON) ? Q.half[u - 1].lb + RS_H : INT32_MIN;
+      if ((fl & HG_ON) && H.lb != expect) fl |= HG_FILL;
+      const int h0 = u & ~1;
+      if (h0 + 1 < nh && S.strip[0].half[h0].units + S.strip[0].half[h0 + 1].units <= RS_TU &&
+          S.strip[1].half[h0].units + S.strip[1].half[h0 + 1].units <= RS_TU) {
+        if (u & 1)
+          tb = Q.half[h0].units;
+        else
+          fl |= HG_JOIN;
+      }
+    }
+    // deramp terms of the lines the halves push
+    for (int i = u; i < nh * RS_H; i += RS_ST)
+      Q.srow[i] = line_terms<kSplit>(Q, J, Q.half[i / RS_H].lb + RS_H + i % RS_H);
+    __syncthreads();
+    if (u < nh) {
+      Q.half[u].flags = fl;
+      Q.half[u].tbase = tb;
+      if (u == nh - 1)
+        Q.prev_line = (fl & HG_ON) && !(nh & 1) ? Q.half[u].lb + RS_H : INT32_MIN;
+    }
+    __syncthreads();
 #pragma unroll
-          for (int m = 0; m < 7; m++) {
-            const float4 t = p[m];
-            V[2 * m] = make_float2(t.x, t.y);
-            V[2 * m + 1] = make_float2(t.z, t.w);
+    for (int h = 0; h < 2; h++) {
+      if (h < nh && (Q.half[h].flags & HG_ON))
+        stage_half(S, J, t, xa, h * RS_H, Q.half[h].lb + RS_H);
+      cp_async_commit();
+    }
+
+    for (int h = 0; h < nh; h++) {
+      const RsHalf H = Q.half[h];
+      const int flags = H.flags;
+      cp_async_wait<1>();                // this thread's staged lines of the half
+      // ---- [A]
+      if (flags & HG_ON) {
+        if (h & 1)
+          az_half<1, kSplit>(S, Q, J, t, u, xa, h, H, w);
+        else
+          az_half<0, kSplit>(S, Q, J, t, u, xa, h, H, w);
+        if (flags & HG_DIRECT) az_direct<kSplit>(Q, J, u, xa, H.tbase, H.pos[0], H.pos[7]);
+      }
+      if (h + 2 < nh && (Q.half[h + 2].flags & HG_ON))
+        stage_half(S, J, t, xa, (h & 1) * RS_H, Q.half[h + 2].lb + RS_H);
+      cp_async_commit();
+      if (flags & HG_JOIN) continue;
+      __syncthreads();
+
+      // ---- [B] range pass, reramp, store: 2 columns x the tile's rows
+      const int h0 = (h & 1) && (Q.half[h - 1].flags & HG_JOIN) ? h - 1 : h;
+      const int k0 = h0 * RS_H, k1 = min((h + 1) * RS_H, n);
+      const int both = Q.half[h0].flags & flags, any = Q.half[h0].flags | flags;
+      unsigned miss = 0;                 // rows the pair path leaves
+      if (dval) {
+        PairRuns P;
+        P.next = INT32_MIN;
+        float2 *orow = J.out + (long)(rb + k0 - J.row0) * J.out_pitch + c0 + dc;
+        const bool one = (both & HG_ONE) != 0;
+        int e = Q.rowe[k0] & 0xffff;     // one entry per row: consecutive
+        int un = 0;
+#pragma unroll 1
+        for (int k = k0; k < k1; k++, orow += J.out_pitch, e++, un += RS_UN) {
+          if (k >= P.next) load_runs(P, Q, J, dc, dtwo, k);
+          bool fast = P.pair;
+          if (!one) {
+            const int re = Q.rowe[k], ne = re >> 16;
+            if (ne == 0) continue;       // a per-pixel row
+            e = re & 0xffff;
+            int4 M = Q.eM[e];
+            for (int q = 1; q < ne && !(dc >= ((M.y >> 16) & 0xff) && dc < ((M.y >> 24) & 0xff));
+                 q++)
+              M = Q.eM[++e];
+            fast = fast && dc + 1 < ((M.y >> 24) & 0xff) && P.unit >= ((M.w >> 16) & 0xff) &&
+                   P.unit + 6 <= ((M.w >> 24) & 0xff) && ((M.y >> 12) & 3) == REG_IN;
+            un = (k >= h * RS_H ? H.tbase : 0) + (short)(M.w & 0xffff);
           }
-          float2 s0, s1;
-          range_pair(cr0, cr1, V, odd, s0, s1);
-          const float2 o0 = cmul_conj_turns(s0, run_phase(R, cr0));
-          const float2 o1 = cmul_conj_turns(s1, run_phase(R, cr1));
-          if (out16) {
-            *reinterpret_cast<float4 *>(orow) = make_float4(o0.x, o0.y, o1.x, o1.y);
+          if (!fast) {
+            miss |= 1u << (k - k0);
+            continue;
+          }
+          const float4 *U = &Q.tile[un + P.unit];
+          float4 V[7];
+#pragma unroll
+          for (int m = 0; m < 7; m++) V[m] = U[m];
+          const float4 A = Q.eA[e];
+          const float R0 = __int_as_float(Q.eM[e].z);
+          const float2 f =
+              turns_to_rad2(make_float2(run_phase(A, R0, P.gx), run_phase(A, R0, P.gy)));
+          float2 vx, vy;
+          if (P.odd) {
+            vx = rg_sum<7>(P.wo, V);
+            vy = rg_sum<6>(P.we, V + 1);
           } else {
-            orow[0] = o0;
-            orow[1] = o1;
+            vx = rg_sum<6>(P.we, V);
+            vy = rg_sum<7>(P.wo, V);
           }
-        } else {
-          // per column, from the run key: outside the slave box 0, at its
-          // edge the nearest sample, inside the window the tile's range
-          // pass, else [C]
-          const RsRow R = S.rows[ri];
-#pragma unroll
-          for (int cc = 0; cc < 2; cc++) {
-            if (cc == 1 && !dval1) break;
-            const ColRun &cr = cc ? cr1 : cr0;
-            const bool dense = cc ? dense1 : dense0;
-            const int p0 = cr.key >> 12;
-            if (dense) {
-              const int e = atomicAdd(&S.gen_d[g], 1);
-              S.gen[RS_GR * RS_TW - 1 - e] = (unsigned short)(k * 128 + dc + cc);
-            } else if (p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7 && !cr.ok) {
-              const int e = atomicAdd(&S.gen_n[g], 1);
-              S.gen[e] = (unsigned short)(k * 128 + dc + cc);
-            } else if (cr.ok) {
-              orow[cc] = cmul_conj_turns(range_single(vrow, p0 - 5 - xw, cr), run_phase(R, cr));
-            } else if (p0 < J.sx0 || p0 > J.sx1) {
-              orow[cc] = make_float2(0.f, 0.f);
-            } else {
-              const short2 sv = J.slave[(long)(R.L0 - J.sy0) * J.slave_pitch + (p0 - J.sx0)];
-              orow[cc] = make_float2((float)sv.x, (float)sv.y);
-            }
+          vx = cmul_conj(vx, f.x);
+          vy = cmul_conj(vy, f.y);
+          if (out16) {
+            *reinterpret_cast<float4 *>(orow) = make_float4(vx.x, vx.y, vy.x, vy.y);
+          } else {
+            orow[0] = vx;
+            orow[1] = vy;
           }
         }
       }
-    }
-    __syncthreads();
+      {
+        const unsigned b = __ballot_sync(0xffffffffu, miss != 0);
+        if (miss) Q.miss[u] = (unsigned short)miss;
+        if ((t & 31) == 0) Q.missb[u >> 5] = b;
+      }
+      __syncthreads();
 
-    // ---- [C1] pixels of shared rows in columns without a run table, all
-    // threads: the range key and its run terms per pixel, then the range
-    // pass over the tile as in [B]
-    {
-      const int nd = S.gen_d[g];
-      if (nd > 0) {
-        for (int u = tid; u < nd; u += RS_NT) {
-          const int code = S.gen[RS_GR * RS_TW - 1 - u];
-          const int k = code >> 7, c = code & 127;
-          const int r = r_begin + rg0 + k;
-          J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] =
-              pixel_keyed(S, J, S.rows[rg0 + k], &S.vd[k][0], r, c);
-        }
+      // ---- [C] the pixels the pair path left, then per-pixel rows and the
+      // pixels left to the per-pixel path
+      if (S.strip[0].missb[0] | S.strip[0].missb[1] | S.strip[1].missb[0] | S.strip[1].missb[1]) {
+        slow_pixels(Q, J, u, k0, k1 - k0, h * RS_H, H.tbase, cN,
+                    J.out + (long)(rb + k0 - J.row0) * J.out_pitch + c0);
         __syncthreads();
+      }
+      if (Q.gen_any || (any & HG_PIX)) pixel_pass(S, Q, J, u, k0, rb + k0, k1 - k0, c0, cN);
+      if (S.strip[0].gen_any | S.strip[1].gen_any) {
+        __syncthreads();
+        if (u < 2 * RS_H * 4) (&Q.gen[0][0])[u] = 0u;
+        if (u == 0) Q.gen_any = 0;
       }
     }
-
-    // ---- [C2] two-bin rows, all threads, by the keyed path: the columns of
-    // the first bin from the tile; then the rows' azimuth sums with the
-    // second bin, over lines deramped anew from HBM (the line ring already
-    // holds the next group's lines), into their tile rows, and the row terms
-    // of that key; then the columns of the second bin
-    {
-      const int two = (S.gwin[g].y >> 4) & 0xfff;
-      if (two) {
-#pragma unroll 1
-        for (int m = two; m; m &= m - 1) {
-          const int k = __ffs(m) - 1;
-          const int md = S.rows[rg0 + k].mode;
-          const int lo = (md >> 8) & 0xff, hi = (md >> 16) & 0xff;
-          const int r = r_begin + rg0 + k;
-          for (int c = tid; c < cN; c += RS_NT)
-            if (c < lo || c >= hi)
-              J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] =
-                  pixel_keyed(S, J, S.rows[rg0 + k], &S.vd[k][0], r, c);
-        }
-        __syncthreads();
-#pragma unroll 1
-        for (int m = two; m; m &= m - 1) {
-          const int k = __ffs(m) - 1;
-          const RsRow &R = S.rows[rg0 + k];
-          S.vd[k][x] = az_direct<kSplit>(S, J, lut, x, xa, xin, R.L0, (R.bin & 0xffff) + 1, 1,
-                                         0, g2c, g1c, g0c, cq);
-        }
-        if (tid < RS_GR && ((two >> tid) & 1)) {
-          const RsRow &R = S.rows[rg0 + tid];
-          RsRow R2 = R;
-          row_terms(S, J, lut, R.L0, (R.bin & 0xffff) + 1, R2);
-          S.r2[tid] = R2;
-        }
-        __syncthreads();
-#pragma unroll 1
-        for (int m = two; m; m &= m - 1) {
-          const int k = __ffs(m) - 1;
-          const int md = S.rows[rg0 + k].mode;
-          const int r = r_begin + rg0 + k;
-          for (int c = ((md >> 8) & 0xff) + tid; c < ((md >> 16) & 0xff); c += RS_NT)
-            J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] =
-                pixel_keyed(S, J, S.r2[k], &S.vd[k][0], r, c);
-        }
-        __syncthreads();
-      }
-    }
-
-    // ---- [C] per-pixel path, all threads: the rows without a shared pass,
-    // then the listed pixels
-    {
-      const int pixmask = S.gwin[g].w & 0xfff;
-      const int npr = __popc(pixmask);
-      const int nrow_units = npr * cN;
-      const int total = nrow_units + S.gen_n[g];
-      // the tile is free after [B]: each thread parks its column of the
-      // window there while the per-pixel path runs, so the window holds no
-      // registers during it
-      if (total > 0) {
-#pragma unroll
-        for (int j = 0; j < RS_GR; j++) S.vd[j][x] = w[j];
-      }
-      for (int u = tid; u < total; u += RS_NT) {
-        int k, c;
-        if (u < nrow_units) {
-          int nth = u / cN;
-          c = u - nth * cN;
-          int m = pixmask;
-          while (nth-- > 0) m &= m - 1;   // drop the lower set bits
-          k = __ffs(m) - 1;
-        } else {
-          const int code = S.gen[u - nrow_units];
-          k = code >> 7;
-          c = code & 127;
-        }
-        const int r = r_begin + rg0 + k;
-        J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] = pixel_generic(S, J, r, c);
-      }
-      if (total > 0) {
-#pragma unroll
-        for (int j = 0; j < RS_GR; j++) w[j] = S.vd[j][x];
-      }
-    }
+    cp_async_wait<0>();
+    ch0 += n;
+    want = max(2 * RS_H, n + n);         // shrink to what the tables held, then grow
+    want = (want + 2 * RS_H - 1) / (2 * RS_H) * (2 * RS_H);
+    __syncthreads();   // the next chunk's (or item's) prologue rewrites the tables
   }
-  __syncthreads();   // the next item's prologue rewrites the tables
 }
 
 template <bool kSplit>
 __global__ void __launch_bounds__(RS_NT, 3)
     resample_kernel(const __grid_constant__ RsBatch B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  RsShared &S = *reinterpret_cast<RsShared *>(smem_raw);
+  RsShared<kSplit> &S = *reinterpret_cast<RsShared<kSplit> *>(smem_raw);
   // one work item per CTA, or (persistent) items from the queue until it
   // is empty; a single call site keeps one inlined copy of the item code
   int item = blockIdx.x;
@@ -1351,9 +1390,10 @@ __global__ void __launch_bounds__(RS_NT, 3)
 }
 
 // ---------------------------------------------------------------- host
+// All tables of one LUT in one device allocation.
 struct LutDev {
-  float *kaz = nullptr, *krg = nullptr, *sp1 = nullptr;
-  float4 *krg2 = nullptr;
+  void *mem = nullptr;
+  LutPtrs p{};
 };
 
 }  // namespace tops
@@ -1366,46 +1406,47 @@ using namespace tops;
 
 extern "C" int tops_lut_create(const float *kaz, const float *krg, tops_lut_dev **out) {
   if (!kaz || !krg || !out) return TOPS_E_INVALID;
-  tops_lut_dev *L = new tops_lut_dev();
-  std::vector<float> sp1(kLutBins), krg2((size_t)kLutBins * kTaps * 2);
-  for (int b = 0; b < kLutBins; b++) {
+  // device layout: kaz2 [2048][24] | krgo [2048][16] | kaz [2048][12] |
+  // krg [2048][12] | sp1 [2048]
+  const size_t nb = kLutBins;
+  const size_t o_krgo = nb * 24, o_kaz = o_krgo + nb * 16, o_krg = o_kaz + nb * kTaps,
+               o_sp1 = o_krg + nb * kTaps, total = (o_sp1 + nb) * sizeof(float);
+  std::vector<float> h(o_sp1 + nb, 0.f);
+  float *kaz2 = h.data(), *krgo = kaz2 + o_krgo, *sp1 = kaz2 + o_sp1;
+  std::copy(kaz, kaz + nb * kTaps, kaz2 + o_kaz);
+  std::copy(krg, krg + nb * kTaps, kaz2 + o_krg);
+  for (size_t b = 0; b < nb; b++) {
     double s = 0.0;
     for (int i = 0; i < kTaps; i++) {
       s += (double)krg[b * kTaps + i];
-      krg2[(size_t)b * kTaps * 2 + 2 * i] = krg[b * kTaps + i];
-      krg2[(size_t)b * kTaps * 2 + 2 * i + 1] = krg[b * kTaps + i];
+      kaz2[b * 24 + 2 * i] = kaz2[b * 24 + 2 * i + 1] = kaz[b * kTaps + i];
+      krgo[b * 16 + 1 + i] = krg[b * kTaps + i];
     }
     sp1[b] = (float)(s - 1.0);
   }
-  size_t nb = sizeof(float) * kLutBins * kTaps;
-  cudaError_t e = cudaMalloc(&L->d.kaz, nb);
-  if (e == cudaSuccess) e = cudaMalloc(&L->d.krg, nb);
-  if (e == cudaSuccess) e = cudaMalloc(&L->d.krg2, 2 * nb);
-  if (e == cudaSuccess) e = cudaMalloc(&L->d.sp1, sizeof(float) * kLutBins);
-  if (e == cudaSuccess) e = cudaMemcpy(L->d.kaz, kaz, nb, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(L->d.krg, krg, nb, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(L->d.krg2, krg2.data(), 2 * nb, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess)
-    e = cudaMemcpy(L->d.sp1, sp1.data(), sizeof(float) * kLutBins, cudaMemcpyHostToDevice);
+  tops_lut_dev *L = new tops_lut_dev();
+  cudaError_t e = cudaMalloc(&L->d.mem, total);
+  if (e == cudaSuccess) e = cudaMemcpy(L->d.mem, h.data(), total, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     set_cuda_error(e);
-    cudaFree(L->d.kaz);
-    cudaFree(L->d.krg);
-    cudaFree(L->d.krg2);
-    cudaFree(L->d.sp1);
+    (void)cudaGetLastError();
+    cudaFree(L->d.mem);
     delete L;
     return e == cudaErrorMemoryAllocation ? TOPS_E_NOMEM : TOPS_E_CUDA;
   }
+  const float *m = static_cast<const float *>(L->d.mem);
+  L->d.p.kaz2 = reinterpret_cast<const float4 *>(m);
+  L->d.p.krgo = reinterpret_cast<const float4 *>(m + o_krgo);
+  L->d.p.kaz = m + o_kaz;
+  L->d.p.krg = m + o_krg;
+  L->d.p.sp1 = m + o_sp1;
   *out = L;
   return TOPS_OK;
 }
 
 extern "C" int tops_lut_destroy(tops_lut_dev *L) {
   if (!L) return TOPS_OK;
-  cudaFree(L->d.kaz);
-  cudaFree(L->d.krg);
-  cudaFree(L->d.krg2);
-  cudaFree(L->d.sp1);
+  cudaFree(L->d.mem);
   delete L;
   return TOPS_OK;
 }
@@ -1458,9 +1499,9 @@ int fill_resample_job(const tops_resample_job &u, ResampleJob &J) {
   J.midL = 0.5 * ((double)u.mbox[2] + (double)u.mbox[3]);
   J.invL = 1.0 / (0.25 * ((double)u.mbox[3] - (double)u.mbox[2]));
   const int mpix = u.mbox[1] - u.mbox[0] + 1;
-  J.strips = (mpix + RS_TW - 1) / RS_TW;
-  J.seg_rows = RS_SEG;
-  J.segs = (J.nrows + RS_SEG - 1) / RS_SEG;
+  J.strips = (mpix + RS_NS * RS_TW - 1) / (RS_NS * RS_TW);   // strip pairs
+  J.seg_rows = RS_MAXSEG;
+  J.segs = (J.nrows + RS_MAXSEG - 1) / RS_MAXSEG;
   return TOPS_OK;
 }
 
@@ -1475,32 +1516,35 @@ static int launch_resample_t(const ResampleJob *jobs, int njobs, const TileCfg &
   const int s0 = once_per_device(
       setup, dev,
       [&](int &v) -> int {
-        TOPS_CUDA_TRY(cudaFuncSetAttribute(resample_kernel<kSplit>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(RsShared)));
+        TOPS_CUDA_TRY(cudaFuncSetAttribute(
+            resample_kernel<kSplit>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RsShared<kSplit>)));
         int per_sm = 0, sms = 0;
-        TOPS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, resample_kernel<kSplit>, RS_NT, sizeof(RsShared)));
+        TOPS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resample_kernel<kSplit>, RS_NT,
+                                                                    sizeof(RsShared<kSplit>)));
         TOPS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         v = per_sm * sms;
         return TOPS_OK;
       },
       &resident);
   if (s0 != TOPS_OK) return s0;
-  if (cfg.seg_rows < 0 || cfg.seg_rows > RS_MAXSEG || (cfg.seg_rows && cfg.seg_rows < RS_GR))
+  if (cfg.seg_rows < 0 || cfg.seg_rows > RS_MAXSEG || (cfg.seg_rows && cfg.seg_rows < 2 * RS_H))
     return TOPS_E_INVALID;
-  // default segment rows: the longest (least prologue per output row) that
-  // still gives every SM two waves of items; small launches (a narrow burst,
-  // a single burst) take shorter segments.  Outputs do not depend on it.
+  // default segment rows: the fewest row times of the last CTA to finish,
+  // waves x (rows + the prologue and the window's fill, worth about 24 rows).
+  // Outputs do not depend on it.
   int seg_rows = cfg.seg_rows;
   if (!seg_rows) {
-    static const int kSegs[] = {RS_SEG, 168, 120, 84};
+    static const int kSegs[] = {252, 204, 168, 144, 120, 96, 84, 72, 60, 48, 36, 24};
+    long best = 0;
     for (int sr : kSegs) {
       long items = 0;
       for (int j = 0; j < njobs; j++)
         items += (long)jobs[j].strips * ((jobs[j].nrows + sr - 1) / sr);
-      seg_rows = sr;
-      if (items >= 2L * resident) break;
+      const long cost = (items + resident - 1) / resident * (sr + 24);
+      if (!seg_rows || cost < best) {
+        best = cost;
+        seg_rows = sr;
+      }
     }
   }
   for (int j0 = 0, k = 0; j0 < njobs; j0 += RS_MAXJOBS, k++) {
@@ -1524,14 +1568,14 @@ static int launch_resample_t(const ResampleJob *jobs, int njobs, const TileCfg &
       TOPS_CUDA_TRY(cudaMemsetAsync(B.counter, 0, sizeof(int), st));
       grid = min(items, cfg.grid > 0 ? cfg.grid : resident);
     }
-    resample_kernel<kSplit><<<grid, RS_NT, sizeof(RsShared), st>>>(B);
+    resample_kernel<kSplit><<<grid, RS_NT, sizeof(RsShared<kSplit>), st>>>(B);
     TOPS_CUDA_TRY(cudaGetLastError());
   }
   return TOPS_OK;
 }
 
-int launch_resample(const ResampleJob *jobs, int njobs, int precision, const TileCfg &cfg,
-                    cudaStream_t st) {
+static int launch_resample(const ResampleJob *jobs, int njobs, int precision, const TileCfg &cfg,
+                           cudaStream_t st) {
   if (precision == TOPS_PREC_FP64) return launch_resample_t<false>(jobs, njobs, cfg, st);
   if (precision == TOPS_PREC_SPLIT) return launch_resample_t<true>(jobs, njobs, cfg, st);
   return TOPS_E_INVALID;
@@ -1545,8 +1589,7 @@ int resample_launch_multi(const tops_lut_dev *const *luts, const tops_resample_j
     if (!luts[j]) return TOPS_E_INVALID;
     int s = fill_resample_job(jobs[j], J[j]);
     if (s != TOPS_OK) return s;
-    const LutDev &L = luts[j]->d;
-    J[j].lut = LutPtrs{L.kaz, L.krg, L.krg2, L.sp1};
+    J[j].lut = luts[j]->d.p;
   }
   return launch_resample(J.data(), njobs, precision, cfg, st);
 }
