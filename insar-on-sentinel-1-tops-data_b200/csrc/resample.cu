@@ -55,11 +55,14 @@
 // What bounds it: instruction issue with 12 warps per SM (168 registers and 72
 // KB of shared memory per CTA allow 3 CTAs).  Two columns per thread share a
 // line's terms, a row's taps and the bookkeeping, and fill the FP32x2 lanes:
-// 105 instead of 158 thread instructions per pixel on a burst of 1500 x 21000
-// (one entry per row, nearly no key changes), 0.463 -> 0.351 ms (816 -> 1077
-// GB/s of 12 bytes per pixel).  Rows whose strip spans several azimuth keys
+// 117 instead of 158 thread instructions per pixel on a burst of 1500 x 21000
+// (one entry per row, nearly no key changes), 0.463 -> 0.351 ms; the range
+// runs kept over a chunk's tiles instead of loaded per tile, and a shorter
+// prologue (entries found once, columns of one key and plain halves without a
+// search): 0.351 -> 0.305 ms (816 -> 1239 GB/s of 12 bytes per pixel in all).
+// Rows whose strip spans several azimuth keys
 // took a per-pixel path from HBM before, columns with many range keys a keyed
-// one: a burst of 1539 x 10867 of crossing orbits 3.92 -> 0.87 ms.
+// one: a burst of 1539 x 10867 of crossing orbits 3.92 -> 0.79 ms.
 //
 // Which path a pixel takes, and the order of its sums, depend on its row, its
 // column and its strip only, never on the work item, so a job that produces a
@@ -101,11 +104,12 @@ constexpr int RS_NH = RS_CH / RS_H;        // halves per chunk
 constexpr int RS_ECAP = 136;               // entries per chunk and strip
 constexpr int RS_TU = 2 * RS_H * RS_UN;    // tile units per strip
 constexpr int RS_ROWU = RS_TU / RS_H;      // most tile units of a row
-constexpr int RS_MAXKEY = 16;              // most entries of a row
+constexpr int RS_MAXKEY = 12;              // most entries of a row
 constexpr int RS_MAXJOBS = 32;
 static_assert(RS_UN == RS_ST, "one unit per thread in the azimuth pass");
 static_assert(RS_DT <= RS_ST && RS_CH <= 2 * RS_ST && RS_CH % (2 * RS_H) == 0 &&
-                  RS_MAXKEY <= RS_ECAP && RS_TW < 128 && RS_NH <= RS_ST,
+                  RS_MAXKEY <= RS_ECAP && RS_TW < 128 && RS_NH <= RS_ST &&
+                  RS_CH * RS_MAXKEY * 8 <= RS_TU * 16,
               "thread mappings and table fields assume these sizes");
 
 enum : int { REG_OUT = 0, REG_EDGE = 1, REG_IN = 2 };
@@ -157,7 +161,7 @@ struct __align__(16) RsStrip {
   static constexpr int kRuns = kSplit ? 3 : 2;   // range-key runs per column and chunk
   float4 tile[RS_TU];                 // azimuth-interpolated units
   float4 run_g[kRuns][RS_TW];         // per run: (sp, G2, G1, G0)
-  int2 run_rk[kRuns][RS_TW];          // (first chunk row, key = p0 * 4096 + bin)
+  int2 run_rk[kRuns][RS_TW];          // (chunk row of the next run, key = p0 * 4096 + bin)
   float4 ring_gc[RS_FW];              // per ring column (g2, g1, g0, 0)
   float4 eA[RS_ECAP];                 // entries: reramp terms (rho, psif, R2, R1)
   int4 eM[RS_ECAP];                   // (L0, bin | region << 12 | c_lo << 16 | c_hi << 24, R0,
@@ -168,7 +172,6 @@ struct __align__(16) RsStrip {
   unsigned gen[2 * RS_H][4];          // pixels of the tile's rows left to the per-pixel path
   unsigned missb[RS_ST / 32];         // pairs with rows the pair path left, and the rows
   unsigned short miss[RS_ST];
-  unsigned char run_n[RS_TW];
   int scan[RS_ST / 32];
   RsRing<kSplit> ring;
   double ref_a0, ref_a1, ref_a2, tm;  // reference column's phase, burst centre time
@@ -307,12 +310,16 @@ __device__ __forceinline__ void quad_span(double a, double b, double c, double p
   hi += 1e-9;
 }
 
-// Range key (p0 * 4096 + bin) of pixel (box row r, box column c).
+// Range key (p0 * 4096 + bin) of a row's terms (A, B) and a column's P, and of
+// pixel (box row r, P).
+__device__ __forceinline__ int rg_key_at(double A, double B, double c5, double P) {
+  int p0, b;
+  split_pos(pix_pos(A, B, c5, P), p0, b);
+  return min(max(p0, -(1 << 19)), (1 << 19) - 1) * 4096 + b;
+}
 __device__ __forceinline__ int rg_key(const double *crg, const ResampleJob &J, int r, double P) {
   const double L = row_L(J, r);
-  int p0, b;
-  split_pos(pix_pos(row_a(crg, L), row_b(crg, L), crg[5], P), p0, b);
-  return min(max(p0, -(1 << 19)), (1 << 19) - 1) * 4096 + b;
+  return rg_key_at(row_a(crg, L), row_b(crg, L), crg[5], P);
 }
 
 // ---------------------------------------------------- HBM slow path
@@ -549,6 +556,7 @@ __device__ __forceinline__ void az_half(RsShared<kSplit> &S, RsStrip<kSplit> &Q,
   const RsLut &lut = J.lut;
   const RsSlaveRow *sr = &Q.srow[h * RS_H];
   if (H.flags & HG_FILL) az_fill<HALF, kSplit>(Q, J, xa, H.lb, R, w);
+  cp_async_wait<1>();                    // this thread's staged lines of the half
   if (H.flags & HG_PLAIN) {
     float4 wz[6];
     az_taps(wz, lut, Q.eM[H.pos[0]].y & 0xfff);
@@ -643,11 +651,13 @@ __device__ __forceinline__ float run_phase(float4 A, float R0, float4 g) {
   return fmaf(g.x, A.y, A.x) + fmaf(g.y, A.z, fmaf(g.z, A.w, g.w * R0));
 }
 
-// The current runs of a thread's two output columns.
+// The current runs of a thread's two output columns, kept over a chunk's tiles.
 struct PairRuns {
   float4 gx, gy;
   float4 we[3], wo[4];   // pair: taps of the even-aligned and of the odd column
-  int next;              // chunk row of the next change
+  int keyx, keyy;
+  int nextx, nexty;      // chunk row of each column's next run
+  int mx, my;            // run numbers (-1: none yet)
   int unit;              // pair: first tile unit of its 14 samples
   bool pair, odd;        // pair: both columns in the ring, adjacent samples;
                          // odd: the first column is the odd-aligned one
@@ -660,32 +670,68 @@ __device__ __forceinline__ int ring_col(int xo, const ResampleJob &J, int key) {
   return (p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7 && xb >= 0 && xb + 13 < RS_FW) ? xb : -1;
 }
 
+// Moves the runs on to chunk row `row`.
 template <bool kSplit>
-__device__ __forceinline__ void load_runs(PairRuns &P, const RsStrip<kSplit> &Q,
+__device__ __forceinline__ void next_runs(PairRuns &P, const RsStrip<kSplit> &Q,
                                           const ResampleJob &J, int c, bool two, int row) {
-  int next = INT32_MAX, n = Q.run_n[c], m = 0;
-  while (m + 1 < n && Q.run_rk[m + 1][c].x <= row) m++;
-  if (m + 1 < n) next = Q.run_rk[m + 1][c].x;
-  P.gx = Q.run_g[m][c];
-  const int keyx = Q.run_rk[m][c].y;
-  P.pair = false;
-  if (two) {
-    n = Q.run_n[c + 1];
-    m = 0;
-    while (m + 1 < n && Q.run_rk[m + 1][c + 1].x <= row) m++;
-    if (m + 1 < n) next = min(next, Q.run_rk[m + 1][c + 1].x);
-    P.gy = Q.run_g[m][c + 1];
-    const int keyy = Q.run_rk[m][c + 1].y;
-    const int xb = ring_col(Q.xo, J, keyx);
-    if (xb >= 0 && ring_col(Q.xo, J, keyy) == xb + 1) {
-      P.pair = true;
-      P.odd = (xb & 1) != 0;
-      P.unit = xb >> 1;
-      taps_even(P.we, J.lut, (P.odd ? keyy : keyx) & 4095);
-      taps_odd(P.wo, J.lut, (P.odd ? keyx : keyy) & 4095);
-    }
+  while (row >= P.nextx) {
+    P.mx++;
+    const int2 rk = Q.run_rk[P.mx][c];
+    P.gx = Q.run_g[P.mx][c];
+    P.nextx = rk.x;
+    P.keyx = rk.y;
   }
-  P.next = next;
+  while (row >= P.nexty) {
+    P.my++;
+    const int2 rk = Q.run_rk[P.my][c + 1];
+    P.gy = Q.run_g[P.my][c + 1];
+    P.nexty = rk.x;
+    P.keyy = rk.y;
+  }
+  const int xb = ring_col(Q.xo, J, P.keyx);
+  P.pair = two && xb >= 0 && ring_col(Q.xo, J, P.keyy) == xb + 1;
+  if (P.pair) {
+    P.odd = (xb & 1) != 0;
+    P.unit = xb >> 1;
+    taps_even(P.we, J.lut, (P.odd ? P.keyy : P.keyx) & 4095);
+    taps_odd(P.wo, J.lut, (P.odd ? P.keyx : P.keyy) & 4095);
+  }
+}
+
+__device__ __forceinline__ void store_pair(float2 *o, bool out16, float2 a, float2 b) {
+  if (out16) {
+    *reinterpret_cast<float4 *>(o) = make_float4(a.x, a.y, b.x, b.y);
+  } else {
+    o[0] = a;
+    o[1] = b;
+  }
+}
+// Both columns of a pair in one row: U the units of its 14 samples, A and R0
+// the entry's reramp terms.
+__device__ __forceinline__ void pair_row(const PairRuns &P, const float4 *U, float4 A, float R0,
+                                         float2 *o, bool out16) {
+  float4 V[7];
+#pragma unroll
+  for (int m = 0; m < 7; m++) V[m] = U[m];
+  const float2 f = turns_to_rad2(make_float2(run_phase(A, R0, P.gx), run_phase(A, R0, P.gy)));
+  float2 vx, vy;
+  if (P.odd) {
+    vx = rg_sum<7>(P.wo, V);
+    vy = rg_sum<6>(P.we, V + 1);
+  } else {
+    vx = rg_sum<6>(P.we, V);
+    vy = rg_sum<7>(P.wo, V);
+  }
+  store_pair(o, out16, cmul_conj(vx, f.x), cmul_conj(vy, f.y));
+}
+
+// A pixel off the slave box's interior: 0 outside, the nearest sample at the
+// edge.
+__device__ __forceinline__ float2 border_pixel(const ResampleJob &J, int reg, int L0, int p0) {
+  reg = min(reg, region_1d(p0, J.sx0, J.sx1));
+  if (reg == REG_OUT) return make_float2(0.f, 0.f);
+  const short2 sv = J.slave[(long)(L0 - J.sy0) * J.slave_pitch + (p0 - J.sx0)];
+  return make_float2((float)sv.x, (float)sv.y);
 }
 
 // One pixel (chunk row k, strip column c) of a shared row outside the pair path.
@@ -699,18 +745,13 @@ __device__ __forceinline__ void pixel_shared(RsStrip<kSplit> &Q, const ResampleJ
     if (c >= ((z >> 16) & 0xff) && c < ((z >> 24) & 0xff)) break;
   }
   int m = 0;
-  while (m + 1 < Q.run_n[c] && Q.run_rk[m + 1][c].x <= k) m++;
+  while (k >= Q.run_rk[m][c].x) m++;
   const int key = Q.run_rk[m][c].y;
   const int4 M = Q.eM[e];
   const int p0 = key >> 12;
-  const int reg = min((M.y >> 12) & 3, region_1d(p0, J.sx0, J.sx1));
-  if (reg == REG_OUT) {
-    *out = make_float2(0.f, 0.f);
-    return;
-  }
-  if (reg == REG_EDGE) {
-    const short2 sv = J.slave[(long)(M.x - J.sy0) * J.slave_pitch + (p0 - J.sx0)];
-    *out = make_float2((float)sv.x, (float)sv.y);
+  const int reg = (M.y >> 12) & 3;
+  if (min(reg, region_1d(p0, J.sx0, J.sx1)) != REG_IN) {
+    *out = border_pixel(J, reg, M.x, p0);
     return;
   }
   const int xb = ring_col(Q.xo, J, key);
@@ -849,12 +890,15 @@ __device__ __forceinline__ void entry_units(const RsStrip<kSplit> &Q, int c_lo, 
   uhi = min(max(c_hi - 1 + Q.dhi + 13, 0), RS_FW - 1) >> 1;
 }
 
-// [P4] Counts the entries of a row (0: a per-pixel row).
+// [P4] A row's entries, to `out` (at most RS_MAXKEY): (line, bin | region << 12 |
+// c_lo << 16 | c_hi << 24).  Returns their number, 0 for a per-pixel row.
 template <bool kSplit>
-__device__ __forceinline__ int count_entries(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
-                                             const ResampleJob &J, int r, int c0, int cN) {
+__device__ __forceinline__ int find_entries(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
+                                            const ResampleJob &J, int r, int c0, int cN,
+                                            int2 *out) {
   int m = 0, units = 0;
-  walk_row(S, J, r, c0, cN, [&](int reg, int, int, int c_lo, int c_hi) -> bool {
+  walk_row(S, J, r, c0, cN, [&](int reg, int L0, int bin, int c_lo, int c_hi) -> bool {
+    if (m < RS_MAXKEY) out[m] = make_int2(L0, bin | reg << 12 | c_lo << 16 | c_hi << 24);
     m++;
     if (reg == REG_IN) {
       int ulo, uhi;
@@ -875,10 +919,11 @@ __device__ __forceinline__ float4 row_terms(const RsStrip<kSplit> &Q, const Resa
   const DerampQuad refq = {Q.ref_a0, Q.ref_a1, Q.ref_a2};
   const float *kl = J.lut.kaz + bin * kTaps;
   double psi = 0.0, m0 = 0.0, m1 = 0.0, m2 = 0.0;
-#pragma unroll 4
+  const double n0 = (double)(L0 - 5 - J.s_first_line);
+#pragma unroll
   for (int j = 0; j < kTaps; j++) {
     const double w = (double)__ldg(kl + j), u = (double)(j - 5);
-    const double ta = (double)(L0 - 5 + j - J.s_first_line) * J.dt;
+    const double ta = (n0 + (double)j) * J.dt;
     psi = fma(w, quad_eval(refq, ta), psi);
     m0 += w;
     m1 = fma(w, u, m1);
@@ -892,21 +937,16 @@ __device__ __forceinline__ float4 row_terms(const RsStrip<kSplit> &Q, const Resa
                      (float)(m0 * tc0 + dt * m1));
 }
 
-// [P5] Writes a row's entries from entry e on, with the reramp terms of their
-// keys.
+// [P5] An entry, with the reramp terms of its key.
 template <bool kSplit>
-__device__ __forceinline__ void write_entries(const RsShared<kSplit> &S, RsStrip<kSplit> &Q,
-                                              const ResampleJob &J, int r, int c0, int cN, int e) {
-  walk_row(S, J, r, c0, cN, [&](int reg, int L0, int bin, int c_lo, int c_hi) -> bool {
-    int ulo = 0, uhi = RS_UN - 1;
-    if (c_hi - c_lo < cN) entry_units(Q, c_lo, c_hi, ulo, uhi);
-    float R0 = 0.f;
-    if (reg == REG_IN) Q.eA[e] = row_terms(Q, J, L0, bin, R0);
-    Q.eM[e] = make_int4(L0, bin | reg << 12 | c_lo << 16 | c_hi << 24, __float_as_int(R0),
-                        ulo << 16 | uhi << 24);
-    e++;
-    return true;
-  });
+__device__ __forceinline__ void write_entry(RsStrip<kSplit> &Q, const ResampleJob &J, int2 E,
+                                            int cN, int e) {
+  const int c_lo = (E.y >> 16) & 0xff, c_hi = (E.y >> 24) & 0xff;
+  int ulo = 0, uhi = RS_UN - 1;
+  if (c_hi - c_lo < cN) entry_units(Q, c_lo, c_hi, ulo, uhi);
+  float R0 = 0.f;
+  if (((E.y >> 12) & 15) == REG_IN) Q.eA[e] = row_terms(Q, J, E.x, E.y & 0xfff, R0);
+  Q.eM[e] = make_int4(E.x, E.y, __float_as_int(R0), ulo << 16 | uhi << 24);
 }
 
 // Phase terms of a range-key run: (sp, G2, G1, G0) with Gk = sum_i kRg[i]
@@ -935,46 +975,47 @@ __device__ __forceinline__ float4 run_terms(const RsStrip<kSplit> &Q, const RsLu
 }
 
 // [P6] The runs of column c's range key over chunk rows [0, n) (box rows rb
-// ...), by bisection of the exact per-pixel key on the pieces where the
-// position is monotone in the row; rows from the first change that does not
-// fit the table on are left to the next chunk (Q.cov).
+// ...).  Most columns hold one key: when the position is monotone over the
+// rows and both ends agree (k0, k1 from the caller).  Else by bisection of the
+// exact per-pixel key on the pieces where the position is monotone in the row;
+// rows from the first change that does not fit the table on are left to the
+// next chunk (Q.cov).
 template <bool kSplit>
 __device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kSplit> &Q,
-                                           const ResampleJob &J, int rb, int n, int c0, int c) {
+                                           const ResampleJob &J, int rb, int n, int c0, int c,
+                                           bool mono, int ka, int kz) {
+  Q.run_g[0][c] = run_terms(Q, J.lut, ka);
+  if (mono && ka == kz) {
+    Q.run_rk[0][c] = make_int2(INT32_MAX, ka);
+    return;
+  }
   const double P = col_P(J, c0 + c);
   auto keyat = [&](int ri) { return rg_key(S.crg, J, rb + ri, P); };
-  int ends[2] = {n - 1, n - 1};
-  int np = 1;
-  {
+  int split = n - 1;                     // last row of the first piece
+  if (!mono) {
     // x(L) = g0 + g2 P + g5 P^2 + (g1 + g4 P) L + g3 L^2: vertex in L
     const double *g = S.crg;
-    if (g[3] != 0.0) {
-      const double Lv = -(g[1] + g[4] * P) / (2.0 * g[3]);
-      const double rv = Lv / J.invL + J.midL - (double)J.my0 - (double)rb;
-      if (rv > 0.0 && rv < (double)(n - 1)) {
-        ends[0] = (int)rv;
-        np = 2;
-      }
-    }
+    const double Lv = -(g[1] + g[4] * P) / (2.0 * g[3]);
+    const double rv = Lv / J.invL + J.midL - (double)J.my0 - (double)rb;
+    if (rv > 0.0 && rv < (double)(n - 1)) split = (int)rv;
   }
-  int m = 0, last_key = 0, a = 0;
-  bool full = false;
-  for (int pc = 0; pc < np && !full; pc++) {
-    const int bend = ends[pc];
-    if (a > bend) continue;
-    int r = a, k = keyat(a);
-    const int kb = keyat(bend);
+  int m = 0, key = ka, from = 0;
+  for (int pc = 0; pc < 2; pc++) {
+    const int bend = pc == 0 ? split : n - 1;
+    if (from > bend) continue;
+    int r = from, k = pc == 0 ? ka : keyat(r);
+    const int kb = bend == n - 1 ? kz : keyat(bend);
     for (;;) {
-      if (m == 0 || k != last_key) {
+      if (k != key) {
+        // run m ends here; is there room for the next?
+        Q.run_rk[m][c] = make_int2(r, key);
+        m++;
         if (m == RsStrip<kSplit>::kRuns) {
           atomicMin(&Q.cov, r);
-          full = true;
-          break;
+          return;
         }
-        Q.run_rk[m][c] = make_int2(r, k);
         Q.run_g[m][c] = run_terms(Q, J.lut, k);
-        m++;
-        last_key = k;
+        key = k;
       }
       if (k == kb) break;   // monotone: the rest of the piece has this key
       int lo = r, hi = bend, khi = kb;
@@ -991,9 +1032,9 @@ __device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kS
       r = hi;
       k = khi;
     }
-    a = bend + 1;
+    from = bend + 1;
   }
-  Q.run_n[c] = (unsigned char)m;
+  Q.run_rk[m][c] = make_int2(INT32_MAX, key);
 }
 
 // [P7] Half h of a chunk of n rows: its window's lines, the entries of each
@@ -1006,6 +1047,35 @@ __device__ __forceinline__ void plan_half(RsStrip<kSplit> &Q, int h, int n) {
   H.tbase = 0;
   H.units = 0;
   const int r0 = h * RS_H, r1 = min(r0 + RS_H, n);
+  if (r1 - r0 == RS_H) {
+    // the usual half: one interior entry per row, consecutive lines, one bin
+    int re[RS_H];
+    int2 M[RS_H];
+    bool plain = true;
+#pragma unroll
+    for (int k = 0; k < RS_H; k++) re[k] = Q.rowe[r0 + k];
+    const int e0 = re[0] & 0xffff;
+#pragma unroll
+    for (int k = 0; k < RS_H; k++) {
+      plain = plain && re[k] >> 16 == 1;
+      M[k] = *reinterpret_cast<const int2 *>(&Q.eM[min(e0 + k, RS_ECAP - 1)]);
+    }
+#pragma unroll
+    for (int k = 0; k < RS_H; k++)
+      plain = plain && ((M[k].y >> 12) & 15) == REG_IN && M[k].x == M[0].x + k &&
+              (M[k].y & 0xfff) == (M[0].y & 0xfff);
+    if (plain) {
+      H.flags = HG_ON | HG_ONE | HG_PLAIN;
+      H.lb = M[0].x;
+      H.units = RS_H * RS_UN;
+#pragma unroll
+      for (int k = 0; k < 8; k++) H.pos[k] = (short)(e0 + min(max(k - 1, 0), RS_H));
+#pragma unroll
+      for (int k = 0; k < RS_H; k++) Q.eM[e0 + k].w = k * RS_UN | (RS_UN - 1) << 24;
+      Q.half[h] = H;
+      return;
+    }
+  }
   for (int r = r0; r < r1 && !(H.flags & HG_ON); r++) {
     const int re = Q.rowe[r], e0 = re & 0xffff, ne = re >> 16;
     for (int e = e0; e < e0 + ne; e++)
@@ -1014,8 +1084,8 @@ __device__ __forceinline__ void plan_half(RsStrip<kSplit> &Q, int h, int n) {
         H.lb = Q.eM[e].x - (r - r0);   // the row's last (highest) line
       }
   }
-  int cur = -1, end = Q.rowe[r0] & 0xffff, bin0 = -1;
-  bool one = true, plain = r1 - r0 == RS_H;
+  int cur = -1, end = Q.rowe[r0] & 0xffff;
+  bool one = true;
   H.pos[0] = (short)end;
   for (int r = r0; r < r1; r++) {
     const int re = Q.rowe[r], e0 = re & 0xffff, ne = re >> 16;
@@ -1026,8 +1096,6 @@ __device__ __forceinline__ void plan_half(RsStrip<kSplit> &Q, int h, int n) {
       if (((M.y >> 12) & 15) == REG_IN) {
         const int ulo = (M.w >> 16) & 0xff, uhi = (M.w >> 24) & 0xff;
         const int p = M.x - H.lb;
-        plain = plain && p == r - r0 && (bin0 < 0 || (M.y & 0xfff) == bin0);
-        bin0 = M.y & 0xfff;
         if (p < cur || p >= RS_H) {
           M.y |= E_DIRECT << 12;
           H.flags |= HG_DIRECT;
@@ -1042,7 +1110,7 @@ __device__ __forceinline__ void plan_half(RsStrip<kSplit> &Q, int h, int n) {
     }
   }
   for (; cur < RS_H; cur++) H.pos[cur + 2] = (short)end;
-  if (one) H.flags |= HG_ONE | (plain ? HG_PLAIN : 0);
+  if (one) H.flags |= HG_ONE;
   Q.half[h] = H;
 }
 
@@ -1161,6 +1229,8 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
   for (int j = 0; j < 12; j++) w[j].re = w[j].im = make_float2(0.f, 0.f);
 
   int want = RS_CH;                      // rows to try for a chunk
+  // the tile is free while a chunk is prepared: the rows' entries as found
+  int2 *const found = reinterpret_cast<int2 *>(&Q.tile[0]);
   for (int ch0 = 0; ch0 < nr;) {
     // ---- [P4] the azimuth entries of the chunk's rows (thread u: rows u and
     // u + 64): counts, and a scan of both packed in one word
@@ -1176,7 +1246,8 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
 #pragma unroll 1
       for (int i = 0; i < 2; i++) {
         const int r = u + RS_ST * i;
-        if (live && r < nrc) mm |= count_entries(S, Q, J, rb + r, c0, cN) << (16 * i);
+        if (live && r < nrc)
+          mm |= find_entries(S, Q, J, rb + r, c0, cN, found + r * RS_MAXKEY) << (16 * i);
       }
       int v = mm;
 #pragma unroll
@@ -1203,12 +1274,29 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
     // ---- [P5] the entries, [P6] the range-key runs
 #pragma unroll 1
     for (int r = u; r < nfit; r += RS_ST) {
-      const int re = Q.rowe[r];
-      if (re >> 16) write_entries(S, Q, J, rb + r, c0, cN, re & 0xffff);
+      const int re = Q.rowe[r], e = re & 0xffff;
+      for (int i = 0; i < re >> 16; i++)
+        write_entry(Q, J, found[r * RS_MAXKEY + i], cN, e + i);
     }
     if (dval) {
+      const double La = row_L(J, rb), Lz = row_L(J, rb + nfit - 1), c5 = S.crg[5];
+      const double Aa = row_a(S.crg, La), Ba = row_b(S.crg, La);
+      const double Az = row_a(S.crg, Lz), Bz = row_b(S.crg, Lz);
+      int ka[2], kz[2];
+      bool mono[2];
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const double Pc = col_P(J, c0 + dc + i);
+        ka[i] = rg_key_at(Aa, Ba, c5, Pc);
+        kz[i] = rg_key_at(Az, Bz, c5, Pc);
+        // slope in the row: (g1 + g4 P) + 2 g3 L, of one sign over the rows
+        const double s1 = fma(S.crg[4], Pc, S.crg[1]), s2 = 2.0 * S.crg[3];
+        mono[i] = (fma(s2, La, s1) < 0.0) == (fma(s2, Lz, s1) < 0.0);
+      }
 #pragma unroll 1
-      for (int c = dc; c < min(dc + 2, cN); c++) build_runs(S, Q, J, rb, nfit, c0, c);
+      for (int i = 0; i < (dtwo ? 2 : 1); i++)
+        build_runs(S, Q, J, rb, nfit, c0, dc + i, i ? mono[1] : mono[0], i ? ka[1] : ka[0],
+                   i ? kz[1] : kz[0]);
     }
     __syncthreads();
     // ---- [P7] the halves; a chunk that does not end the item ends with a
@@ -1260,10 +1348,15 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       cp_async_commit();
     }
 
+    PairRuns P;
+    P.mx = P.my = -1;
+    P.nextx = INT32_MIN;
+    P.nexty = dtwo ? INT32_MIN : INT32_MAX;
+    P.keyx = P.keyy = 0;
+    P.pair = false;
     for (int h = 0; h < nh; h++) {
       const RsHalf H = Q.half[h];
       const int flags = H.flags;
-      cp_async_wait<1>();                // this thread's staged lines of the half
       // ---- [A]
       if (flags & HG_ON) {
         if (h & 1)
@@ -1271,68 +1364,60 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
         else
           az_half<0, kSplit>(S, Q, J, t, u, xa, h, H, w);
         if (flags & HG_DIRECT) az_direct<kSplit>(Q, J, u, xa, H.tbase, H.pos[0], H.pos[7]);
+      } else {
+        cp_async_wait<1>();
       }
       if (h + 2 < nh && (Q.half[h + 2].flags & HG_ON))
         stage_half(S, J, t, xa, (h & 1) * RS_H, Q.half[h + 2].lb + RS_H);
       cp_async_commit();
       if (flags & HG_JOIN) continue;
-      __syncthreads();
-
       // ---- [B] range pass, reramp, store: 2 columns x the tile's rows
       const int h0 = (h & 1) && (Q.half[h - 1].flags & HG_JOIN) ? h - 1 : h;
       const int k0 = h0 * RS_H, k1 = min((h + 1) * RS_H, n);
       const int both = Q.half[h0].flags & flags, any = Q.half[h0].flags | flags;
+      if (dval && k0 >= min(P.nextx, P.nexty)) next_runs(P, Q, J, dc, dtwo, k0);
+      __syncthreads();
       unsigned miss = 0;                 // rows the pair path leaves
       if (dval) {
-        PairRuns P;
-        P.next = INT32_MIN;
         float2 *orow = J.out + (long)(rb + k0 - J.row0) * J.out_pitch + c0 + dc;
-        const bool one = (both & HG_ONE) != 0;
-        int e = Q.rowe[k0] & 0xffff;     // one entry per row: consecutive
-        int un = 0;
+        const long pitch = J.out_pitch;
+        int k = k0;
+        if (both & HG_ONE) {
+          // one interior entry per row: consecutive entries and tile rows
+          const int e0 = (Q.rowe[k0] & 0xffff) - k0;
+          const float4 *U = &Q.tile[0], *A = &Q.eA[e0 + k];
+          const int *R = &Q.eM[e0 + k].z;
 #pragma unroll 1
-        for (int k = k0; k < k1; k++, orow += J.out_pitch, e++, un += RS_UN) {
-          if (k >= P.next) load_runs(P, Q, J, dc, dtwo, k);
-          bool fast = P.pair;
-          if (!one) {
-            const int re = Q.rowe[k], ne = re >> 16;
-            if (ne == 0) continue;       // a per-pixel row
-            e = re & 0xffff;
-            int4 M = Q.eM[e];
-            for (int q = 1; q < ne && !(dc >= ((M.y >> 16) & 0xff) && dc < ((M.y >> 24) & 0xff));
-                 q++)
-              M = Q.eM[++e];
-            fast = fast && dc + 1 < ((M.y >> 24) & 0xff) && P.unit >= ((M.w >> 16) & 0xff) &&
-                   P.unit + 6 <= ((M.w >> 24) & 0xff) && ((M.y >> 12) & 3) == REG_IN;
-            un = (k >= h * RS_H ? H.tbase : 0) + (short)(M.w & 0xffff);
+          for (; k < k1; k++, orow += pitch, U += RS_UN, A++, R += 4) {
+            if (k >= min(P.nextx, P.nexty)) next_runs(P, Q, J, dc, dtwo, k);
+            if (P.pair) {
+              pair_row(P, U + P.unit, *A, __int_as_float(*R), orow, out16);
+            } else {
+              miss |= 1u << (k - k0);
+            }
           }
-          if (!fast) {
+        }
+#pragma unroll 1
+        for (; k < k1; k++, orow += pitch) {
+          if (k >= min(P.nextx, P.nexty)) next_runs(P, Q, J, dc, dtwo, k);
+          const int re = Q.rowe[k], ne = re >> 16;
+          if (ne == 0) continue;         // a per-pixel row
+          int e = re & 0xffff;
+          int4 M = Q.eM[e];
+          for (int q = 1; q < ne && !(dc >= ((M.y >> 16) & 0xff) && dc < ((M.y >> 24) & 0xff));
+               q++)
+            M = Q.eM[++e];
+          const bool same = dtwo && dc + 1 < ((M.y >> 24) & 0xff);
+          const int reg = (M.y >> 12) & 3;
+          if (reg != REG_IN && same) {
+            store_pair(orow, false, border_pixel(J, reg, M.x, P.keyx >> 12),
+                       border_pixel(J, reg, M.x, P.keyy >> 12));
+          } else if (P.pair && same && P.unit >= ((M.w >> 16) & 0xff) &&
+                     P.unit + 6 <= ((M.w >> 24) & 0xff)) {
+            pair_row(P, &Q.tile[(k >= h * RS_H ? H.tbase : 0) + (short)(M.w & 0xffff) + P.unit],
+                     Q.eA[e], __int_as_float(M.z), orow, out16);
+          } else {
             miss |= 1u << (k - k0);
-            continue;
-          }
-          const float4 *U = &Q.tile[un + P.unit];
-          float4 V[7];
-#pragma unroll
-          for (int m = 0; m < 7; m++) V[m] = U[m];
-          const float4 A = Q.eA[e];
-          const float R0 = __int_as_float(Q.eM[e].z);
-          const float2 f =
-              turns_to_rad2(make_float2(run_phase(A, R0, P.gx), run_phase(A, R0, P.gy)));
-          float2 vx, vy;
-          if (P.odd) {
-            vx = rg_sum<7>(P.wo, V);
-            vy = rg_sum<6>(P.we, V + 1);
-          } else {
-            vx = rg_sum<6>(P.we, V);
-            vy = rg_sum<7>(P.wo, V);
-          }
-          vx = cmul_conj(vx, f.x);
-          vy = cmul_conj(vy, f.y);
-          if (out16) {
-            *reinterpret_cast<float4 *>(orow) = make_float4(vx.x, vx.y, vy.x, vy.y);
-          } else {
-            orow[0] = vx;
-            orow[1] = vy;
           }
         }
       }
@@ -1361,7 +1446,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
     ch0 += n;
     want = max(2 * RS_H, n + n);         // shrink to what the tables held, then grow
     want = (want + 2 * RS_H - 1) / (2 * RS_H) * (2 * RS_H);
-    __syncthreads();   // the next chunk's (or item's) prologue rewrites the tables
+    __syncthreads();   // the next chunk's (or item's) prologue rewrites the tables and the tile
   }
 }
 
