@@ -147,22 +147,25 @@ union RsSlaveRow {
   } f;
 };
 
-// FP64 deramp quadratics of the ring columns (FP64 mode).
+// Deramp coefficients of the ring columns: G's (split mode) or the FP64
+// quadratics (FP64 mode, G's formed from them where needed).
 template <bool kSplit>
 struct RsRing {
   double2 a21[RS_FW];
   double a0[RS_FW];
 };
 template <>
-struct RsRing<true> {};
+struct RsRing<true> {
+  float2 g2[RS_UN], g1[RS_UN], g0[RS_UN];   // by unit
+};
 
 template <bool kSplit>
 struct __align__(16) RsStrip {
-  static constexpr int kRuns = kSplit ? 3 : 2;   // range-key runs per column and chunk
+  // range-key runs per column and chunk: what 75 KB per CTA leave room for
+  static constexpr int kRuns = kSplit ? 5 : 4;
   float4 tile[RS_TU];                 // azimuth-interpolated units
-  float4 run_g[kRuns][RS_TW];         // per run: (sp, G2, G1, G0)
+  float run_g[kRuns][3][RS_TW];       // per run: G2, G1, G0
   int2 run_rk[kRuns][RS_TW];          // (chunk row of the next run, key = p0 * 4096 + bin)
-  float4 ring_gc[RS_FW];              // per ring column (g2, g1, g0, 0)
   float4 eA[RS_ECAP];                 // entries: reramp terms (rho, psif, R2, R1)
   int4 eM[RS_ECAP];                   // (L0, bin | region << 12 | c_lo << 16 | c_hi << 24, R0,
                                       //  (tile offset & 0xffff) | first unit << 16 | last unit << 24)
@@ -224,6 +227,13 @@ __device__ __forceinline__ DerampQuad deramp_quad(double kt, double tref, double
 }
 __device__ __forceinline__ double quad_eval(const DerampQuad &q, double ta) {
   return fma(fma(q.a2, ta, q.a1), ta, q.a0);
+}
+// G = phi - phi_ref about the centre time tm, in turns: (g2, g1, g0).
+__device__ __forceinline__ float3 residual_phase(const DerampQuad &q, const DerampQuad &ref,
+                                                 double tm) {
+  const double d2 = q.a2 - ref.a2, d1 = q.a1 - ref.a1, d0 = q.a0 - ref.a0;
+  return make_float3((float)(d2 * kInvTwoPi), (float)((2.0 * d2 * tm + d1) * kInvTwoPi),
+                     (float)(((d2 * tm + d1) * tm + d0) * kInvTwoPi));
 }
 __device__ __forceinline__ double deramp_phase(double ta, double kt, double tref, double fdc) {
   const double e = ta - tref;
@@ -406,8 +416,7 @@ struct RingPhase<false> {
 template <bool kSplit>
 __device__ __forceinline__ RingPhase<kSplit> ring_load(const RsStrip<kSplit> &Q, int u) {
   if constexpr (kSplit) {
-    const float4 a = Q.ring_gc[2 * u], b = Q.ring_gc[2 * u + 1];
-    return {make_float2(a.x, b.x), make_float2(a.y, b.y), make_float2(a.z, b.z)};
+    return {Q.ring.g2[u], Q.ring.g1[u], Q.ring.g0[u]};
   } else {
     const double2 a = Q.ring.a21[2 * u], b = Q.ring.a21[2 * u + 1];
     return {DerampQuad{Q.ring.a0[2 * u], a.y, a.x}, DerampQuad{Q.ring.a0[2 * u + 1], b.y, b.x}};
@@ -670,6 +679,14 @@ __device__ __forceinline__ int ring_col(int xo, const ResampleJob &J, int key) {
   return (p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7 && xb >= 0 && xb + 13 < RS_FW) ? xb : -1;
 }
 
+// A run's terms with sp = sum_i kRg[i] - 1: (sp, G2, G1, G0).
+template <bool kSplit>
+__device__ __forceinline__ float4 run_load(const RsStrip<kSplit> &Q, const RsLut &lut, int m,
+                                           int c, int key) {
+  return make_float4(__ldg(lut.sp1 + (key & 4095)), Q.run_g[m][0][c], Q.run_g[m][1][c],
+                     Q.run_g[m][2][c]);
+}
+
 // Moves the runs on to chunk row `row`.
 template <bool kSplit>
 __device__ __forceinline__ void next_runs(PairRuns &P, const RsStrip<kSplit> &Q,
@@ -677,16 +694,16 @@ __device__ __forceinline__ void next_runs(PairRuns &P, const RsStrip<kSplit> &Q,
   while (row >= P.nextx) {
     P.mx++;
     const int2 rk = Q.run_rk[P.mx][c];
-    P.gx = Q.run_g[P.mx][c];
     P.nextx = rk.x;
     P.keyx = rk.y;
+    P.gx = run_load(Q, J.lut, P.mx, c, rk.y);
   }
   while (row >= P.nexty) {
     P.my++;
     const int2 rk = Q.run_rk[P.my][c + 1];
-    P.gy = Q.run_g[P.my][c + 1];
     P.nexty = rk.x;
     P.keyy = rk.y;
+    P.gy = run_load(Q, J.lut, P.my, c + 1, rk.y);
   }
   const int xb = ring_col(Q.xo, J, P.keyx);
   P.pair = two && xb >= 0 && ring_col(Q.xo, J, P.keyy) == xb + 1;
@@ -772,7 +789,8 @@ __device__ __forceinline__ void pixel_shared(RsStrip<kSplit> &Q, const ResampleJ
     taps_even(w, J.lut, key & 4095);
     v = rg_sum<6>(w, U);
   }
-  *out = cmul_conj_turns(v, run_phase(Q.eA[e], __int_as_float(M.z), Q.run_g[m][c]));
+  *out = cmul_conj_turns(v, run_phase(Q.eA[e], __int_as_float(M.z),
+                                      run_load(Q, J.lut, m, c, key)));
 }
 
 // The pixels the pair path left, all threads of a strip: pairs with a row in
@@ -949,31 +967,39 @@ __device__ __forceinline__ void write_entry(RsStrip<kSplit> &Q, const ResampleJo
   Q.eM[e] = make_int4(E.x, E.y, __float_as_int(R0), ulo << 16 | uhi << 24);
 }
 
-// Phase terms of a range-key run: (sp, G2, G1, G0) with Gk = sum_i kRg[i]
+// Residual-phase terms of a range-key run, (G2, G1, G0) with Gk = sum_i kRg[i]
 // gk(x_i) over the ring columns of its taps (0 when they leave the window).
 template <bool kSplit>
-__device__ __forceinline__ float4 run_terms(const RsStrip<kSplit> &Q, const RsLut &lut, int key) {
+__device__ __forceinline__ void run_terms(RsStrip<kSplit> &Q, const RsLut &lut, int m, int c,
+                                          int key) {
   const int p0 = key >> 12, bp = key & 4095;
   const int xb = p0 - 5 - Q.xo;
-  float4 gg = make_float4(__ldg(lut.sp1 + bp), 0.f, 0.f, 0.f);
+  float G2 = 0.f, G1 = 0.f, G0 = 0.f;
   if (xb >= 0 && xb + kTaps <= RS_FW) {
     const float *kp = lut.krg + bp * kTaps;
-    float G2 = 0.f, G1 = 0.f, G0 = 0.f;
 #pragma unroll
     for (int i = 0; i < kTaps; i++) {
       const float w = __ldg(kp + i);
-      const float4 gc = Q.ring_gc[xb + i];
-      G2 = fmaf(w, gc.x, G2);
-      G1 = fmaf(w, gc.y, G1);
-      G0 = fmaf(w, gc.z, G0);
+      const int x = xb + i;
+      float3 g;
+      if constexpr (kSplit) {
+        g = make_float3(reinterpret_cast<const float *>(Q.ring.g2)[x],
+                        reinterpret_cast<const float *>(Q.ring.g1)[x],
+                        reinterpret_cast<const float *>(Q.ring.g0)[x]);
+      } else {
+        const double2 a = Q.ring.a21[x];
+        g = residual_phase(DerampQuad{Q.ring.a0[x], a.y, a.x},
+                           DerampQuad{Q.ref_a0, Q.ref_a1, Q.ref_a2}, Q.tm);
+      }
+      G2 = fmaf(w, g.x, G2);
+      G1 = fmaf(w, g.y, G1);
+      G0 = fmaf(w, g.z, G0);
     }
-    gg.y = G2;
-    gg.z = G1;
-    gg.w = G0;
   }
-  return gg;
+  Q.run_g[m][0][c] = G2;
+  Q.run_g[m][1][c] = G1;
+  Q.run_g[m][2][c] = G0;
 }
-
 // [P6] The runs of column c's range key over chunk rows [0, n) (box rows rb
 // ...).  Most columns hold one key: when the position is monotone over the
 // rows and both ends agree (k0, k1 from the caller).  Else by bisection of the
@@ -984,7 +1010,7 @@ template <bool kSplit>
 __device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kSplit> &Q,
                                            const ResampleJob &J, int rb, int n, int c0, int c,
                                            bool mono, int ka, int kz) {
-  Q.run_g[0][c] = run_terms(Q, J.lut, ka);
+  run_terms(Q, J.lut, 0, c, ka);
   if (mono && ka == kz) {
     Q.run_rk[0][c] = make_int2(INT32_MAX, ka);
     return;
@@ -1014,7 +1040,7 @@ __device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kS
           atomicMin(&Q.cov, r);
           return;
         }
-        Q.run_g[m][c] = run_terms(Q, J.lut, k);
+        run_terms(Q, J.lut, m, c, k);
         key = k;
       }
       if (k == kb) break;   // monotone: the rest of the piece has this key
@@ -1201,20 +1227,23 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
   const int xa = Q.xo + 2 * u;           // absolute slave column
   {
     const DerampQuad refq = {Q.ref_a0, Q.ref_a1, Q.ref_a2};
-    const double tm = Q.tm;
+    float3 g[2];
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       const int x = xa + q;
       DerampQuad cq = refq;
       if (x >= J.sx0 && x <= J.sx1) cq = deramp_quad(J.kt[x], J.tref[x], J.fdc[x]);
-      const double d2 = cq.a2 - refq.a2, d1 = cq.a1 - refq.a1, d0 = cq.a0 - refq.a0;
-      Q.ring_gc[2 * u + q] = make_float4((float)(d2 * kInvTwoPi),   // in turns
-                                         (float)((2.0 * d2 * tm + d1) * kInvTwoPi),
-                                         (float)(((d2 * tm + d1) * tm + d0) * kInvTwoPi), 0.f);
-      if constexpr (!kSplit) {
+      if constexpr (kSplit) {
+        g[q] = residual_phase(cq, refq, Q.tm);
+      } else {
         Q.ring.a21[2 * u + q] = make_double2(cq.a2, cq.a1);
         Q.ring.a0[2 * u + q] = cq.a0;
       }
+    }
+    if constexpr (kSplit) {
+      Q.ring.g2[u] = make_float2(g[0].x, g[1].x);
+      Q.ring.g1[u] = make_float2(g[0].y, g[1].y);
+      Q.ring.g0[u] = make_float2(g[0].z, g[1].z);
     }
   }
 
@@ -1240,7 +1269,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       Q.nfit = nrc;
       Q.cov = nrc;
     }
-    __syncthreads();                     // also: ring_gc is written
+    __syncthreads();                     // also: the ring's terms are written
     {
       int mm = 0;
 #pragma unroll 1
