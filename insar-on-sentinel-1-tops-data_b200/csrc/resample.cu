@@ -12,19 +12,18 @@
 //             deramped slave d = s exp(i phi), reramped with the LUT-weighted
 //             sum of the deramp phase phi.
 //
-// B200 design (no textures, no phase array in HBM).  A CTA of 128 threads
-// owns two adjacent strips of RS_TW = 112 output columns, 64 threads and a
-// ring of 128 slave columns (two per thread) each, and a segment of up to 252
-// output rows (a work item).  The rows are prepared in chunks and computed in
+// B200 design (no textures, no phase array in HBM).  A CTA of 64 threads
+// owns a strip of RS_TW = 112 output columns with a ring of 128 slave columns
+// (two per thread) and a segment of up to 252 output rows (a work item).  The rows are prepared in chunks and computed in
 // halves of 6 rows:
 //
-// Chunk prologue.  Row keys: per row and strip, the runs of equal azimuth key
+// Chunk prologue.  Row keys: per row, the runs of equal azimuth key
 // (L0, bin) along the strip, found by bisection of the exact per-pixel key on
 // monotone pieces; each run is an "entry" (its columns, its reramp terms).
 // Nearly parallel orbits give one entry per row, crossing orbits a few.
 // Column keys: thread per column pair, the runs of the range key over the
 // chunk's rows, each with its residual phase terms.  A chunk is as many rows
-// (up to 120) as the entry and run tables hold.
+// (up to 96) as the entry and run tables hold.
 //
 // Half of 6 rows.
 //   [A] azimuth pass, thread = 2 adjacent ring columns: six new slave lines
@@ -52,17 +51,16 @@
 //        (entry; M0..M2 the azimuth taps' moments, tc0 = tc(L0)),
 // equal to the reference's sum in exact arithmetic.
 //
-// What bounds it: instruction issue with 12 warps per SM (168 registers and 72
-// KB of shared memory per CTA allow 3 CTAs).  Two columns per thread share a
-// line's terms, a row's taps and the bookkeeping, and fill the FP32x2 lanes:
-// 117 instead of 158 thread instructions per pixel on a burst of 1500 x 21000
-// (one entry per row, nearly no key changes), 0.463 -> 0.351 ms; the range
-// runs kept over a chunk's tiles instead of loaded per tile, and a shorter
-// prologue (entries found once, columns of one key and plain halves without a
-// search): 0.351 -> 0.305 ms (816 -> 1239 GB/s of 12 bytes per pixel in all).
-// Rows whose strip spans several azimuth keys
-// took a per-pixel path from HBM before, columns with many range keys a keyed
-// one: a burst of 1539 x 10867 of crossing orbits 3.92 -> 0.79 ms.
+// What bounds it: the latency of each warp's instruction stream (about 7 cycles
+// per instruction) with 12 warps per SM: the window, the taps of two columns and
+// a row's samples need 168 registers.  Two columns per thread share a line's
+// terms, a row's taps and the bookkeeping, and fill the FP32x2 lanes: 105
+// instead of 158 thread instructions per pixel.  A burst of 1500 x 21000 (one
+// entry per row) 0.463 -> 0.300 ms (816 -> 1260 GB/s of 12 bytes per pixel); a
+// burst of 300 x 512 70 -> 23 us (short segments: a row costs a lone CTA 0.7
+// us).  Rows whose strip spans several azimuth keys took a per-pixel path from
+// HBM before, columns with many range keys a keyed one: a burst of 1539 x 10867
+// of crossing orbits 3.92 -> 0.62 ms.
 //
 // Which path a pixel takes, and the order of its sums, depend on its row, its
 // column and its strip only, never on the work item, so a job that produces a
@@ -90,25 +88,23 @@
 
 namespace tops {
 
-constexpr int RS_NT = 128;                 // threads per CTA
-constexpr int RS_NS = 2;                   // strips per CTA
-constexpr int RS_ST = RS_NT / RS_NS;       // threads per strip
+constexpr int RS_NT = 64;                  // threads per CTA
 constexpr int RS_TW = 112;                 // output columns per strip
 constexpr int RS_FW = 128;                 // ring (slave) columns of a strip
 constexpr int RS_UN = RS_FW / 2;           // 2-column units of a ring
 constexpr int RS_DT = RS_TW / 2;           // range-pass threads per strip
 constexpr int RS_H = 6;                    // rows (and pushed lines) per half
 constexpr int RS_MAXSEG = 252;             // longest work item
-constexpr int RS_CH = 120;                 // rows per chunk
+constexpr int RS_CH = 96;                  // rows per chunk
 constexpr int RS_NH = RS_CH / RS_H;        // halves per chunk
-constexpr int RS_ECAP = 136;               // entries per chunk and strip
-constexpr int RS_TU = 2 * RS_H * RS_UN;    // tile units per strip
+constexpr int RS_ECAP = 112;               // entries per chunk and strip
+constexpr int RS_TU = 2 * RS_H * RS_UN;    // tile units
 constexpr int RS_ROWU = RS_TU / RS_H;      // most tile units of a row
 constexpr int RS_MAXKEY = 12;              // most entries of a row
 constexpr int RS_MAXJOBS = 32;
-static_assert(RS_UN == RS_ST, "one unit per thread in the azimuth pass");
-static_assert(RS_DT <= RS_ST && RS_CH <= 2 * RS_ST && RS_CH % (2 * RS_H) == 0 &&
-                  RS_MAXKEY <= RS_ECAP && RS_TW < 128 && RS_NH <= RS_ST &&
+static_assert(RS_UN == RS_NT, "one unit per thread in the azimuth pass");
+static_assert(RS_DT <= RS_NT && RS_CH <= 2 * RS_NT && RS_CH % (2 * RS_H) == 0 &&
+                  RS_MAXKEY <= RS_ECAP && RS_TW < 128 && RS_NH <= RS_NT &&
                   RS_CH * RS_MAXKEY * 8 <= RS_TU * 16,
               "thread mappings and table fields assume these sizes");
 
@@ -161,7 +157,7 @@ struct RsRing<true> {
 
 template <bool kSplit>
 struct __align__(16) RsStrip {
-  // range-key runs per column and chunk: what 75 KB per CTA leave room for
+  // range-key runs per column and chunk: what 37 KB per CTA leave room for
   static constexpr int kRuns = kSplit ? 5 : 4;
   float4 tile[RS_TU];                 // azimuth-interpolated units
   float run_g[kRuns][3][RS_TW];       // per run: G2, G1, G0
@@ -173,18 +169,20 @@ struct __align__(16) RsStrip {
   RsSlaveRow srow[RS_NH * RS_H];      // the lines the halves push
   int rowe[RS_CH];                    // first entry | entries << 16 (0 entries: per-pixel row)
   unsigned gen[2 * RS_H][4];          // pixels of the tile's rows left to the per-pixel path
-  unsigned missb[RS_ST / 32];         // pairs with rows the pair path left, and the rows
-  unsigned short miss[RS_ST];
-  int scan[RS_ST / 32];
+  unsigned missb[RS_NT / 32];         // pairs with rows the pair path left, and the rows
+  unsigned short miss[RS_NT];
+  int scan[RS_NT / 32];
   RsRing<kSplit> ring;
   double ref_a0, ref_a1, ref_a2, tm;  // reference column's phase, burst centre time
   int xo, dlo, dhi;                   // ring origin, bounds of (ring column - strip column)
   int nfit, cov, gen_any, prev_line;
+  int n_border;                       // border columns of the chunk
+  unsigned char border[RS_TW];
 };
 
 template <bool kSplit>
 struct __align__(16) RsShared {
-  RsStrip<kSplit> strip[RS_NS];
+  RsStrip<kSplit> strip;
   uint2 stage[2 * RS_H][RS_NT];       // raw slave lines of the next two halves
   double caz[6], crg[6], shift;
   int next_item;
@@ -387,7 +385,7 @@ __device__ __forceinline__ float2 pixel_generic(const RsShared<kSplit> &S, const
 }
 
 // The per-pixel rows and the listed pixels of nrows tile rows (chunk rows from
-// cr0, box rows from r0 on), all threads of a strip.
+// cr0, box rows from r0 on), all threads.
 template <bool kSplit>
 __device__ __forceinline__ void pixel_pass(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
                                            const ResampleJob &J, int u, int cr0, int r0, int nrows,
@@ -395,7 +393,7 @@ __device__ __forceinline__ void pixel_pass(const RsShared<kSplit> &S, const RsSt
   for (int k = 0; k < nrows; k++) {
     const bool whole = (Q.rowe[cr0 + k] >> 16) == 0;
     const int r = r0 + k;
-    for (int c = u; c < cN; c += RS_ST)
+    for (int c = u; c < cN; c += RS_NT)
       if (whole || ((Q.gen[k][c >> 5] >> (c & 31)) & 1u))
         J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] = pixel_generic(S, J, r, c0 + c);
   }
@@ -478,9 +476,9 @@ __device__ __forceinline__ uint2 raw_pair(const ResampleJob &J, int xa, int y) {
 
 // Stages lines y0 .. y0 + 5 into `slot` .. `slot + 5` (zeros outside the box).
 template <bool kSplit>
-__device__ __forceinline__ void stage_half(RsShared<kSplit> &S, const ResampleJob &J, int t,
+__device__ __forceinline__ void stage_half(RsShared<kSplit> &S, const ResampleJob &J, int u,
                                            int xa, int slot, int y0) {
-  const unsigned d = smem_u32(&S.stage[slot][t]);
+  const unsigned d = smem_u32(&S.stage[slot][u]);
   constexpr unsigned kRow = RS_NT * sizeof(uint2);
   const bool in0 = xa >= J.sx0 && xa <= J.sx1, in1 = xa + 1 >= J.sx0 && xa + 1 <= J.sx1;
   const long off = (long)(y0 - J.sy0) * J.slave_pitch + (xa - J.sx0);
@@ -558,7 +556,7 @@ __device__ __forceinline__ void az_fill(const RsStrip<kSplit> &Q, const Resample
 // (6 HALF + k + j) % 12.  A plain half takes its taps once and one sum per push.
 template <int HALF, bool kSplit>
 __device__ __forceinline__ void az_half(RsShared<kSplit> &S, RsStrip<kSplit> &Q,
-                                        const ResampleJob &J, int t, int u, int xa, int h,
+                                        const ResampleJob &J, int u, int xa, int h,
                                         const RsHalf &H, Dpair (&w)[12]) {
   constexpr int R0 = RS_H * HALF;
   const RingPhase<kSplit> R = ring_load<kSplit>(Q, u);
@@ -571,7 +569,7 @@ __device__ __forceinline__ void az_half(RsShared<kSplit> &S, RsStrip<kSplit> &Q,
     az_taps(wz, lut, Q.eM[H.pos[0]].y & 0xfff);
     float4 *o = &Q.tile[H.tbase + u];
 #define RS_PUSH(k)                                                              \
-  w[(R0 + (k) + 11) % 12] = deramp_pair<kSplit>(S.stage[R0 + (k)][t], sr[k], R); \
+  w[(R0 + (k) + 11) % 12] = deramp_pair<kSplit>(S.stage[R0 + (k)][u], sr[k], R); \
   o[(k) * RS_UN] = az_sum<(R0 + (k)) % 12>(wz, w);
     RS_PUSH(0)
     RS_PUSH(1)
@@ -584,7 +582,7 @@ __device__ __forceinline__ void az_half(RsShared<kSplit> &S, RsStrip<kSplit> &Q,
   }
   az_entries<(R0 + 11) % 12, kSplit>(Q, lut, u, H.pos[0], H.pos[1], H.tbase, w);
 #define RS_PUSH(k)                                                              \
-  w[(R0 + (k) + 11) % 12] = deramp_pair<kSplit>(S.stage[R0 + (k)][t], sr[k], R); \
+  w[(R0 + (k) + 11) % 12] = deramp_pair<kSplit>(S.stage[R0 + (k)][u], sr[k], R); \
   az_entries<(R0 + (k)) % 12, kSplit>(Q, lut, u, H.pos[(k) + 1], H.pos[(k) + 2], H.tbase, w);
   RS_PUSH(0)
   RS_PUSH(1)
@@ -662,21 +660,26 @@ __device__ __forceinline__ float run_phase(float4 A, float R0, float4 g) {
 
 // The current runs of a thread's two output columns, kept over a chunk's tiles.
 struct PairRuns {
-  float4 gx, gy;
+  float4 gx, gy;         // pair: the columns' terms
   float4 we[3], wo[4];   // pair: taps of the even-aligned and of the odd column
-  int keyx, keyy;
-  int nextx, nexty;      // chunk row of each column's next run
-  int mx, my;            // run numbers (-1: none yet)
-  int unit;              // pair: first tile unit of its 14 samples
-  bool pair, odd;        // pair: both columns in the ring, adjacent samples;
-                         // odd: the first column is the odd-aligned one
+  int next;              // chunk row of either column's next run
+  int unit;              // first tile unit of the 14 samples; -1: no pair (the
+                         // columns' samples are not adjacent or leave the ring)
+  int m;                 // run numbers, first | second << 8
+  bool odd;              // the first column is the odd-aligned one
+  bool vec;              // both columns range-interior, outputs 16-byte aligned
+  int in;                // range-interior columns: 1 the first, 2 the second
 };
 
-// Ring column of a key's first tap when the column is range-interior and
-// inside the ring, else -1.
-__device__ __forceinline__ int ring_col(int xo, const ResampleJob &J, int key) {
-  const int p0 = key >> 12, xb = p0 - 5 - xo;
-  return (p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7 && xb >= 0 && xb + 13 < RS_FW) ? xb : -1;
+// Ring column of a key's first tap when its 14 samples are inside the ring,
+// else -1.
+__device__ __forceinline__ int ring_col(int xo, int key) {
+  const int xb = (key >> 12) - 5 - xo;
+  return xb >= 0 && xb + 13 < RS_FW ? xb : -1;
+}
+__device__ __forceinline__ bool range_in(const ResampleJob &J, int key) {
+  const int p0 = key >> 12;
+  return p0 >= J.sx0 + 5 && p0 <= J.sx1 - 7;
 }
 
 // A run's terms with sp = sum_i kRg[i] - 1: (sp, G2, G1, G0).
@@ -691,42 +694,32 @@ __device__ __forceinline__ float4 run_load(const RsStrip<kSplit> &Q, const RsLut
 template <bool kSplit>
 __device__ __forceinline__ void next_runs(PairRuns &P, const RsStrip<kSplit> &Q,
                                           const ResampleJob &J, int c, bool two, int row) {
-  while (row >= P.nextx) {
-    P.mx++;
-    const int2 rk = Q.run_rk[P.mx][c];
-    P.nextx = rk.x;
-    P.keyx = rk.y;
-    P.gx = run_load(Q, J.lut, P.mx, c, rk.y);
-  }
-  while (row >= P.nexty) {
-    P.my++;
-    const int2 rk = Q.run_rk[P.my][c + 1];
-    P.nexty = rk.x;
-    P.keyy = rk.y;
-    P.gy = run_load(Q, J.lut, P.my, c + 1, rk.y);
-  }
-  const int xb = ring_col(Q.xo, J, P.keyx);
-  P.pair = two && xb >= 0 && ring_col(Q.xo, J, P.keyy) == xb + 1;
-  if (P.pair) {
-    P.odd = (xb & 1) != 0;
+  int mx = P.m & 0xff, my = P.m >> 8;
+  int2 rx = Q.run_rk[mx][c];
+  int2 ry = two ? Q.run_rk[my][c + 1] : make_int2(INT32_MAX, 0);
+  while (row >= rx.x) rx = Q.run_rk[++mx][c];
+  while (row >= ry.x) ry = Q.run_rk[++my][c + 1];
+  P.m = mx | my << 8;
+  P.next = min(rx.x, ry.x);
+  const int xb = ring_col(Q.xo, rx.y);
+  P.in = (range_in(J, rx.y) ? 1 : 0) | (two && range_in(J, ry.y) ? 2 : 0);
+  P.vec = P.in == 3 && J.out_al16;
+  P.unit = -1;
+  if (two && xb >= 0 && ring_col(Q.xo, ry.y) == xb + 1) {
+    const bool odd = (xb & 1) != 0;
+    P.odd = odd;
     P.unit = xb >> 1;
-    taps_even(P.we, J.lut, (P.odd ? P.keyy : P.keyx) & 4095);
-    taps_odd(P.wo, J.lut, (P.odd ? P.keyx : P.keyy) & 4095);
+    taps_even(P.we, J.lut, (odd ? ry.y : rx.y) & 4095);
+    taps_odd(P.wo, J.lut, (odd ? rx.y : ry.y) & 4095);
+    P.gx = run_load(Q, J.lut, mx, c, rx.y);
+    P.gy = run_load(Q, J.lut, my, c + 1, ry.y);
   }
 }
 
-__device__ __forceinline__ void store_pair(float2 *o, bool out16, float2 a, float2 b) {
-  if (out16) {
-    *reinterpret_cast<float4 *>(o) = make_float4(a.x, a.y, b.x, b.y);
-  } else {
-    o[0] = a;
-    o[1] = b;
-  }
-}
 // Both columns of a pair in one row: U the units of its 14 samples, A and R0
-// the entry's reramp terms.
+// the entry's reramp terms.  Border columns are not stored.
 __device__ __forceinline__ void pair_row(const PairRuns &P, const float4 *U, float4 A, float R0,
-                                         float2 *o, bool out16) {
+                                         float2 *o) {
   float4 V[7];
 #pragma unroll
   for (int m = 0; m < 7; m++) V[m] = U[m];
@@ -739,7 +732,14 @@ __device__ __forceinline__ void pair_row(const PairRuns &P, const float4 *U, flo
     vx = rg_sum<6>(P.we, V);
     vy = rg_sum<7>(P.wo, V);
   }
-  store_pair(o, out16, cmul_conj(vx, f.x), cmul_conj(vy, f.y));
+  vx = cmul_conj(vx, f.x);
+  vy = cmul_conj(vy, f.y);
+  if (P.vec) {
+    *reinterpret_cast<float4 *>(o) = make_float4(vx.x, vx.y, vy.x, vy.y);
+  } else {
+    if (P.in & 1) o[0] = vx;
+    if (P.in & 2) o[1] = vy;
+  }
 }
 
 // A pixel off the slave box's interior: 0 outside, the nearest sample at the
@@ -771,7 +771,7 @@ __device__ __forceinline__ void pixel_shared(RsStrip<kSplit> &Q, const ResampleJ
     *out = border_pixel(J, reg, M.x, p0);
     return;
   }
-  const int xb = ring_col(Q.xo, J, key);
+  const int xb = ring_col(Q.xo, key);
   const int ulo = (M.w >> 16) & 0xff, uhi = (M.w >> 24) & 0xff;
   if (xb < 0 || (xb >> 1) < ulo || ((xb + 12) >> 1) > uhi) {
     atomicOr(&Q.gen[kt][c >> 5], 1u << (c & 31));
@@ -793,7 +793,32 @@ __device__ __forceinline__ void pixel_shared(RsStrip<kSplit> &Q, const ResampleJ
                                       run_load(Q, J.lut, m, c, key)));
 }
 
-// The pixels the pair path left, all threads of a strip: pairs with a row in
+// The border pixels of a chunk's columns listed in Q.border (those off the
+// range interior in some row): all rows at once, so that their loads overlap.
+template <bool kSplit>
+__device__ __forceinline__ void border_columns(const RsStrip<kSplit> &Q, const ResampleJob &J,
+                                               int u, int n, float2 *obase) {
+  const int nb = Q.n_border;
+#pragma unroll 4
+  for (int v = u; v < nb * n; v += RS_NT) {
+    const int k = v / nb, c = Q.border[v - k * nb];
+    const int re = Q.rowe[k], ne = re >> 16;
+    if (ne == 0) continue;               // a per-pixel row
+    int e = re & 0xffff;
+    for (int q = 1; q < ne; q++, e++) {
+      const int z = Q.eM[e].y;
+      if (c >= ((z >> 16) & 0xff) && c < ((z >> 24) & 0xff)) break;
+    }
+    int m = 0;
+    while (k >= Q.run_rk[m][c].x) m++;
+    const int key = Q.run_rk[m][c].y;
+    if (range_in(J, key)) continue;
+    const int4 M = Q.eM[e];
+    obase[(long)k * J.out_pitch + c] = border_pixel(J, (M.y >> 12) & 3, M.x, key >> 12);
+  }
+}
+
+// The pixels the pair path left, all threads: pairs with a row in
 // Q.miss, nrows tile rows from chunk row k0 on; from row ks on the entries'
 // tile starts at tb1.  obase: the output at chunk row k0, strip column 0.
 template <bool kSplit>
@@ -802,7 +827,7 @@ __device__ __forceinline__ void slow_pixels(RsStrip<kSplit> &Q, const ResampleJo
                                             float2 *obase) {
   const int n0 = __popc(Q.missb[0]), np = n0 + __popc(Q.missb[1]);
   const int per = 2 * nrows;
-  for (int v = u0; v < np * per; v += RS_ST) {
+  for (int v = u0; v < np * per; v += RS_NT) {
     int i = v / per;
     const int w = v - i * per, q = w >> 1;
     const int wq = i >= n0 ? 1 : 0;
@@ -1140,35 +1165,33 @@ __device__ __forceinline__ void plan_half(RsStrip<kSplit> &Q, int h, int n) {
   Q.half[h] = H;
 }
 
-// One work item (strip pair x segment of one job); all threads of the CTA call
-// it with the same item.  Threads 0..63 work on the first strip, the others on
-// the second; only the barriers and the row loop are common.
+// One work item (strip x segment of one job); all threads of the CTA call it
+// with the same item.
 template <bool kSplit>
 __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch &B, int item) {
-  const int t = threadIdx.x, side = t / RS_ST, u = t % RS_ST;
-  RsStrip<kSplit> &Q = S.strip[side];
+  const int u = threadIdx.x;
+  RsStrip<kSplit> &Q = S.strip;
 
-  // ---- locate the work item (job, strip pair, segment)
+  // ---- locate the work item (job, strip, segment)
   int jb = 0;
   while (jb + 1 < B.njobs && B.jobs[jb + 1].item_begin <= item) jb++;
   const ResampleJob &J = B.jobs[jb];
   const int local = item - J.item_begin;
   const int seg = local / J.strips;
-  const int c0 = ((local - seg * J.strips) * RS_NS + side) * RS_TW;
-  const int cN = min(RS_TW, J.mx1 - J.mx0 + 1 - c0);   // <= 0: no such strip
-  const bool live = cN > 0;
+  const int c0 = (local - seg * J.strips) * RS_TW;
+  const int cN = min(RS_TW, J.mx1 - J.mx0 + 1 - c0);
   const int r_begin = J.row0 + seg * J.seg_rows;
   const int nr = min(J.seg_rows, J.row0 + J.nrows - r_begin);
 
   // ---- [P1] polynomials and shift
-  if (t < 12) {
-    const double v = J.cpm_dev ? J.cpm_dev[t] : (t < 6 ? J.caz[t] : J.crg[t - 6]);
-    if (t < 6)
-      S.caz[t] = v;
+  if (u < 12) {
+    const double v = J.cpm_dev ? J.cpm_dev[u] : (u < 6 ? J.caz[u] : J.crg[u - 6]);
+    if (u < 6)
+      S.caz[u] = v;
     else
-      S.crg[t - 6] = v;
+      S.crg[u - 6] = v;
   }
-  if (t == 12) {
+  if (u == 12) {
     double sh = J.az_shift;
     if (J.az_shift_dev) {
       // a device-provided ESD shift above 100 px is invalid and reset to 0,
@@ -1250,7 +1273,6 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
   // range-pass columns
   const int dc = 2 * u;
   const bool dval = u < RS_DT && dc < cN, dtwo = dval && dc + 1 < cN;
-  const bool out16 = J.out_al16 != 0;
 
   // the 12-line window of the two ring columns
   Dpair w[12];
@@ -1268,29 +1290,30 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
     if (u == 0) {
       Q.nfit = nrc;
       Q.cov = nrc;
+      Q.n_border = 0;
     }
     __syncthreads();                     // also: the ring's terms are written
     {
       int mm = 0;
 #pragma unroll 1
       for (int i = 0; i < 2; i++) {
-        const int r = u + RS_ST * i;
-        if (live && r < nrc)
+        const int r = u + RS_NT * i;
+        if (r < nrc)
           mm |= find_entries(S, Q, J, rb + r, c0, cN, found + r * RS_MAXKEY) << (16 * i);
       }
       int v = mm;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const int x = __shfl_up_sync(0xffffffffu, v, o);
-        if ((t & 31) >= o) v += x;
+        if ((u & 31) >= o) v += x;
       }
-      if ((t & 31) == 31) Q.scan[u >> 5] = v;
+      if ((u & 31) == 31) Q.scan[u >> 5] = v;
       __syncthreads();
       if (u >= 32) v += Q.scan[0];
       const int total0 = (Q.scan[0] + Q.scan[1]) & 0xffff;
 #pragma unroll
       for (int i = 0; i < 2; i++) {
-        const int r = u + RS_ST * i, m = (mm >> (16 * i)) & 0xffff;
+        const int r = u + RS_NT * i, m = (mm >> (16 * i)) & 0xffff;
         const int end = ((v >> (16 * i)) & 0xffff) + (i ? total0 : 0);
         if (r < nrc) {
           Q.rowe[r] = (end - m) | m << 16;
@@ -1299,10 +1322,10 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       }
     }
     __syncthreads();
-    const int nfit = min(S.strip[0].nfit, S.strip[1].nfit);
+    const int nfit = Q.nfit;
     // ---- [P5] the entries, [P6] the range-key runs
 #pragma unroll 1
-    for (int r = u; r < nfit; r += RS_ST) {
+    for (int r = u; r < nfit; r += RS_NT) {
       const int re = Q.rowe[r], e = re & 0xffff;
       for (int i = 0; i < re >> 16; i++)
         write_entry(Q, J, found[r * RS_MAXKEY + i], cN, e + i);
@@ -1330,18 +1353,21 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
     __syncthreads();
     // ---- [P7] the halves; a chunk that does not end the item ends with a
     // pair of halves, so that the window carries over
-    int n = min(nfit, min(S.strip[0].cov, S.strip[1].cov));
+    int n = min(nfit, Q.cov);
     if (n < nr - ch0 && n >= 2 * RS_H) n -= n % (2 * RS_H);
     const int nh = (n + RS_H - 1) / RS_H;
-    if (u < nh) {
-      if (live) {
-        plan_half(Q, u, n);
-      } else {
-        Q.half[u].flags = 0;
-        Q.half[u].units = 0;
-        Q.half[u].lb = 0;
+    if (dval) {
+      for (int c = dc; c < min(dc + 2, cN); c++) {
+        bool out = false;
+        for (int m = 0;; m++) {
+          const int2 rk = Q.run_rk[m][c];
+          out = out || !range_in(J, rk.y);
+          if (rk.x >= n) break;
+        }
+        if (out) Q.border[atomicAdd(&Q.n_border, 1)] = (unsigned char)c;
       }
     }
+    if (u < nh) plan_half(Q, u, n);
     __syncthreads();
     int fl = 0, tb = 0;
     if (u < nh) {
@@ -1351,8 +1377,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
                          : (Q.half[u - 1].flags & HG_ON) ? Q.half[u - 1].lb + RS_H : INT32_MIN;
       if ((fl & HG_ON) && H.lb != expect) fl |= HG_FILL;
       const int h0 = u & ~1;
-      if (h0 + 1 < nh && S.strip[0].half[h0].units + S.strip[0].half[h0 + 1].units <= RS_TU &&
-          S.strip[1].half[h0].units + S.strip[1].half[h0 + 1].units <= RS_TU) {
+      if (h0 + 1 < nh && Q.half[h0].units + Q.half[h0 + 1].units <= RS_TU) {
         if (u & 1)
           tb = Q.half[h0].units;
         else
@@ -1360,7 +1385,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       }
     }
     // deramp terms of the lines the halves push
-    for (int i = u; i < nh * RS_H; i += RS_ST)
+    for (int i = u; i < nh * RS_H; i += RS_NT)
       Q.srow[i] = line_terms<kSplit>(Q, J, Q.half[i / RS_H].lb + RS_H + i % RS_H);
     __syncthreads();
     if (u < nh) {
@@ -1373,38 +1398,39 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       if (h < nh && (Q.half[h].flags & HG_ON))
-        stage_half(S, J, t, xa, h * RS_H, Q.half[h].lb + RS_H);
+        stage_half(S, J, u, xa, h * RS_H, Q.half[h].lb + RS_H);
       cp_async_commit();
     }
 
+    if (Q.n_border)
+      border_columns(Q, J, u, n, J.out + (long)(rb - J.row0) * J.out_pitch + c0);
     PairRuns P;
-    P.mx = P.my = -1;
-    P.nextx = INT32_MIN;
-    P.nexty = dtwo ? INT32_MIN : INT32_MAX;
-    P.keyx = P.keyy = 0;
-    P.pair = false;
+    P.m = 0;
+    P.next = INT32_MIN;
+    P.unit = -1;
+    P.in = 0;
     for (int h = 0; h < nh; h++) {
       const RsHalf H = Q.half[h];
       const int flags = H.flags;
       // ---- [A]
       if (flags & HG_ON) {
         if (h & 1)
-          az_half<1, kSplit>(S, Q, J, t, u, xa, h, H, w);
+          az_half<1, kSplit>(S, Q, J, u, xa, h, H, w);
         else
-          az_half<0, kSplit>(S, Q, J, t, u, xa, h, H, w);
+          az_half<0, kSplit>(S, Q, J, u, xa, h, H, w);
         if (flags & HG_DIRECT) az_direct<kSplit>(Q, J, u, xa, H.tbase, H.pos[0], H.pos[7]);
       } else {
         cp_async_wait<1>();
       }
       if (h + 2 < nh && (Q.half[h + 2].flags & HG_ON))
-        stage_half(S, J, t, xa, (h & 1) * RS_H, Q.half[h + 2].lb + RS_H);
+        stage_half(S, J, u, xa, (h & 1) * RS_H, Q.half[h + 2].lb + RS_H);
       cp_async_commit();
       if (flags & HG_JOIN) continue;
       // ---- [B] range pass, reramp, store: 2 columns x the tile's rows
       const int h0 = (h & 1) && (Q.half[h - 1].flags & HG_JOIN) ? h - 1 : h;
       const int k0 = h0 * RS_H, k1 = min((h + 1) * RS_H, n);
       const int both = Q.half[h0].flags & flags, any = Q.half[h0].flags | flags;
-      if (dval && k0 >= min(P.nextx, P.nexty)) next_runs(P, Q, J, dc, dtwo, k0);
+      if (dval && k0 >= P.next) next_runs(P, Q, J, dc, dtwo, k0);
       __syncthreads();
       unsigned miss = 0;                 // rows the pair path leaves
       if (dval) {
@@ -1418,17 +1444,17 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
           const int *R = &Q.eM[e0 + k].z;
 #pragma unroll 1
           for (; k < k1; k++, orow += pitch, U += RS_UN, A++, R += 4) {
-            if (k >= min(P.nextx, P.nexty)) next_runs(P, Q, J, dc, dtwo, k);
-            if (P.pair) {
-              pair_row(P, U + P.unit, *A, __int_as_float(*R), orow, out16);
-            } else {
+            if (k >= P.next) next_runs(P, Q, J, dc, dtwo, k);
+            if (P.unit >= 0) {
+              pair_row(P, U + P.unit, *A, __int_as_float(*R), orow);
+            } else if (P.in) {
               miss |= 1u << (k - k0);
             }
           }
         }
 #pragma unroll 1
         for (; k < k1; k++, orow += pitch) {
-          if (k >= min(P.nextx, P.nexty)) next_runs(P, Q, J, dc, dtwo, k);
+          if (k >= P.next) next_runs(P, Q, J, dc, dtwo, k);
           const int re = Q.rowe[k], ne = re >> 16;
           if (ne == 0) continue;         // a per-pixel row
           int e = re & 0xffff;
@@ -1439,13 +1465,13 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
           const bool same = dtwo && dc + 1 < ((M.y >> 24) & 0xff);
           const int reg = (M.y >> 12) & 3;
           if (reg != REG_IN && same) {
-            store_pair(orow, false, border_pixel(J, reg, M.x, P.keyx >> 12),
-                       border_pixel(J, reg, M.x, P.keyy >> 12));
-          } else if (P.pair && same && P.unit >= ((M.w >> 16) & 0xff) &&
+            orow[0] = border_pixel(J, reg, M.x, Q.run_rk[P.m & 0xff][dc].y >> 12);
+            orow[1] = border_pixel(J, reg, M.x, Q.run_rk[P.m >> 8][dc + 1].y >> 12);
+          } else if (P.unit >= 0 && same && P.unit >= ((M.w >> 16) & 0xff) &&
                      P.unit + 6 <= ((M.w >> 24) & 0xff)) {
             pair_row(P, &Q.tile[(k >= h * RS_H ? H.tbase : 0) + (short)(M.w & 0xffff) + P.unit],
-                     Q.eA[e], __int_as_float(M.z), orow, out16);
-          } else {
+                     Q.eA[e], __int_as_float(M.z), orow);
+          } else if (P.in) {
             miss |= 1u << (k - k0);
           }
         }
@@ -1453,19 +1479,19 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       {
         const unsigned b = __ballot_sync(0xffffffffu, miss != 0);
         if (miss) Q.miss[u] = (unsigned short)miss;
-        if ((t & 31) == 0) Q.missb[u >> 5] = b;
+        if ((u & 31) == 0) Q.missb[u >> 5] = b;
       }
       __syncthreads();
 
       // ---- [C] the pixels the pair path left, then per-pixel rows and the
       // pixels left to the per-pixel path
-      if (S.strip[0].missb[0] | S.strip[0].missb[1] | S.strip[1].missb[0] | S.strip[1].missb[1]) {
+      if (Q.missb[0] | Q.missb[1]) {
         slow_pixels(Q, J, u, k0, k1 - k0, h * RS_H, H.tbase, cN,
                     J.out + (long)(rb + k0 - J.row0) * J.out_pitch + c0);
         __syncthreads();
       }
       if (Q.gen_any || (any & HG_PIX)) pixel_pass(S, Q, J, u, k0, rb + k0, k1 - k0, c0, cN);
-      if (S.strip[0].gen_any | S.strip[1].gen_any) {
+      if (Q.gen_any) {
         __syncthreads();
         if (u < 2 * RS_H * 4) (&Q.gen[0][0])[u] = 0u;
         if (u == 0) Q.gen_any = 0;
@@ -1479,8 +1505,12 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
   }
 }
 
+static_assert(6 * (sizeof(RsShared<true>) + 1024) <= 228 * 1024 &&
+                  6 * (sizeof(RsShared<false>) + 1024) <= 228 * 1024,
+              "6 CTAs per SM");
+
 template <bool kSplit>
-__global__ void __launch_bounds__(RS_NT, 3)
+__global__ void __launch_bounds__(RS_NT, 6)
     resample_kernel(const __grid_constant__ RsBatch B) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RsShared<kSplit> &S = *reinterpret_cast<RsShared<kSplit> *>(smem_raw);
@@ -1613,7 +1643,7 @@ int fill_resample_job(const tops_resample_job &u, ResampleJob &J) {
   J.midL = 0.5 * ((double)u.mbox[2] + (double)u.mbox[3]);
   J.invL = 1.0 / (0.25 * ((double)u.mbox[3] - (double)u.mbox[2]));
   const int mpix = u.mbox[1] - u.mbox[0] + 1;
-  J.strips = (mpix + RS_NS * RS_TW - 1) / (RS_NS * RS_TW);   // strip pairs
+  J.strips = (mpix + RS_TW - 1) / RS_TW;
   J.seg_rows = RS_MAXSEG;
   J.segs = (J.nrows + RS_MAXSEG - 1) / RS_MAXSEG;
   return TOPS_OK;
@@ -1648,7 +1678,7 @@ static int launch_resample_t(const ResampleJob *jobs, int njobs, const TileCfg &
   // Outputs do not depend on it.
   int seg_rows = cfg.seg_rows;
   if (!seg_rows) {
-    static const int kSegs[] = {252, 204, 168, 144, 120, 96, 84, 72, 60, 48, 36, 24};
+    static const int kSegs[] = {252, 204, 168, 144, 120, 96, 84, 72, 60, 48, 36, 24, 12};
     long best = 0;
     for (int sr : kSegs) {
       long items = 0;
