@@ -41,9 +41,9 @@ typedef struct {
   int precision;            /* resample deramp phase: TOPS_PREC_SPLIT (default)
                                or TOPS_PREC_FP64 */
   int compensated;          /* 1: ESD phasor sums with Kahan compensation and
-                               coherence window sums without the sliding
-                               update (pairwise per output); 0 (default): the
-                               plain fixed-order FP32 sums */
+                               coherence with its reciprocal square roots
+                               refined (its window sums are trees in both
+                               modes); 0 (default): plain fixed-order FP32 */
   int coh_overlap;          /* 1: the ReSlaveESD resample in up to 3 chunks of
                                bursts, the coherence of each chunk on a second
                                stream as soon as it is resampled, overlapping
@@ -181,9 +181,10 @@ typedef struct tops_batch tops_batch;
 
 /* Tile and scheduling of the resample and coherence launches. */
 typedef struct {
-  int rs_seg_rows;      /* resample output rows per work item, 12..252 (0: 252) */
+  int rs_seg_rows;      /* resample output rows per work item, 12..252 (0: chosen
+                           by the number of items) */
   int rs_persistent;    /* 1: persistent kernel pulling items from a queue */
-  int coh_seg_rows;     /* coherence rows per work item, 8..512 (0: 128) */
+  int coh_seg_rows;     /* coherence rows per work item, 8..512 (0: chosen) */
   int coh_persistent;
 } tops_tune;
 

@@ -8,23 +8,32 @@
 // with gamma = 0 where |s(r,c)| < 0.001.  The reference leaves the pad
 // uninitialised (EstCoh.cu:581-583); here it is zero.
 //
-// B200 design: one CTA per (strip of CO_TW columns, segment of rows).  Each
-// thread owns one loaded column and walks the segment in groups of CO_GR
-// rows.  For the common azimuth windows (template WAZ = 3 and the
-// reference's 6) the products (m s*, |s|^2, |m|^2) of the last WAZ - 1 input
-// rows stay in registers from one group to the next, so every input row is
-// read once, and the loads of the next group are issued before the
-// horizontal pass of the current one, so HBM latency overlaps the shared-
-// memory work.  The vertical sums go to shared memory; the horizontal box is
-// a sliding sum over CO_CPI consecutive outputs per thread, written with
-// 16-byte stores.  Other window heights (WAZ = 0) reload the halo rows of
-// each group.  HBM traffic is the algorithmic 4 + 8 + 4 bytes per pixel plus
-// the column halo.
-#include <cuda.h>
-#include <cudaTypedefs.h>
+// B200 design: no block barriers.  A warp owns a strip of 128 loaded columns,
+// four per lane, and marches down a segment of rows.  Its rows come through a
+// private ring of 4 slots in shared memory filled by asynchronous copies (three
+// 16-byte ones per lane and row, or single samples where rows do not start on
+// 16-byte boundaries; both zero-fill outside the image).  The products (m s*,
+// |s|^2, |m|^2) of the last winAz - 1 rows stay in registers, so every input
+// row is read once; output rows go in pairs whose common rows are summed once.
+// The horizontal sums come from prefix, suffix and whole sums of the lanes' four
+// columns that the lanes exchange with shuffles.  No sum is updated by
+// subtraction, so the rounding error does not grow along a row or with the
+// window (7.8e-8 relative RMS at 10 x 3, 8.0e-8 at 24 x 6).
+//
+// What bounds it: instruction issue (10 x 3: 64 per output pixel, 11 of them
+// packed adds and 9 shuffles; about 65% of the issue slots) at 16 warps per SM
+// by registers, then the 16 bytes per pixel of memory traffic.  Measured, in
+// us, against a kernel that staged the products of a block in shared memory
+// and summed windows by sliding updates behind block barriers:
+//   1500 x 21000, 10 x 3   154 -> 102 (4.9 TB/s)     24 x 6   243 -> 158
+//   1523 x 8193, 5 x 5     147 -> 49                 1200 x 7000, 30 x 9  180 -> 134
+//   1200 x 7000, 17 x 2    129 -> 49                 300 x 512, 10 x 3    66 -> 9
+//   800 x 9000, 2 x 1      111 -> 24                 33 x 7               152 -> 77
+// Rows prefetched into registers instead of the ring took 121 us (10 x 3) and
+// 229 us (24 x 6); a ring of 7 slots 109 us; 18 warps per SM, by spilling, 149.
 #include <cuda_runtime.h>
 
-#include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -32,25 +41,20 @@
 
 namespace tops {
 
-constexpr int CO_NT = 256;
-constexpr int CO_TW = 224;   // output columns per strip (win_rg <= 33)
-constexpr int CO_GR = 8;     // rows per group
-constexpr int CO_SEG = 128;  // rows per work item
-constexpr int CO_CPI = 8;    // output columns per horizontal item
+constexpr int CO_CPL = 4;          // columns per lane
+constexpr int CO_NW = 2;           // warps (adjacent strips) per CTA
+constexpr int CO_NT = 32 * CO_NW;
+constexpr int CO_D = 4;            // slots per warp: the row read last and 3 in flight
+constexpr int CO_ROW = 2048;       // bytes of a slot: 128 columns of 4 and of 8, and a gap
 constexpr int CO_MAXJOBS = 32;
-constexpr int CO_MAX_WIN_RG = CO_NT - CO_TW + 1;
+constexpr int CO_MAX_WIN_RG = 33;
 
 struct CoBatch {
   int njobs, total_items, win_rg, win_az;
-  int compensated;         // 1: each output's window summed pairwise
+  int nl, nr;              // lanes whose columns only feed the windows: left, right
+  int compensated;         // 1: both reciprocal square roots refined by a Newton step
   int *counter;            // persistent launch: work-item queue (else null)
   CohJob jobs[CO_MAXJOBS];
-};
-
-struct CoShared {
-  float4 V[CO_GR][pad8(CO_NT)];      // vertical sums (re, im, |s|^2, |m|^2), pad8(x)
-  float spow[CO_GR][pad8(CO_NT)];   // |s|^2 of the centre pixel, pad8(x)
-  int next_item;                     // persistent launch: the item just taken
 };
 
 __device__ __forceinline__ float4 coh_product(short2 m, float2 s) {
@@ -59,583 +63,554 @@ __device__ __forceinline__ float4 coh_product(short2 m, float2 s) {
                      mi * s.x - mr * s.y, s.x * s.x + s.y * s.y, mr * mr + mi * mi);
 }
 
-// a += b with packed FP32x2 adds
-__device__ __forceinline__ void add4(float4 &a, const float4 &b) {
+// a + b with packed FP32x2 adds
+__device__ __forceinline__ float4 add4(const float4 &a, const float4 &b) {
   const float2 c = __fadd2_rn(make_float2(a.x, a.y), make_float2(b.x, b.y));
   const float2 p = __fadd2_rn(make_float2(a.z, a.w), make_float2(b.z, b.w));
-  a = make_float4(c.x, c.y, p.x, p.y);
+  return make_float4(c.x, c.y, p.x, p.y);
 }
-
-// Pairwise sum of n window columns V[idx(0)] .. V[idx(n - 1)] (the
-// compensated mode: no sliding update, rounding error O(log n)).
-template <class Idx>
-__device__ __forceinline__ float4 window_pairwise(const float4 *V, int n, Idx idx) {
-  float4 p[16];
-  int m = 0;
-  for (int i = 0; i + 1 < n; i += 2, m++) {
-    p[m] = V[idx(i)];
-    add4(p[m], V[idx(i + 1)]);
-  }
-  if (n & 1) p[m++] = V[idx(n - 1)];
-  for (int h = 1; h < m; h <<= 1)
-    for (int i = 0; i + h < m; i += 2 * h) add4(p[i], p[i + h]);
-  return p[0];
+// the value of lane + off
+__device__ __forceinline__ float4 lane4(const float4 &v, int off) {
+  const int src = (int)(threadIdx.x & 31) + off;
+  return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+                     __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
 }
-
-// Horizontal pass of one group: CO_CPI consecutive outputs per item.  The
-// amplitude mask |s| < 0.001 of the reference (EstCoh.cu:393, 446) is
-// evaluated as |s|^2 < 1e-6.  WRG > 0: range window known at compile time;
-// an item starts at a multiple of 8 columns, so pad8(cg + i) = pad8(cg) +
-// pad8(i) and every shared-memory offset below is a constant.
-template <int WRG, bool COMP>
-__device__ __forceinline__ void coh_horizontal(const CoShared &S, const CohJob &J, int tid,
-                                               int rg, int gr, int c0, int cN, int win_rg_rt,
-                                               int dx_rt) {
-  constexpr int NG = CO_TW / CO_CPI;
-  static_assert(CO_CPI % 8 == 0, "items must start at multiples of 8 columns");
-  const int win_rg = WRG > 0 ? WRG : win_rg_rt;
-  const int dx = WRG > 0 ? (WRG - 1) / 2 : dx_rt;
-  for (int it = tid; it < gr * NG; it += CO_NT) {
-    const int k = it / NG;
-    const int cg = (it - k * NG) * CO_CPI;
-    if (cg >= cN) continue;
-    const float4 *V = &S.V[k][pad8(cg)];
-    const float *Jd = &S.spow[k][pad8(cg)];
-    float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (WRG > 0) {
-#pragma unroll
-      for (int i = 0; i < WRG; i++) add4(w, V[pad8(i)]);
-    } else {
-      for (int i = 0; i < win_rg; i++) add4(w, V[pad8(i)]);
-    }
-    float out[CO_CPI];
-#pragma unroll
-    for (int u = 0; u < CO_CPI; u++) {
-      if (COMP) {
-        w = window_pairwise(V, win_rg, [&](int i) { return pad8(u + i); });
-      } else if (u > 0) {
-        const float4 a = V[pad8(u - 1 + win_rg)];
-        const float4 b = V[pad8(u - 1)];
-        const float2 m1 = make_float2(-1.f, -1.f);
-        const float2 wc = __fadd2_rn(make_float2(w.x, w.y),
-                                     __ffma2_rn(make_float2(b.x, b.y), m1, make_float2(a.x, a.y)));
-        const float2 wp = __fadd2_rn(make_float2(w.z, w.w),
-                                     __ffma2_rn(make_float2(b.z, b.w), m1, make_float2(a.z, a.w)));
-        w = make_float4(wc.x, wc.y, wp.x, wp.y);
-      }
-      // |sum m s*| / sqrt(sum |s|^2 sum |m|^2) as num rsqrt(num) rsqrt(p):
-      // two MUFU reciprocal square roots instead of an IEEE square root
-      // (relative error a few 1e-7)
-      const float p = w.z * w.w;
-      const float num = fmaf(w.x, w.x, w.y * w.y);
-      float g = (p > 0.f && num > 0.f) ? num * rsqrtf(num) * rsqrtf(p) : 0.f;
-      if (Jd[pad8(u + dx)] < 1e-6f) g = 0.f;
-      out[u] = g;
-    }
-    float *orow = J.coh + (long)(rg + k) * J.coh_pitch + c0 + cg;
-    if (cg + CO_CPI <= cN && ((reinterpret_cast<uintptr_t>(orow) & 15) == 0)) {
-#pragma unroll
-      for (int u = 0; u < CO_CPI; u += 4)
-        *reinterpret_cast<float4 *>(orow + u) = make_float4(out[u], out[u + 1], out[u + 2],
-                                                            out[u + 3]);
-    } else {
-#pragma unroll
-      for (int u = 0; u < CO_CPI; u++)
-        if (cg + u < cN) orow[u] = out[u];
-    }
-  }
-}
-
-// One work item (strip x segment of one job); all threads of the CTA call it
-// with the same item.
-template <int WAZ, int WRG, bool COMP>
-__device__ __forceinline__ void coherence_item(CoShared &S, const CoBatch &B, int item) {
-  const int tid = threadIdx.x;
-  int jb = 0;
-  while (jb + 1 < B.njobs && B.jobs[jb + 1].item_begin <= item) jb++;
-  const CohJob &J = B.jobs[jb];
-  const int local = item - J.item_begin;
-  const int strip = local % J.strips, seg = local / J.strips;
-  const int win_rg = B.win_rg;
-  const int win_az = WAZ > 0 ? WAZ : B.win_az;
-  const int dx = (win_rg - 1) / 2, dy = (win_az - 1) / 2;
-  const int c0 = strip * CO_TW;
-  const int cN = min(CO_TW, J.pixels - c0);
-  const int nload = cN + win_rg - 1;
-  const int r_begin = seg * J.seg_rows;
-  const int r_end = min(r_begin + J.seg_rows, J.lines);
-  const int x = c0 - dx + tid;          // this thread's loaded column
-  const bool xin = tid < nload && x >= 0 && x < J.pixels;
-  auto load = [&](int y, short2 &m, float2 &s) {
-    m = make_short2(0, 0);
-    s = make_float2(0.f, 0.f);
-    if (xin && y >= 0 && y < J.lines) {
-      m = J.master[(long)y * J.master_pitch + x];
-      s = J.slave[(long)y * J.slave_pitch + x];
-    }
+template <int OFF>
+__device__ __forceinline__ float4 lane4(const float4 &v) {
+  constexpr int n = OFF < 0 ? -OFF : OFF;
+  auto s = [](float x) {
+    return OFF < 0 ? __shfl_up_sync(0xffffffffu, x, n) : __shfl_down_sync(0xffffffffu, x, n);
   };
-
-  if constexpr (WAZ > 0) {
-    // products of input rows: q[0 .. WAZ-2] carried, then the group's rows
-    constexpr int NQ = WAZ > 0 ? WAZ - 1 : 1;
-    float4 q[NQ];
-    {
-      // rows r_begin - dy .. r_begin - dy + WAZ - 2 (the first group's halo)
-#pragma unroll
-      for (int j = 0; j < NQ; j++) {
-        short2 m;
-        float2 s;
-        load(r_begin - dy + j, m, s);
-        q[j] = coh_product(m, s);
-      }
-    }
-    // loads of the first group: input rows r_begin - dy + WAZ - 1 + k
-    short2 mv[CO_GR];
-    float2 sv[CO_GR];
-#pragma unroll
-    for (int k = 0; k < CO_GR; k++) load(r_begin - dy + WAZ - 1 + k, mv[k], sv[k]);
-    for (int rg = r_begin; rg < r_end; rg += CO_GR) {
-      const int gr = min(CO_GR, r_end - rg);
-      float4 p[NQ + CO_GR];
-#pragma unroll
-      for (int j = 0; j < NQ; j++) p[j] = q[j];
-#pragma unroll
-      for (int k = 0; k < CO_GR; k++) p[NQ + k] = coh_product(mv[k], sv[k]);
-      // issue the next group's loads now; they land during the rest
-      const int rn = rg + CO_GR;
-      if (rn < r_end) {
-#pragma unroll
-        for (int k = 0; k < CO_GR; k++) load(rn - dy + WAZ - 1 + k, mv[k], sv[k]);
-      }
-#pragma unroll
-      for (int k = 0; k < CO_GR; k++) {
-        float4 a = p[k];
-#pragma unroll
-        for (int j = 1; j < WAZ; j++) add4(a, p[k + j]);
-        S.V[k][pad8(tid)] = a;
-        S.spow[k][pad8(tid)] = p[k + dy].z;
-      }
-#pragma unroll
-      for (int j = 0; j < NQ; j++) q[j] = p[CO_GR + j];
-      __syncthreads();
-      coh_horizontal<WRG, COMP>(S, J, tid, rg, gr, c0, cN, win_rg, dx);
-      __syncthreads();
-    }
-  } else {
-    for (int rg = r_begin; rg < r_end; rg += CO_GR) {
-      const int gr = min(CO_GR, r_end - rg);
-      // vertical pass: input rows rg-dy .. rg-dy+gr+win_az-2
-      float4 acc[CO_GR];
-      float spow[CO_GR];
-#pragma unroll
-      for (int k = 0; k < CO_GR; k++) {
-        acc[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        spow[k] = 0.f;
-      }
-      const int nin = gr + win_az - 1;
-      for (int qi = 0; qi < nin; qi++) {
-        short2 m;
-        float2 sl;
-        load(rg - dy + qi, m, sl);
-        const float4 pr = coh_product(m, sl);
-#pragma unroll
-        for (int k = 0; k < CO_GR; k++) {
-          const int j = qi - k;
-          if (j >= 0 && j < win_az) add4(acc[k], pr);
-          if (qi == k + dy) spow[k] = pr.z;
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < CO_GR; k++) {
-        S.V[k][pad8(tid)] = acc[k];
-        S.spow[k][pad8(tid)] = spow[k];
-      }
-      __syncthreads();
-      coh_horizontal<WRG, COMP>(S, J, tid, rg, gr, c0, cN, win_rg, dx);
-      __syncthreads();
-    }
-  }
+  return make_float4(s(v.x), s(v.y), s(v.z), s(v.w));
 }
 
-// COMP: the compensated window sums (a separate instantiation, so the plain
-// kernels carry none of its code or registers)
-template <int WAZ, int WRG, bool COMP>
-__global__ void __launch_bounds__(CO_NT, 3) coherence_kernel(const __grid_constant__ CoBatch B) {
-  __shared__ CoShared S;
-  // one work item per CTA, or (persistent) items from the queue until it
-  // is empty; a single call site keeps one inlined copy of the item code
-  int item = blockIdx.x;
-  if (B.counter) {
-    if (threadIdx.x == 0) S.next_item = atomicAdd(B.counter, 1);
-    __syncthreads();
-    item = S.next_item;
-    __syncthreads();
-  }
-  while (item < B.total_items) {
-    coherence_item<WAZ, WRG, COMP>(S, B, item);
-    if (!B.counter) break;
-    if (threadIdx.x == 0) S.next_item = atomicAdd(B.counter, 1);
-    __syncthreads();
-    item = S.next_item;
-    __syncthreads();
-  }
-}
-
-// ------------------------------------------------ TMA-staged variant
-// For the pipeline's 10-sample and the reference driver's 24-sample range
-// windows.  A CTA of CT_NT threads owns a strip of TW output columns and a
-// segment of rows; its input rows come in chunks of CT_CH rows x CT_LW
-// columns (master as 32-bit, slave as 64-bit elements), each chunk one
-// cp.async.bulk.tensor box per image on an mbarrier, CT_NST - 1 chunks ahead
-// of the one being summed.  The box starts XOFF columns left of the strip:
-// dx rounded up to a multiple of 4, so every box's x coordinate is 16-byte
-// aligned in both images; the copy engine fills rows and columns outside the
-// image with zeros -- the zero pad.  The
-// vertical sums are those of coherence_item; the horizontal sliding sum
-// restarts every CT_CPI = 4 outputs instead of every CO_CPI = 8 (measured
-// faster: 0.398 against 0.490 ms for 3 bursts of 1500 x 21000), so the two
-// kernels agree to FP32 rounding of the window sums (a few 1e-7).
-constexpr int CT_NT = 256;
-constexpr int CT_LW = 256;                 // loaded columns (box width)
-constexpr int CT_CH = 4;                   // rows per chunk (box height)
-constexpr int CT_NST = 4;                  // chunk slots
-constexpr int CT_CPI = 4;                  // outputs per horizontal item
-constexpr int CT_SEG = 256;                // rows per work item
-constexpr int CT_MAXJOBS = 16;
-constexpr unsigned long long CT_WAIT_NS = 2000000000ull;   // a chunk is given up after 2 s
-// Geometry of a range window of WRG samples: the box starts XOFF columns
-// left of the strip, the window of the strip's first output starts B0
-// columns into the box, and a strip has TW outputs.
-template <int WRG>
-struct CtWin {
-  static constexpr int DX = (WRG - 1) / 2;
-  static constexpr int XOFF = (DX + 3) & ~3;
-  static constexpr int B0 = XOFF - DX;
-  static constexpr int TW = WRG == 10 ? 240 : ((CT_LW - XOFF - (WRG - 1 - DX)) & ~(CT_CPI - 1));
-  static_assert(XOFF % 4 == 0, "box x coordinates stay 16-byte aligned");
-  static_assert(XOFF + TW + WRG - 1 - DX <= CT_LW, "the strip's boxes cover its windows");
-  static_assert(TW % CT_CPI == 0 && CT_CH * (TW / CT_CPI) <= CT_NT, "one horizontal item per thread");
-};
-
-__host__ __device__ constexpr int pad4(int x) { return x + (x >> 2); }
-
-struct __align__(64) CtBatch {
-  CUtensorMap tm_m[CT_MAXJOBS];   // master: int32 [lines][pixels], box CT_LW x CT_CH
-  CUtensorMap tm_s[CT_MAXJOBS];   // slave: 64-bit [lines][pixels], same box
-  CohJob jobs[CT_MAXJOBS];
-  int njobs, total_items;
-  int compensated;                // 1: each output's window summed pairwise
-  int *counter;                   // persistent launch: work-item queue (else null)
-};
-
-struct __align__(128) CtShared {
-  int m[CT_NST][CT_CH][CT_LW];          // master chunks (CInt16 pairs)
-  float2 s[CT_NST][CT_CH][CT_LW];       // slave chunks
-  float4 V[CT_CH][pad4(CT_LW)];         // vertical sums (re, im, |s|^2, |m|^2)
-  float spow[CT_CH][pad4(CT_LW)];       // |s|^2 of the centre pixel
-  unsigned long long full[CT_NST];      // one mbarrier per slot
-  int next_item;
-};
-
-__device__ int g_coh_wait_faults;       // chunks whose wait ran out (0 normally)
-
-__device__ __forceinline__ unsigned ct_smem(const void *p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void ct_mbar_init(unsigned long long *bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(ct_smem(bar)) : "memory");
-}
-__device__ __forceinline__ void ct_expect_tx(unsigned long long *bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(ct_smem(bar)),
-               "r"(bytes)
+// Asynchronous global -> shared copies of B bytes: n from src, then zeros.
+template <int B>
+__device__ __forceinline__ void co_copy(unsigned d, const void *src, int n) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(d), "l"(src), "n"(B),
+               "r"(n)
                : "memory");
 }
-__device__ __forceinline__ bool ct_try_wait(unsigned long long *bar, unsigned parity) {
-  unsigned ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      " selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(ct_smem(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void ct_tma_2d(void *dst, const CUtensorMap *tm, int x, int y,
-                                          unsigned long long *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3}], [%4];" ::"r"(ct_smem(dst)),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(ct_smem(bar))
-      : "memory");
-}
-__device__ __forceinline__ unsigned long long ct_now_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-// Waits for the slot's chunk for at most CT_WAIT_NS of wall time (the
-// bound is on time, not on polls: a poll may suspend the thread); false if
-// it never arrived (recorded in g_coh_wait_faults).
-__device__ __forceinline__ bool ct_wait(unsigned long long *bar, unsigned parity) {
-  if (ct_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = ct_now_ns();
-  do {
-    if (ct_try_wait(bar, parity)) return true;
-  } while (ct_now_ns() - t0 < CT_WAIT_NS);
-  return false;
+
+// A lane's column sums: the single columns, the whole, first two, first three,
+// last two and last three of them.
+struct CoSums {
+  float4 v[CO_CPL], f, p2, p3, s2, s3;
+  // the sum of the first / last N columns
+  template <int N>
+  __device__ __forceinline__ const float4 &first() const {
+    return N == 1 ? v[0] : N == 2 ? p2 : N == 3 ? p3 : f;
+  }
+  template <int N>
+  __device__ __forceinline__ const float4 &last() const {
+    return N == 1 ? v[3] : N == 2 ? s2 : N == 3 ? s3 : f;
+  }
+};
+
+// Windows of W <= 6 columns, W at compile time: column a of the window is in
+// lane a >> 2, and at most one lane is whole.
+template <int W>
+__device__ __forceinline__ void box_small(const CoSums &c, float4 (&o)[CO_CPL]) {
+  auto out = [&](auto uu) {
+    constexpr int u = decltype(uu)::value;
+    constexpr int a = u - (W - 1) / 2, b = a + W - 1;
+    constexpr int lo = (a + 64) / 4 - 16, hi = (b + 64) / 4 - 16;
+    constexpr int ka = a - 4 * lo, kb = b - 4 * hi;
+    if constexpr (lo == hi) {
+      float4 t = ka == 0 ? c.template first<kb + 1>() : c.v[ka];
+      if constexpr (ka == 1 && kb == 3) t = c.s3;
+      if constexpr (ka == 2 && kb == 3) t = c.s2;
+      if constexpr (ka == 1 && kb == 2) t = add4(c.v[1], c.v[2]);
+      o[u] = lo == 0 ? t : lane4<lo>(t);
+    } else {
+      const float4 &e0 = c.template last<4 - ka>(), &e1 = c.template first<kb + 1>();
+      float4 t = lo == 0 ? e0 : lane4<lo>(e0);
+      if constexpr (hi > lo + 1) t = add4(t, lo + 1 == 0 ? c.f : lane4<lo + 1>(c.f));
+      o[u] = add4(t, hi == 0 ? e1 : lane4<hi>(e1));
+    }
+  };
+  out(std::integral_constant<int, 0>());
+  out(std::integral_constant<int, 1>());
+  out(std::integral_constant<int, 2>());
+  out(std::integral_constant<int, 3>());
 }
 
-// One work item; returns false (all threads) when a chunk never arrived.
-// `seq` counts the chunks this CTA has consumed (slot and mbarrier phase).
-template <int WAZ, int WRG, bool COMP>
-__device__ __forceinline__ bool coh_tma_item(CtShared &S, const CtBatch &B, int item,
-                                             unsigned &seq) {
-  using Win = CtWin<WRG>;
-  constexpr int DY = (WAZ - 1) / 2;
-  constexpr int NQ = WAZ - 1;
-  constexpr int H = (NQ + CT_CH - 1) / CT_CH;   // chunks holding the first halo rows
-  constexpr unsigned kChunkBytes = CT_CH * CT_LW * (4 + 8);
-  const int tid = threadIdx.x;
+// Windows of 7 columns or more: some lanes are whole in the windows of all four
+// columns; before them column u's window holds another Q + 3 - u columns (Q 0
+// to 3), after them Q + u.
+template <int Q>
+__device__ __forceinline__ void box_left(const CoSums &c, int l, float4 (&o)[CO_CPL]) {
+  if constexpr (Q == 0) {                   // 3 2 1 0
+    o[0] = lane4(c.s3, l);
+    o[1] = lane4(c.s2, l);
+    o[2] = lane4(c.v[3], l);
+    o[3] = make_float4(0.f, 0.f, 0.f, 0.f);
+  } else if constexpr (Q == 1) {            // 4 3 2 1
+    o[0] = lane4(c.f, l);
+    o[1] = lane4(c.s3, l);
+    o[2] = lane4(c.s2, l);
+    o[3] = lane4(c.v[3], l);
+  } else if constexpr (Q == 2) {            // 5 4 3 2
+    const float4 w = lane4(c.f, l);
+    o[0] = add4(lane4(c.v[3], l - 1), w);
+    o[1] = w;
+    o[2] = lane4(c.s3, l);
+    o[3] = lane4(c.s2, l);
+  } else {                                  // 6 5 4 3
+    const float4 w = lane4(c.f, l);
+    o[0] = add4(lane4(c.s2, l - 1), w);
+    o[1] = add4(lane4(c.v[3], l - 1), w);
+    o[2] = w;
+    o[3] = lane4(c.s3, l);
+  }
+}
+template <int Q>
+__device__ __forceinline__ void box_right(const CoSums &c, int l, float4 (&o)[CO_CPL]) {
+  if constexpr (Q == 0) {                   // 0 1 2 3
+    o[1] = add4(o[1], lane4(c.v[0], l));
+    o[2] = add4(o[2], lane4(c.p2, l));
+    o[3] = add4(o[3], lane4(c.p3, l));
+  } else if constexpr (Q == 1) {            // 1 2 3 4
+    o[0] = add4(o[0], lane4(c.v[0], l));
+    o[1] = add4(o[1], lane4(c.p2, l));
+    o[2] = add4(o[2], lane4(c.p3, l));
+    o[3] = add4(o[3], lane4(c.f, l));
+  } else if constexpr (Q == 2) {            // 2 3 4 5
+    const float4 w = lane4(c.f, l);
+    o[0] = add4(o[0], lane4(c.p2, l));
+    o[1] = add4(o[1], lane4(c.p3, l));
+    o[2] = add4(o[2], w);
+    o[3] = add4(o[3], add4(w, lane4(c.v[0], l + 1)));
+  } else {                                  // 3 4 5 6
+    const float4 w = lane4(c.f, l);
+    o[0] = add4(o[0], lane4(c.p3, l));
+    o[1] = add4(o[1], w);
+    o[2] = add4(o[2], add4(w, lane4(c.v[0], l + 1)));
+    o[3] = add4(o[3], add4(w, lane4(c.p2, l + 1)));
+  }
+}
+template <int WRG>
+__device__ __forceinline__ void box_large(const CoSums &c, int win, int dx,
+                                          float4 (&o)[CO_CPL]) {
+  const int ql = (dx + 1) & 3, qr = (win - dx) & 3;
+  const int l0 = (ql + 3 - dx) / 4, l1 = (win - dx - qr) / 4;   // the whole lanes l0 .. l1 - 1
+  // 1 to 7 whole lanes, from the sums of 1, 2 and 4 lanes from each lane on
+  const int n = l1 - l0;
+  int l = l0;
+  bool any = false;
+  float4 g = c.f, m = g;
+  auto piece = [&](int lanes) {
+    const float4 y = WRG > 0 && l == 0 ? g : lane4(g, l);
+    m = any ? add4(m, y) : y;
+    any = true;
+    l += lanes;
+  };
+  if (n & 1) piece(1);
+  if (n >= 2) g = add4(g, lane4<1>(g));
+  if (n & 2) piece(2);
+  if (n >= 4) {
+    g = add4(g, lane4<2>(g));
+    piece(4);
+  }
+  switch (ql) {
+    case 0: box_left<0>(c, l0 - 1, o); break;
+    case 1: box_left<1>(c, l0 - 1, o); break;
+    case 2: box_left<2>(c, l0 - 1, o); break;
+    default: box_left<3>(c, l0 - 1, o);
+  }
+  switch (qr) {
+    case 0: box_right<0>(c, l1, o); break;
+    case 1: box_right<1>(c, l1, o); break;
+    case 2: box_right<2>(c, l1, o); break;
+    default: box_right<3>(c, l1, o);
+  }
+  // the ends first: one rounding at the size of the whole sum
+#pragma unroll
+  for (int u = 0; u < CO_CPL; u++) o[u] = add4(m, o[u]);
+}
+
+// Horizontal sums o[u] of columns x + u - dx .. x + u - dx + win - 1 (x the
+// lane's first column) from the lanes' vertical sums v.  WRG > 0: the window
+// at compile time; CO_SMALL, CO_LARGE: any of up to 6, of 7 or more columns.
+constexpr int CO_SMALL = 0, CO_LARGE = -1;
+template <int WRG>
+__device__ __forceinline__ void coh_box(const float4 (&v)[CO_CPL], int win, int dx,
+                                        float4 (&o)[CO_CPL]) {
+  CoSums c;
+#pragma unroll
+  for (int i = 0; i < CO_CPL; i++) c.v[i] = v[i];
+  c.p2 = add4(v[0], v[1]);
+  c.s2 = add4(v[2], v[3]);
+  c.p3 = add4(c.p2, v[2]);
+  c.s3 = add4(v[1], c.s2);
+  c.f = add4(c.p2, c.s2);
+  if constexpr (WRG == CO_SMALL) {
+    switch (win) {
+      case 1: box_small<1>(c, o); break;
+      case 2: box_small<2>(c, o); break;
+      case 3: box_small<3>(c, o); break;
+      case 4: box_small<4>(c, o); break;
+      case 5: box_small<5>(c, o); break;
+      default: box_small<6>(c, o);
+    }
+  } else if constexpr (WRG == CO_LARGE) {
+    box_large<0>(c, win, dx, o);
+  } else {
+    box_large<WRG>(c, WRG, (WRG - 1) / 2, o);
+  }
+}
+
+// 1 / sqrt(x); FINE: with a Newton step
+template <bool FINE>
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  if (FINE && x <= 3.4e38f) r = fmaf(0.5f * r, fmaf(-x * r, r, 1.f), r);
+  return r;
+}
+// |sum m s*| / sqrt(sum |s|^2 sum |m|^2) as num rsqrt(num) rsqrt(p): two MUFU
+// reciprocal square roots instead of an IEEE square root (relative error a few
+// 1e-7); the amplitude mask |s| < 0.001 of the reference (EstCoh.cu:393, 446)
+// is evaluated as |s|^2 < 1e-6.  A num below FLT_MIN is a coherence below
+// 1e-15 and taken for 0; above it some |m|^2, a whole number, is not 0, so p
+// is at least 1e-6 where the mask passes.
+template <bool FINE>
+__device__ __forceinline__ float coh_gamma(const float4 &w, float spow) {
+  const float p = w.z * w.w;
+  const float num = fmaf(w.x, w.x, w.y * w.y);
+  const bool ok = num >= 1.17549435e-38f && spow >= 1e-6f;
+  if (FINE && !ok) return 0.f;
+  const float g = num * rsqrt_ftz<FINE>(num) * rsqrt_ftz<FINE>(p);
+  return ok ? g : 0.f;
+}
+
+// One work item: the warp's strip of one segment; no thread synchronises with
+// another warp.  WAZ > 0: the window height at compile time; AL: the input rows
+// start on 16-byte boundaries.
+template <int WAZ, int WRG, bool AL>
+__device__ __forceinline__ void coherence_item(const CoBatch &B, int item,
+                                               unsigned char *stage) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int jb = 0;
   while (jb + 1 < B.njobs && B.jobs[jb + 1].item_begin <= item) jb++;
   const CohJob &J = B.jobs[jb];
   const int local = item - J.item_begin;
-  const int strip = local % J.strips, seg = local / J.strips;
-  const int c0 = strip * Win::TW;
-  const int cN = min(Win::TW, J.pixels - c0);
-  const int r_begin = seg * J.seg_rows;
-  const int r_end = min(r_begin + J.seg_rows, J.lines);
-  const int nout = (r_end - r_begin + CT_CH - 1) / CT_CH;
-  const int T = H + nout;
-  const int x0 = c0 - Win::XOFF;
-  // chunk u holds input rows base(u) .. base(u) + CT_CH - 1: output chunk
-  // u - H's new rows, the halo rows r_begin - DY .. r_begin - DY + NQ - 1
-  // at the end of the first H chunks
-  auto base = [&](int u) { return r_begin + CT_CH * (u - H) + (NQ - DY); };
-  auto issue = [&](int u) {
-    const unsigned slot = (seq + u) % CT_NST;
-    ct_expect_tx(&S.full[slot], kChunkBytes);
-    ct_tma_2d(&S.m[slot][0][0], &B.tm_m[jb], x0, base(u), &S.full[slot]);
-    ct_tma_2d(&S.s[slot][0][0], &B.tm_s[jb], x0, base(u), &S.full[slot]);
+  const int seg = local / J.strips;
+  constexpr int DY = WAZ > 0 ? (WAZ - 1) / 2 : 0;
+  constexpr int R = WAZ > 0 ? WAZ - 1 : 0; // rows of products kept
+  const int win = WRG > 0 ? WRG : B.win_rg, dx = (win - 1) / 2;
+  const int nl = WRG == 10 ? 1 : WRG == 24 ? 3 : B.nl, nr = WRG == 10 ? 2 : WRG == 24 ? 3 : B.nr;
+  const int tw = CO_CPL * (32 - nl - nr);  // output columns of a warp
+  const int x = ((local - seg * J.strips) * CO_NW + warp) * tw + CO_CPL * (lane - nl);
+  if (x - CO_CPL * (lane - nl) >= J.pixels) return;   // the whole warp
+  const int r_begin = seg * J.seg_rows, r_end = min(r_begin + J.seg_rows, J.lines);
+  const bool out_lane = lane >= nl && lane < 32 - nr && x < J.pixels;
+  const bool vec_out = out_lane && x + CO_CPL <= J.pixels && J.out_al16;
+  // rows from here on are not needed
+  const int y_end = WAZ > 0 ? min(r_end - DY + R, J.lines) : J.lines;
+  // The warp's copies of a row: 128 columns from xw on.  AL: 16-byte pieces,
+  // one of the master (columns c0 .. c0 + 3) and two of the slave (c1, c1 + 1
+  // and c1 + 64, c1 + 65) per lane; a piece is cut off at the end of the row
+  // (xw is a multiple of 4, so none reaches across column 0) and the copy puts
+  // zeros behind.  Else single columns, xw + lane + 32 k.
+  const int xw = x - CO_CPL * lane;
+  const int c0 = AL ? x : xw + lane, c1 = xw + 2 * lane;
+  auto bytes = [&](int c, int esz) {
+    return c < 0 ? 0 : min(max(J.pixels - c, 0) * esz, 16);
   };
-  if (tid == 0)
-    for (int u = 0; u < CT_NST - 1 && u < T; u++) issue(u);
+  auto clip = [&](int c) { return min(max(c, 0), J.pixels - 1); };
+  const int nb0 = AL ? bytes(c0, 4) : 0, nb1 = AL ? bytes(c1, 8) : 0,
+            nb2 = AL ? bytes(c1 + 64, 8) : 0;
+  const short2 *const m0 = J.master + (AL ? clip(c0) & ~3 : 0);
+  const float2 *const s1 = J.slave + (AL ? clip(c1) & ~1 : 0);
+  const int s2 = AL ? (clip(c1 + 64) & ~1) - (clip(c1) & ~1) : 0;
+  unsigned char *const mine = stage + warp * (CO_D * CO_ROW);
+  const unsigned base = (unsigned)__cvta_generic_to_shared(mine);
+  // copies left of the item before end here: no slot is written twice at a time
+  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+  __syncwarp();
+  unsigned wr = 0;                         // the slot to write next (byte offset)
+  auto after = [](unsigned slot) { return (slot + CO_ROW) & (CO_D * CO_ROW - 1); };
+  int y = 0;                               // the next row to copy, and where it is
+  const short2 *mp = m0;
+  const float2 *sp = s1;
+  auto seek = [&](int row) {
+    y = row;
+    const long yc = min(max(row, 0), J.lines - 1);
+    mp = m0 + yc * J.master_pitch;
+    sp = s1 + yc * J.slave_pitch;
+  };
+  // copies row y's columns into the next slot; zeros outside the image
+  auto issue = [&]() {
+    const bool row = (unsigned)y < (unsigned)y_end;
+    const unsigned d = base + wr;
+    if (AL) {
+      co_copy<16>(d + 16 * lane, mp, row ? nb0 : 0);
+      co_copy<16>(d + 512 + 16 * lane, sp, row ? nb1 : 0);
+      co_copy<16>(d + 1024 + 16 * lane, sp + s2, row ? nb2 : 0);
+    } else {
+#pragma unroll
+      for (int k = 0; k < CO_CPL; k++) {
+        const int c = c0 + 32 * k, o = clip(c);
+        const bool ok = row && c == o;
+        co_copy<4>(d + 4 * (lane + 32 * k), mp + o, ok ? 4 : 0);
+        co_copy<8>(d + 512 + 8 * (lane + 32 * k), sp + o, ok ? 8 : 0);
+      }
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    wr = after(wr);
+    if ((unsigned)y < (unsigned)(y_end - 1)) {
+      mp += J.master_pitch;
+      sp += J.slave_pitch;
+    }
+    y++;
+  };
+  // the oldest row in flight: its products.  The barrier shows every lane's
+  // copies to the warp, and lets the slot read last be written again.
+  auto take = [&](float4 (&p)[CO_CPL]) {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(CO_D - 2) : "memory");
+    __syncwarp();
+    const unsigned char *q = mine + after(wr);
+    const int4 a = *reinterpret_cast<const int4 *>(q + 16 * lane);
+    const float4 b = *reinterpret_cast<const float4 *>(q + 512 + 32 * lane);
+    const float4 c = *reinterpret_cast<const float4 *>(q + 528 + 32 * lane);
+    const int m[CO_CPL] = {a.x, a.y, a.z, a.w};
+    const float2 sv[CO_CPL] = {make_float2(b.x, b.y), make_float2(b.z, b.w),
+                               make_float2(c.x, c.y), make_float2(c.z, c.w)};
+#pragma unroll
+    for (int i = 0; i < CO_CPL; i++)
+      p[i] = coh_product(*reinterpret_cast<const short2 *>(&m[i]), sv[i]);
+  };
+  float *orow = J.coh + (long)r_begin * J.coh_pitch + x;
+  // the next output row
+  auto store = [&](const float4 (&o)[CO_CPL], const float (&c)[CO_CPL]) {
+    float g[CO_CPL];
+#pragma unroll
+    for (int u = 0; u < CO_CPL; u++) g[u] = coh_gamma<false>(o[u], c[u]);
+    if (B.compensated) {
+#pragma unroll
+      for (int u = 0; u < CO_CPL; u++) g[u] = coh_gamma<true>(o[u], c[u]);
+    }
+    if (vec_out) {
+      *reinterpret_cast<float4 *>(orow) = make_float4(g[0], g[1], g[2], g[3]);
+    } else if (out_lane) {
+#pragma unroll
+      for (int u = 0; u < CO_CPL; u++)
+        if (x + u < J.pixels) orow[u] = g[u];
+    }
+    orow += J.coh_pitch;
+  };
 
-  float4 q[NQ > 0 ? NQ : 1];
-#pragma unroll
-  for (int j = 0; j < NQ; j++) q[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int t = tid;                       // loaded column
-  bool ok = true;
-  for (int u = 0; u < T; u++) {
-    const unsigned slot = (seq + u) % CT_NST;
-    const unsigned parity = ((seq + u) / CT_NST) & 1u;
-    const bool got = ct_wait(&S.full[slot], parity);
-    if (__syncthreads_or(!got)) {
-      ok = false;
-      if (tid == 0) {
-        atomicAdd(&g_coh_wait_faults, 1);
-        // let the copies in flight land (bounded) before the CTA moves on
-        for (int v = u; v < T && v < u + CT_NST - 1; v++)
-          (void)ct_wait(&S.full[(seq + v) % CT_NST], ((seq + v) / CT_NST) & 1u);
+  if constexpr (WAZ == 0) {
+    // taller windows: 4 output rows at a time over their common input rows
+    constexpr int GR = 4;
+    const int win_az = B.win_az, dy = (win_az - 1) / 2;
+    int rows = 0;                          // copied of the group; groups overlap
+    auto next = [&]() {
+      issue();
+      if (++rows == win_az + GR - 1) {
+        rows = 0;
+        seek(y + 1 - win_az);
       }
-      __syncthreads();
-      break;
-    }
-    // the next chunk into the slot freed by the previous one
-    if (tid == 0 && u + CT_NST - 1 < T) issue(u + CT_NST - 1);
-    if (u < H) {
-      // halo rows: products of input rows r_begin - DY + i
+    };
+    seek(r_begin - dy);
+#pragma unroll 1
+    for (int j = 0; j < CO_D - 1; j++) next();
+    auto add_to = [&](float4 (&a)[CO_CPL], const float4 (&b)[CO_CPL]) {
 #pragma unroll
-      for (int hu = 0; hu < H; hu++) {
-        if (u == hu) {
+      for (int i = 0; i < CO_CPL; i++) a[i] = add4(a[i], b[i]);
+    };
+    for (int r = r_begin; r < r_end; r += GR) {
+      float4 a[GR][CO_CPL], pn[CO_CPL];
+      float c[GR][CO_CPL];
+      // the rows of the first windows only: a[k] = rows k .. GR - 2
 #pragma unroll
-          for (int k = 0; k < CT_CH; k++) {
-            const int i = CT_CH * (hu - H) + NQ + k;
-            if (i >= 0 && i < NQ) {
-              const int mv = S.m[slot][k][t];
-              q[i] = coh_product(*reinterpret_cast<const short2 *>(&mv), S.s[slot][k][t]);
-            }
-          }
-        }
+      for (int k = 0; k < GR - 1; k++) {
+        take(a[k]);
+        next();
+#pragma unroll
+        for (int q = 0; q < k; q++) add_to(a[q], a[k]);
       }
-      continue;
-    }
-    // vertical sums of the chunk's output rows (as coherence_item sums them)
+      // the rows of all windows, the centre rows among them (win_az >= 7)
+      take(a[GR - 1]);
+      next();
 #pragma unroll
-    for (int k = 0; k < CT_CH; k++) {
-      const int mv = S.m[slot][k][t];
-      const float4 p = coh_product(*reinterpret_cast<const short2 *>(&mv), S.s[slot][k][t]);
-      float4 a = NQ > 0 ? q[0] : p;
+      for (int k = 0; k < GR; k++)
 #pragma unroll
-      for (int j = 1; j < NQ; j++) add4(a, q[j]);
-      if (NQ > 0) add4(a, p);
-      S.V[k][pad4(t)] = a;
-      S.spow[k][pad4(t)] = (DY < NQ) ? q[DY < NQ ? DY : 0].z : p.z;
+        for (int i = 0; i < CO_CPL; i++) c[k][i] = a[GR - 1][i].z;
+#pragma unroll 1
+      for (int j = GR; j < win_az; j++) {
+        take(pn);
+        next();
+        add_to(a[GR - 1], pn);
 #pragma unroll
-      for (int j = 0; j + 1 < NQ; j++) q[j] = q[j + 1];
-      if (NQ > 0) q[NQ - 1] = p;
-    }
-    __syncthreads();
-    // horizontal box: CT_CPI consecutive outputs per item; an item starts at
-    // a multiple of 4 columns, so every padded offset below is a constant
-    {
-      constexpr int NG = Win::TW / CT_CPI;
-      constexpr int B0 = Win::B0;
-      const int k = tid / NG;
-      const int cg = (tid - k * NG) * CT_CPI;
-      const int o = r_begin + CT_CH * (u - H) + k;   // output row
-      if (k < CT_CH && o < r_end && cg < cN) {
-        const float4 *V = &S.V[k][pad4(cg)];
-        const float *Jd = &S.spow[k][pad4(cg)];
-        float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < GR; k++)
 #pragma unroll
-        for (int i = 0; i < WRG; i++) add4(w, V[pad4(B0 + i)]);
-        float out[CT_CPI];
+          for (int i = 0; i < CO_CPL; i++) c[k][i] = j <= dy + k ? pn[i].z : c[k][i];
+      }
 #pragma unroll
-        for (int uu = 0; uu < CT_CPI; uu++) {
-          if (COMP) {
-            w = window_pairwise(V, WRG, [&](int i) { return pad4(B0 + uu + i); });
-          } else if (uu > 0) {
-            const float4 a = V[pad4(B0 + uu - 1 + WRG)];
-            const float4 b = V[pad4(B0 + uu - 1)];
-            const float2 m1 = make_float2(-1.f, -1.f);
-            const float2 wc = __fadd2_rn(make_float2(w.x, w.y),
-                                         __ffma2_rn(make_float2(b.x, b.y), m1, make_float2(a.x, a.y)));
-            const float2 wp = __fadd2_rn(make_float2(w.z, w.w),
-                                         __ffma2_rn(make_float2(b.z, b.w), m1, make_float2(a.z, a.w)));
-            w = make_float4(wc.x, wc.y, wp.x, wp.y);
-          }
-          const float pp = w.z * w.w;
-          const float num = fmaf(w.x, w.x, w.y * w.y);
-          float g = (pp > 0.f && num > 0.f) ? num * rsqrtf(num) * rsqrtf(pp) : 0.f;
-          if (Jd[pad4(uu + Win::XOFF)] < 1e-6f) g = 0.f;
-          out[uu] = g;
+      for (int k = 0; k < GR - 1; k++) add_to(a[k], a[GR - 1]);
+      // the rows of the last windows only
+      float4 o[CO_CPL], e[CO_CPL];
+      coh_box<WRG>(a[0], win, dx, o);
+      store(o, c[0]);
+#pragma unroll
+      for (int k = 1; k < GR; k++) {
+        take(pn);
+        next();
+#pragma unroll
+        for (int i = 0; i < CO_CPL; i++) {
+          e[i] = k == 1 ? pn[i] : add4(e[i], pn[i]);
+          a[k][i] = add4(a[k][i], e[i]);
         }
-        float *orow = J.coh + (long)o * J.coh_pitch + c0 + cg;
-        if (cg + CT_CPI <= cN && ((reinterpret_cast<uintptr_t>(orow) & 15) == 0)) {
-#pragma unroll
-          for (int v = 0; v < CT_CPI; v += 4)
-            *reinterpret_cast<float4 *>(orow + v) =
-                make_float4(out[v], out[v + 1], out[v + 2], out[v + 3]);
-        } else {
-#pragma unroll
-          for (int uu = 0; uu < CT_CPI; uu++)
-            if (cg + uu < cN) orow[uu] = out[uu];
-        }
+        coh_box<WRG>(a[k], win, dx, o);
+        if (r + k < r_end) store(o, c[k]);
       }
     }
-    __syncthreads();
+    return;
   }
-  seq += T;
-  return ok;
+
+  // products of the last R rows in a ring: at a step with phase f, row j (0
+  // the oldest) is p[(f + j) % R]
+  constexpr int RR = R > 0 ? R : 1;
+  float4 p[RR][CO_CPL];
+  seek(r_begin - DY);
+#pragma unroll 1
+  for (int j = 0; j < CO_D - 1; j++) issue();
+#pragma unroll
+  for (int j = 0; j < R; j++) {
+    take(p[j]);
+    issue();
+  }
+  // Output rows in pairs: the R rows that both windows hold are summed once.
+  constexpr int UN = R & 1 ? 2 * R : R > 0 ? R : 1;
+  for (int r = r_begin; r < r_end; r += UN) {
+    float4 t[CO_CPL];                      // the sum of a pair's common rows
+#pragma unroll
+    for (int f = 0; f < UN; f++) {
+      if (r + f < r_end) {
+        float4 pn[CO_CPL], v[CO_CPL], o[CO_CPL];
+        take(pn);
+        issue();
+        float sp_c[CO_CPL];
+#pragma unroll
+        for (int i = 0; i < CO_CPL; i++) {
+          // vertical sums; the centre row is row DY of the window
+          if (R == 0) {
+            v[i] = pn[i];
+          } else if (f & 1) {
+            v[i] = add4(t[i], pn[i]);
+          } else {
+            // (the newest row last: it comes from memory)
+            t[i] = p[(f + 1) % RR][i];
+            if (R == 3) t[i] = add4(t[i], p[(f + 2) % RR][i]);
+            if (R > 3) t[i] = add4(t[i], p[(f + 2) % RR][i]);
+            if (R == 4) t[i] = add4(t[i], p[(f + 3) % RR][i]);
+            if (R == 5) t[i] = add4(t[i], add4(p[(f + 3) % RR][i], p[(f + 4) % RR][i]));
+            t[i] = R > 1 ? add4(t[i], pn[i]) : pn[i];
+            v[i] = add4(p[f % RR][i], t[i]);
+          }
+          sp_c[i] = DY < R ? p[(f + DY) % RR][i].z : pn[i].z;
+          if (R > 0) p[f % RR][i] = pn[i];
+        }
+        coh_box<WRG>(v, win, dx, o);
+        store(o, sp_c);
+      }
+    }
+  }
 }
 
-template <int WAZ, int WRG, bool COMP>
-__global__ void __launch_bounds__(CT_NT, 3) coh_tma_kernel(const __grid_constant__ CtBatch B) {
-  extern __shared__ __align__(128) unsigned char ct_smem_raw[];
-  CtShared &S = *reinterpret_cast<CtShared *>(ct_smem_raw);
-  if (threadIdx.x == 0) {
-    for (int k = 0; k < CT_NST; k++) ct_mbar_init(&S.full[k]);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  unsigned seq = 0;
+// Warps per SM: 16 where up to two rows of products are kept, 12 for three and
+// four rows; 8 for the five rows of a height of 6 (24 x 6: 157 us, 179 with 12
+// warps and spills) and for the four window sums of the taller ones (30 x 9:
+// 137 and 142).
+template <int WAZ, int WRG, bool AL>
+__global__ void __launch_bounds__(CO_NT, WAZ == 0 || WAZ == 6 ? 4 : WAZ <= 3 ? 8 : 6)
+    coherence_kernel(const __grid_constant__ CoBatch B) {
+  __shared__ __align__(16) unsigned char stage[CO_NW * CO_D * CO_ROW];
+  __shared__ int next_item;
+  // one work item per CTA, or (persistent) items from the queue until it is
+  // empty; a single call site keeps one inlined copy of the item code
   int item = blockIdx.x;
   if (B.counter) {
-    if (threadIdx.x == 0) S.next_item = atomicAdd(B.counter, 1);
+    if (threadIdx.x == 0) next_item = atomicAdd(B.counter, 1);
     __syncthreads();
-    item = S.next_item;
+    item = next_item;
     __syncthreads();
   }
   while (item < B.total_items) {
-    if (!coh_tma_item<WAZ, WRG, COMP>(S, B, item, seq)) break;
+    coherence_item<WAZ, WRG, AL>(B, item, stage);
     if (!B.counter) break;
-    if (threadIdx.x == 0) S.next_item = atomicAdd(B.counter, 1);
     __syncthreads();
-    item = S.next_item;
+    if (threadIdx.x == 0) next_item = atomicAdd(B.counter, 1);
     __syncthreads();
+    item = next_item;
   }
 }
 
-// cuTensorMapEncodeTiled from the driver (no link-time dependency on it).
-static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static std::once_flag once;
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-  std::call_once(once, [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    (void)cudaGetLastError();
-  });
-  return fn;
+
+// Lanes whose columns only feed the windows, left and right of the outputs.
+static void window_lanes(int win_rg, int &nl, int &nr) {
+  const int dx = (win_rg - 1) / 2;
+  nl = (dx + CO_CPL - 1) / CO_CPL;
+  nr = (CO_CPL - 1 - dx + win_rg - 1) / CO_CPL;
 }
 
-// The TMA variant takes a job when both images start on a 16-byte boundary
-// and their row pitches are multiples of 16 bytes (a tensor map's rules).
-static bool tma_eligible(const CohJob &J) {
-  const uintptr_t m = reinterpret_cast<uintptr_t>(J.master);
-  const uintptr_t s = reinterpret_cast<uintptr_t>(J.slave);
-  return (m % 16 == 0) && (s % 16 == 0) && ((J.master_pitch * 4) % 16 == 0) &&
-         ((J.slave_pitch * 8) % 16 == 0) && J.pixels >= 1 && J.lines >= 1;
-}
-
-static int encode_maps(const CohJob &J, CUtensorMap *tm_m, CUtensorMap *tm_s) {
-  auto fn = tensor_map_encoder();
-  if (!fn) return TOPS_E_CUDA;
-  const cuuint64_t dims[2] = {(cuuint64_t)J.pixels, (cuuint64_t)J.lines};
-  const cuuint32_t box[2] = {(cuuint32_t)CT_LW, (cuuint32_t)CT_CH};
-  const cuuint32_t estr[2] = {1, 1};
-  const cuuint64_t sm[1] = {(cuuint64_t)J.master_pitch * 4};
-  const cuuint64_t ss[1] = {(cuuint64_t)J.slave_pitch * 8};
-  CUresult r = fn(tm_m, CU_TENSOR_MAP_DATA_TYPE_INT32, 2, const_cast<short2 *>(J.master), dims,
-                  sm, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return TOPS_E_INVALID;
-  r = fn(tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<float2 *>(J.slave), dims, ss, box,
-         estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-         CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? TOPS_OK : TOPS_E_INVALID;
-}
-
-template <int WAZ, int WRG>
-static int launch_coh_tma(const CohJob *jobs, int njobs, const TileCfg &cfg, int dev,
-                          cudaStream_t st) {
+template <int WAZ, int WRG, bool AL>
+static int launch_al(const CohJob *jobs, int njobs, int win_rg, int win_az, const TileCfg &cfg,
+                    int dev, cudaStream_t st) {
   static PerDeviceOnce setup;
   int resident = 0;
   const int s0 = once_per_device(
       setup, dev,
       [&](int &v) -> int {
-        for (auto fn : {coh_tma_kernel<WAZ, WRG, false>, coh_tma_kernel<WAZ, WRG, true>})
-          TOPS_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(CtShared)));
         int per_sm = 0, sms = 0;
         TOPS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, coh_tma_kernel<WAZ, WRG, false>, CT_NT, sizeof(CtShared)));
+            &per_sm, coherence_kernel<WAZ, WRG, AL>, CO_NT, 0));
         TOPS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
         v = per_sm * sms;
         return TOPS_OK;
       },
       &resident);
   if (s0 != TOPS_OK) return s0;
-  for (int j0 = 0, k = 0; j0 < njobs; j0 += CT_MAXJOBS, k++) {
-    CtBatch B;
+  int nl, nr;
+  window_lanes(win_rg, nl, nr);
+  const int tw = CO_NW * CO_CPL * (32 - nl - nr);   // output columns of a CTA
+  // default segment rows: the fewest row times of the last CTA to finish, waves
+  // x (rows + the window's halo and the first loads, worth about 8 rows)
+  int seg_rows = (cfg.seg_rows + 3) & ~3;   // whole groups: a row's sums do not depend on the cut
+  if (!seg_rows) {
+    static const int kSegs[] = {256, 192, 128, 96, 64, 48, 32, 24, 16, 8};
+    long best = 0;
+    for (int sr : kSegs) {
+      long items = 0;
+      for (int j = 0; j < njobs; j++)
+        items += (long)((jobs[j].pixels + tw - 1) / tw) * ((jobs[j].lines + sr - 1) / sr);
+      const long cost = (items + resident - 1) / resident * (sr + 8 + win_az);
+      if (!seg_rows || cost < best) {
+        best = cost;
+        seg_rows = sr;
+      }
+    }
+  }
+  for (int j0 = 0, k = 0; j0 < njobs; j0 += CO_MAXJOBS, k++) {
+    CoBatch B;
     B.njobs = 0;
+    B.win_rg = win_rg;
+    B.win_az = win_az;
     B.compensated = cfg.compensated;
+    B.nl = nl;
+    B.nr = nr;
     B.counter = cfg.counters ? cfg.counters + k : nullptr;
     int items = 0;
-    for (int j = j0; j < njobs && j < j0 + CT_MAXJOBS; j++) {
+    for (int j = j0; j < njobs && j < j0 + CO_MAXJOBS; j++) {
       CohJob &J = B.jobs[B.njobs];
       J = jobs[j];
-      J.seg_rows = cfg.seg_rows ? cfg.seg_rows : CT_SEG;
-      J.segs = (J.lines + J.seg_rows - 1) / J.seg_rows;
-      J.strips = (J.pixels + CtWin<WRG>::TW - 1) / CtWin<WRG>::TW;
+      J.seg_rows = seg_rows;
+      J.segs = (J.lines + seg_rows - 1) / seg_rows;
+      J.strips = (J.pixels + tw - 1) / tw;
       J.item_begin = items;
       items += J.strips * J.segs;
-      const int s = encode_maps(J, &B.tm_m[B.njobs], &B.tm_s[B.njobs]);
-      if (s != TOPS_OK) return s;
       B.njobs++;
     }
     B.total_items = items;
@@ -645,114 +620,60 @@ static int launch_coh_tma(const CohJob *jobs, int njobs, const TileCfg &cfg, int
       TOPS_CUDA_TRY(cudaMemsetAsync(B.counter, 0, sizeof(int), st));
       grid = min(items, cfg.grid > 0 ? cfg.grid : resident);
     }
-    if (B.compensated)
-      coh_tma_kernel<WAZ, WRG, true><<<grid, CT_NT, sizeof(CtShared), st>>>(B);
-    else
-      coh_tma_kernel<WAZ, WRG, false><<<grid, CT_NT, sizeof(CtShared), st>>>(B);
+    coherence_kernel<WAZ, WRG, AL><<<grid, CO_NT, 0, st>>>(B);
     TOPS_CUDA_TRY(cudaGetLastError());
   }
   return TOPS_OK;
 }
 
 template <int WAZ, int WRG>
-static int launch_coh_t(const CoBatch &B, int grid, cudaStream_t st) {
-  if (B.compensated)
-    coherence_kernel<WAZ, WRG, true><<<grid, CO_NT, 0, st>>>(B);
-  else
-    coherence_kernel<WAZ, WRG, false><<<grid, CO_NT, 0, st>>>(B);
-  TOPS_CUDA_TRY(cudaGetLastError());
-  return TOPS_OK;
+static int launch_t(const CohJob *jobs, int njobs, int win_rg, int win_az, const TileCfg &cfg,
+                    int dev, cudaStream_t st) {
+  bool al = true;
+  for (int j = 0; j < njobs; j++) al = al && jobs[j].al16;
+  return al ? launch_al<WAZ, WRG, true>(jobs, njobs, win_rg, win_az, cfg, dev, st)
+            : launch_al<WAZ, WRG, false>(jobs, njobs, win_rg, win_az, cfg, dev, st);
 }
 
-template <int WAZ, int WRG>
-static int coh_resident(int dev) {
-  static PerDeviceOnce setup;
-  int resident = 0;
-  const int s = once_per_device(
-      setup, dev,
-      [&](int &v) -> int {
-        int per_sm = 0, sms = 0;
-        TOPS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, coherence_kernel<WAZ, WRG, false>, CO_NT, 0));
-        TOPS_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        v = per_sm * sms;
-        return TOPS_OK;
-      },
-      &resident);
-  return s == TOPS_OK ? resident : 0;
-}
-
-// The compiled (azimuth, range) windows: the config's 3 x 10 and the
-// reference driver's 6 x 24 (Func.cpp:2583-2584); others run generic code.
-template <int WAZ>
-static int launch_coh_rg(const CoBatch &B, int grid, int resident_only, int dev,
-                         cudaStream_t st) {
-  if (B.win_rg == 10)
-    return resident_only ? coh_resident<WAZ, 10>(dev) : launch_coh_t<WAZ, 10>(B, grid, st);
-  if (B.win_rg == 24)
-    return resident_only ? coh_resident<WAZ, 24>(dev) : launch_coh_t<WAZ, 24>(B, grid, st);
-  return resident_only ? coh_resident<WAZ, 0>(dev) : launch_coh_t<WAZ, 0>(B, grid, st);
-}
-
-static int coh_dispatch(const CoBatch &B, int grid, int resident_only, int dev, cudaStream_t st) {
-  if (B.win_az == 3) return launch_coh_rg<3>(B, grid, resident_only, dev, st);
-  if (B.win_az == 6) return launch_coh_rg<6>(B, grid, resident_only, dev, st);
-  return launch_coh_rg<0>(B, grid, resident_only, dev, st);
-}
-
+// Compiled windows: 10 and the reference driver's 24 samples
+// (Func.cpp:2583-2584), with 3 and 6 rows, and every height up to 6 rows with
+// range windows of up to 6 samples (one compiled case each) and of 7 or more
+// (5 x 5 took 133 us with the lane sums picked at run time, 49 this way).
+// Taller windows sum the rows that 4 output rows share once.
 int launch_coherence(const CohJob *jobs, int njobs, int win_rg, int win_az, const TileCfg &cfg,
                      cudaStream_t st) {
   if (win_rg < 1 || win_az < 1 || win_rg > CO_MAX_WIN_RG) return TOPS_E_INVALID;
-  if (cfg.seg_rows < 0 || cfg.seg_rows > 512 || (cfg.seg_rows && cfg.seg_rows < CO_GR))
+  if (cfg.seg_rows < 0 || cfg.seg_rows > 512 || (cfg.seg_rows && cfg.seg_rows < 8))
     return TOPS_E_INVALID;
   int dev = 0;
   TOPS_CUDA_TRY(cudaGetDevice(&dev));
   if (dev < 0 || dev >= kMaxDevices) return TOPS_E_INVALID;
-  // the TMA-staged kernel for the pipeline's 10 x 3 and the reference
-  // driver's 24 x 6 windows (and 10 x 6, 24 x 3)
-  if ((win_rg == 10 || win_rg == 24) && (win_az == 3 || win_az == 6) && tensor_map_encoder()) {
-    bool all = true;
-    for (int j = 0; j < njobs; j++) all = all && tma_eligible(jobs[j]);
-    if (all) {
-      if (win_rg == 10)
-        return win_az == 3 ? launch_coh_tma<3, 10>(jobs, njobs, cfg, dev, st)
-                           : launch_coh_tma<6, 10>(jobs, njobs, cfg, dev, st);
-      return win_az == 3 ? launch_coh_tma<3, 24>(jobs, njobs, cfg, dev, st)
-                         : launch_coh_tma<6, 24>(jobs, njobs, cfg, dev, st);
+#define CO_LAUNCH(az, rg) return launch_t<az, rg>(jobs, njobs, win_rg, win_az, cfg, dev, st)
+  if (win_rg == 10 && win_az == 3) CO_LAUNCH(3, 10);
+  if (win_rg == 10 && win_az == 6) CO_LAUNCH(6, 10);
+  if (win_rg == 24 && win_az == 3) CO_LAUNCH(3, 24);
+  if (win_rg == 24 && win_az == 6) CO_LAUNCH(6, 24);
+  if (win_rg <= 6) {
+    switch (win_az) {
+      case 1: CO_LAUNCH(1, CO_SMALL);
+      case 2: CO_LAUNCH(2, CO_SMALL);
+      case 3: CO_LAUNCH(3, CO_SMALL);
+      case 4: CO_LAUNCH(4, CO_SMALL);
+      case 5: CO_LAUNCH(5, CO_SMALL);
+      case 6: CO_LAUNCH(6, CO_SMALL);
+      default: CO_LAUNCH(0, CO_SMALL);
     }
   }
-  for (int j0 = 0, k = 0; j0 < njobs; j0 += CO_MAXJOBS, k++) {
-    CoBatch B;
-    B.njobs = 0;
-    B.compensated = cfg.compensated;
-    B.win_rg = win_rg;
-    B.win_az = win_az;
-    B.counter = cfg.counters ? cfg.counters + k : nullptr;
-    int items = 0;
-    for (int j = j0; j < njobs && j < j0 + CO_MAXJOBS; j++) {
-      CohJob &J = B.jobs[B.njobs];
-      J = jobs[j];
-      if (cfg.seg_rows) {
-        J.seg_rows = cfg.seg_rows;
-        J.segs = (J.lines + cfg.seg_rows - 1) / cfg.seg_rows;
-      }
-      J.item_begin = items;
-      items += J.strips * J.segs;
-      B.njobs++;
-    }
-    B.total_items = items;
-    if (!items) continue;
-    int grid = items;
-    if (B.counter) {
-      TOPS_CUDA_TRY(cudaMemsetAsync(B.counter, 0, sizeof(int), st));
-      const int res = coh_dispatch(B, 0, 1, dev, st);
-      if (res <= 0) return TOPS_E_CUDA;
-      grid = min(items, cfg.grid > 0 ? cfg.grid : res);
-    }
-    const int s = coh_dispatch(B, grid, 0, dev, st);
-    if (s != TOPS_OK) return s;
+  switch (win_az) {
+    case 1: CO_LAUNCH(1, CO_LARGE);
+    case 2: CO_LAUNCH(2, CO_LARGE);
+    case 3: CO_LAUNCH(3, CO_LARGE);
+    case 4: CO_LAUNCH(4, CO_LARGE);
+    case 5: CO_LAUNCH(5, CO_LARGE);
+    case 6: CO_LAUNCH(6, CO_LARGE);
+    default: CO_LAUNCH(0, CO_LARGE);
   }
-  return TOPS_OK;
+#undef CO_LAUNCH
 }
 
 int fill_coh_job(const tops_coh_job &u, CohJob &J) {
@@ -770,9 +691,11 @@ int fill_coh_job(const tops_coh_job &u, CohJob &J) {
     return TOPS_E_INVALID;
   J.lines = u.lines;
   J.pixels = u.pixels;
-  J.strips = (u.pixels + CO_TW - 1) / CO_TW;
-  J.seg_rows = CO_SEG;
-  J.segs = (u.lines + CO_SEG - 1) / CO_SEG;
+  // vector access: four columns of a row start on a 16-byte boundary
+  const uintptr_t m = reinterpret_cast<uintptr_t>(u.master);
+  const uintptr_t s = reinterpret_cast<uintptr_t>(u.slave);
+  J.al16 = ((m | s | u.master_pitch | u.slave_pitch) & 15) == 0;
+  J.out_al16 = ((reinterpret_cast<uintptr_t>(u.coh) | u.coh_pitch) & 15) == 0;
   return TOPS_OK;
 }
 

@@ -131,6 +131,7 @@ struct CohJob {
   float *coh;
   long coh_pitch;
   int lines, pixels;
+  int al16, out_al16;     // input rows / output rows start on 16-byte boundaries
   int strips, segs, seg_rows;
   int item_begin;
 };

@@ -3,8 +3,9 @@
 // (rows per item) and the scheduling mode.
 //
 //   seg_rows  output rows per work item; the resample kernel takes 12..252
-//             (0: the longest of 252, 168, 120, 84 that gives two waves of
-//             items), the coherence kernel 8..512 (0: its default)
+//             (0: of a few lengths, the one whose last CTA ends first by the
+//             count of items per CTA), the coherence kernel 8..512, rounded up
+//             to a multiple of 4 (0: chosen the same way)
 //   counters  if non-null: persistent launch.  `grid` CTAs (0: as many as
 //             fit on the device at once) pull work items from a queue -- the
 //             device int counters[k], set to 0 on the stream before the k-th
@@ -21,7 +22,7 @@ struct TileCfg {
   int seg_rows = 0;
   int *counters = nullptr;
   int grid = 0;
-  int compensated = 0;   // coherence: window sums without the sliding update
+  int compensated = 0;   // coherence: reciprocal square roots with a Newton step
 };
 
 int resample_launch(const tops_lut_dev *lut, const tops_resample_job *jobs, int njobs,
