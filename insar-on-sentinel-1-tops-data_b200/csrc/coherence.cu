@@ -21,8 +21,8 @@
 // window (7.8e-8 relative RMS at 10 x 3, 8.0e-8 at 24 x 6).
 //
 // What bounds it: instruction issue (10 x 3: 64 per output pixel, 11 of them
-// packed adds and 9 shuffles; about 65% of the issue slots) at 16 warps per SM
-// by registers, then the 16 bytes per pixel of memory traffic.  Measured, in
+// packed adds and 9 shuffles; 64% of the issue slots, 79% of the L1 data pipe) at
+// 16 warps per SM by registers, then the 16 bytes per pixel of memory traffic.  Measured, in
 // us, against a kernel that staged the products of a block in shared memory
 // and summed windows by sliding updates behind block barriers:
 //   1500 x 21000, 10 x 3   154 -> 102 (4.9 TB/s)     24 x 6   243 -> 158
