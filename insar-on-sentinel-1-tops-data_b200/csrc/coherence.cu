@@ -21,14 +21,15 @@
 // window (7.8e-8 relative RMS at 10 x 3, 8.0e-8 at 24 x 6).
 //
 // What bounds it: instruction issue (10 x 3: 64 per output pixel, 11 of them
-// packed adds and 9 shuffles; 64% of the issue slots, 79% of the L1 data pipe) at
-// 16 warps per SM by registers, then the 16 bytes per pixel of memory traffic.  Measured, in
-// us, against a kernel that staged the products of a block in shared memory
-// and summed windows by sliding updates behind block barriers:
-//   1500 x 21000, 10 x 3   154 -> 102 (4.9 TB/s)     24 x 6   243 -> 158
-//   1523 x 8193, 5 x 5     147 -> 49                 1200 x 7000, 30 x 9  180 -> 134
-//   1200 x 7000, 17 x 2    129 -> 49                 300 x 512, 10 x 3    66 -> 9
-//   800 x 9000, 2 x 1      111 -> 24                 33 x 7               152 -> 77
+// packed adds and 9 shuffles; two thirds of the issue slots) and the L1 data pipe
+// (the shuffles) at 16 warps per SM by registers, then the 16 bytes per pixel of
+// memory traffic.  Measured, in us, against a kernel that staged the products of
+// a block in shared memory and summed windows by sliding updates behind block
+// barriers:
+//   1500 x 21000, 10 x 3   154 -> 97 (5.2 TB/s)      24 x 6   243 -> 156
+//   1523 x 8193, 5 x 5     147 -> 48                 1200 x 7000, 30 x 9  180 -> 133
+//   1200 x 7000, 17 x 2    129 -> 47                 300 x 512, 10 x 3    66 -> 9
+//   800 x 9000, 2 x 1      111 -> 24                 33 x 7               152 -> 78
 // Rows prefetched into registers instead of the ring took 121 us (10 x 3) and
 // 229 us (24 x 6); a ring of 7 slots 109 us; 18 warps per SM, by spilling, 149.
 #include <cuda_runtime.h>
@@ -46,6 +47,7 @@ constexpr int CO_NW = 2;           // warps (adjacent strips) per CTA
 constexpr int CO_NT = 32 * CO_NW;
 constexpr int CO_D = 4;            // slots per warp: the row read last and 3 in flight
 constexpr int CO_ROW = 2048;       // bytes of a slot: 128 columns of 4 and of 8, and a gap
+constexpr int CO_ODD = 512 + 36 * 16;   // the slave's odd pieces in a slot
 constexpr int CO_MAXJOBS = 32;
 constexpr int CO_MAX_WIN_RG = 33;
 
@@ -324,6 +326,12 @@ __device__ __forceinline__ void coherence_item(const CoBatch &B, int item,
   const short2 *const m0 = J.master + (AL ? clip(c0) & ~3 : 0);
   const float2 *const s1 = J.slave + (AL ? clip(c1) & ~1 : 0);
   const int s2 = AL ? (clip(c1 + 64) & ~1) - (clip(c1) & ~1) : 0;
+  // Slave pieces of two columns: the even ones from 512 on, the odd ones from
+  // CO_ODD on, 4 bank groups further, so that neither the copies nor the reads
+  // of a lane's pieces 2 lane and 2 lane + 1 conflict (10 x 3 burst: 103 us with
+  // the pieces in order, 97 so).
+  const unsigned sd = AL ? 16 * (lane >> 1) + (lane & 1 ? CO_ODD : 512)
+                         : 16 * (lane >> 2) + (lane & 2 ? CO_ODD : 512) + 8 * (lane & 1);
   unsigned char *const mine = stage + warp * (CO_D * CO_ROW);
   const unsigned base = (unsigned)__cvta_generic_to_shared(mine);
   // copies left of the item before end here: no slot is written twice at a time
@@ -346,15 +354,15 @@ __device__ __forceinline__ void coherence_item(const CoBatch &B, int item,
     const unsigned d = base + wr;
     if (AL) {
       co_copy<16>(d + 16 * lane, mp, row ? nb0 : 0);
-      co_copy<16>(d + 512 + 16 * lane, sp, row ? nb1 : 0);
-      co_copy<16>(d + 1024 + 16 * lane, sp + s2, row ? nb2 : 0);
+      co_copy<16>(d + sd, sp, row ? nb1 : 0);
+      co_copy<16>(d + sd + 256, sp + s2, row ? nb2 : 0);
     } else {
 #pragma unroll
       for (int k = 0; k < CO_CPL; k++) {
         const int c = c0 + 32 * k, o = clip(c);
         const bool ok = row && c == o;
         co_copy<4>(d + 4 * (lane + 32 * k), mp + o, ok ? 4 : 0);
-        co_copy<8>(d + 512 + 8 * (lane + 32 * k), sp + o, ok ? 8 : 0);
+        co_copy<8>(d + sd + 128 * k, sp + o, ok ? 8 : 0);
       }
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
@@ -372,8 +380,8 @@ __device__ __forceinline__ void coherence_item(const CoBatch &B, int item,
     __syncwarp();
     const unsigned char *q = mine + after(wr);
     const int4 a = *reinterpret_cast<const int4 *>(q + 16 * lane);
-    const float4 b = *reinterpret_cast<const float4 *>(q + 512 + 32 * lane);
-    const float4 c = *reinterpret_cast<const float4 *>(q + 528 + 32 * lane);
+    const float4 b = *reinterpret_cast<const float4 *>(q + 512 + 16 * lane);
+    const float4 c = *reinterpret_cast<const float4 *>(q + CO_ODD + 16 * lane);
     const int m[CO_CPL] = {a.x, a.y, a.z, a.w};
     const float2 sv[CO_CPL] = {make_float2(b.x, b.y), make_float2(b.z, b.w),
                                make_float2(c.x, c.y), make_float2(c.z, c.w)};
