@@ -23,7 +23,9 @@
 // Nearly parallel orbits give one entry per row, crossing orbits a few.
 // Column keys: thread per column pair, the runs of the range key over the
 // chunk's rows, each with its residual phase terms.  A chunk is as many rows
-// (up to 96) as the entry and run tables hold.
+// (up to 96) as the entry and run tables hold; where a run table is full before
+// 12 rows (kKeyedRows), the columns' rows behind it are keyed: [C] finds each
+// pixel's key and terms anew.
 //
 // Half of 6 rows.
 //   [A] azimuth pass, thread = 2 adjacent ring columns: six new slave lines
@@ -64,9 +66,10 @@
 //
 // Which path a pixel takes, and the order of its sums, depend on its row, its
 // column and its strip only, never on the work item, so a job that produces a
-// subset of the rows gives those rows bit for bit.  Rows with more than
-// RS_MAXKEY azimuth runs in the strip and pixels whose range support leaves
-// the ring take the per-pixel path from HBM.
+// subset of the rows gives those rows bit for bit.  The per-pixel path from HBM
+// takes rows with more than RS_MAXKEY azimuth runs in the strip or whose entries
+// need more than RS_ROWU tile units (a full strip: 56 and about 8 for each run,
+// so 9 runs fit), and pixels whose range support leaves the ring.
 //
 // Precision modes: TOPS_PREC_SPLIT (default) forms each sample's deramp
 // phase in FP32 as rho(y) + G(y, x), rho the FP64 reference phase reduced
@@ -108,6 +111,15 @@ static_assert(RS_DT <= RS_NT && RS_CH <= 2 * RS_NT && RS_CH % (2 * RS_H) == 0 &&
                   RS_CH * RS_MAXKEY * 8 <= RS_TU * 16,
               "thread mappings and table fields assume these sizes");
 
+// A chunk whose run tables end before this many rows is not cut there: columns
+// with a full table are keyed behind it.  A shorter chunk prepares and refills
+// for each tile what it needs only once per 96 rows; at the line both cost the
+// same (300 x 6000, 0.34 keys per row: split chunks of 12 rows 83 us, keyed 85;
+// FP64, 4 runs per table, chunks of 9 rows 111 us, keyed 87), and beyond it the
+// chunks lose (310 x 25000, 1.3 keys per row: split 556 and 306, FP64 712 and
+// 308 us; the kernel before the run tables of a chunk took 337 and 341).
+constexpr int kKeyedRows = 2 * RS_H;
+
 enum : int { REG_OUT = 0, REG_EDGE = 1, REG_IN = 2 };
 // A half: has interior entries; fills its window anew; has entries off its
 // window; shares its tile with the next half; has per-pixel rows; every row is
@@ -143,16 +155,17 @@ union RsSlaveRow {
   } f;
 };
 
-// Deramp coefficients of the ring columns: G's (split mode) or the FP64
-// quadratics (FP64 mode, G's formed from them where needed).
+// Deramp coefficients of the ring columns: G's by unit and, in FP64 mode, the
+// FP64 quadratics.
 template <bool kSplit>
 struct RsRing {
+  float2 g2[RS_UN], g1[RS_UN], g0[RS_UN];
   double2 a21[RS_FW];
   double a0[RS_FW];
 };
 template <>
 struct RsRing<true> {
-  float2 g2[RS_UN], g1[RS_UN], g0[RS_UN];   // by unit
+  float2 g2[RS_UN], g1[RS_UN], g0[RS_UN];
 };
 
 template <bool kSplit>
@@ -176,6 +189,7 @@ struct __align__(16) RsStrip {
   double ref_a0, ref_a1, ref_a2, tm;  // reference column's phase, burst centre time
   int xo, dlo, dhi;                   // ring origin, bounds of (ring column - strip column)
   int nfit, cov, gen_any, prev_line;
+  int kfrom;                          // first keyed row of the chunk
   int n_border;                       // border columns of the chunk
   unsigned char border[RS_TW];
 };
@@ -671,6 +685,10 @@ struct PairRuns {
   int in;                // range-interior columns: 1 the first, 2 the second
 };
 
+// The key of a column's last run where its table is full: the rows from there on
+// are keyed, each pixel by its own key (the bin is no LUT bin).
+constexpr int kKeyed = -(1 << 19) * 4096 + 4095;
+
 // Ring column of a key's first tap when its 14 samples are inside the ring,
 // else -1.
 __device__ __forceinline__ int ring_col(int xo, int key) {
@@ -688,6 +706,36 @@ __device__ __forceinline__ float4 run_load(const RsStrip<kSplit> &Q, const RsLut
                                            int c, int key) {
   return make_float4(__ldg(lut.sp1 + (key & 4095)), Q.run_g[m][0][c], Q.run_g[m][1][c],
                      Q.run_g[m][2][c]);
+}
+
+// Residual-phase terms (G2, G1, G0), Gk = sum_i kRg[i] gk(x_i), of the taps that
+// start at element OFF of w and ring column xb.
+template <int OFF, bool kSplit, int N>
+__device__ __forceinline__ float3 taps_terms(const RsStrip<kSplit> &Q, const float4 (&w)[N],
+                                             int xb) {
+  const float *g2 = reinterpret_cast<const float *>(Q.ring.g2) + xb;
+  const float *g1 = reinterpret_cast<const float *>(Q.ring.g1) + xb;
+  const float *g0 = reinterpret_cast<const float *>(Q.ring.g0) + xb;
+  float3 G = make_float3(0.f, 0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < kTaps; i++) {
+    const int j = i + OFF;
+    const float4 q = w[j >> 2];
+    const float t = (j & 3) == 0 ? q.x : (j & 3) == 1 ? q.y : (j & 3) == 2 ? q.z : q.w;
+    G.x = fmaf(t, g2[i], G.x);
+    G.y = fmaf(t, g1[i], G.y);
+    G.z = fmaf(t, g0[i], G.z);
+  }
+  return G;
+}
+// Those of a range key (0 when its taps leave the ring).
+template <bool kSplit>
+__device__ __forceinline__ float3 key_terms(const RsStrip<kSplit> &Q, const RsLut &lut, int key) {
+  const int xb = (key >> 12) - 5 - Q.xo;
+  if (xb < 0 || xb + kTaps > RS_FW) return make_float3(0.f, 0.f, 0.f);
+  float4 w[3];
+  taps_even(w, lut, key & 4095);
+  return taps_terms<0, kSplit>(Q, w, xb);
 }
 
 // Moves the runs on to chunk row `row`.
@@ -751,19 +799,18 @@ __device__ __forceinline__ float2 border_pixel(const ResampleJob &J, int reg, in
   return make_float2((float)sv.x, (float)sv.y);
 }
 
-// One pixel (chunk row k, strip column c) of a shared row outside the pair path.
+// One pixel (chunk row k, strip column c; its range key and the key's terms) of a
+// shared row outside the pair path.
 template <bool kSplit>
 __device__ __forceinline__ void pixel_shared(RsStrip<kSplit> &Q, const ResampleJob &J, int k,
-                                             int tbase, int kt, int c, float2 *out) {
+                                             int tbase, int kt, int c, int key, float4 g,
+                                             float2 *out) {
   const int re = Q.rowe[k], ne = re >> 16;
   int e = re & 0xffff;
   for (int q = 1; q < ne; q++, e++) {
     const int z = Q.eM[e].y;
     if (c >= ((z >> 16) & 0xff) && c < ((z >> 24) & 0xff)) break;
   }
-  int m = 0;
-  while (k >= Q.run_rk[m][c].x) m++;
-  const int key = Q.run_rk[m][c].y;
   const int4 M = Q.eM[e];
   const int p0 = key >> 12;
   const int reg = (M.y >> 12) & 3;
@@ -789,8 +836,77 @@ __device__ __forceinline__ void pixel_shared(RsStrip<kSplit> &Q, const ResampleJ
     taps_even(w, J.lut, key & 4095);
     v = rg_sum<6>(w, U);
   }
-  *out = cmul_conj_turns(v, run_phase(Q.eA[e], __int_as_float(M.z),
-                                      run_load(Q, J.lut, m, c, key)));
+  *out = cmul_conj_turns(v, run_phase(Q.eA[e], __int_as_float(M.z), g));
+}
+
+// A pair of columns (strip columns c, c + 1) in chunk row k with range keys kx, ky.
+template <bool kSplit>
+__device__ __forceinline__ void keyed_pair(RsStrip<kSplit> &Q, const ResampleJob &J, int k, int c,
+                                           int cN, int kx, int ky, int tbase, int kt, float2 *o) {
+  const bool two = c + 1 < cN;
+  const int re = Q.rowe[k], ne = re >> 16;
+  if (ne == 0) return;                   // a per-pixel row
+  int e = re & 0xffff;
+  int4 M = Q.eM[e];
+  for (int q = 1; q < ne && !(c >= ((M.y >> 16) & 0xff) && c < ((M.y >> 24) & 0xff)); q++)
+    M = Q.eM[++e];
+  const int xb = ring_col(Q.xo, kx), unit = xb >> 1;
+  PairRuns P;
+  P.in = (range_in(J, kx) ? 1 : 0) | (two && range_in(J, ky) ? 2 : 0);
+  if (P.in == 3 && ((M.y >> 12) & 3) == REG_IN && c + 1 < ((M.y >> 24) & 0xff) && xb >= 0 &&
+      ring_col(Q.xo, ky) == xb + 1 && unit >= ((M.w >> 16) & 0xff) &&
+      unit + 6 <= ((M.w >> 24) & 0xff)) {
+    P.vec = J.out_al16;
+    P.odd = (xb & 1) != 0;
+    taps_even(P.we, J.lut, (P.odd ? ky : kx) & 4095);
+    taps_odd(P.wo, J.lut, (P.odd ? kx : ky) & 4095);
+    const float3 ge = taps_terms<0, kSplit>(Q, P.we, P.odd ? xb + 1 : xb);
+    const float3 go = taps_terms<1, kSplit>(Q, P.wo, P.odd ? xb : xb + 1);
+    const float3 gx = P.odd ? go : ge, gy = P.odd ? ge : go;
+    P.gx = make_float4(__ldg(J.lut.sp1 + (kx & 4095)), gx.x, gx.y, gx.z);
+    P.gy = make_float4(__ldg(J.lut.sp1 + (ky & 4095)), gy.x, gy.y, gy.z);
+    pair_row(P, &Q.tile[tbase + (short)(M.w & 0xffff) + unit], Q.eA[e], __int_as_float(M.z), o);
+    return;
+  }
+#pragma unroll 1
+  for (int q = 0; q < (two ? 2 : 1); q++) {
+    const int key = q ? ky : kx;
+    const float3 g = key_terms<kSplit>(Q, J.lut, key);
+    pixel_shared(Q, J, k, tbase, kt, c + q, key,
+                 make_float4(__ldg(J.lut.sp1 + (key & 4095)), g.x, g.y, g.z), o + q);
+  }
+}
+
+// The range pass of chunk rows [ka, k1) of the tile that starts at row k0 with
+// each pixel's key found anew, all threads.  From row ks on the entries' tile
+// starts at tb1.
+template <bool kSplit>
+__device__ __noinline__ void keyed_pairs(const ResampleJob &J, int rb, int k0, int ka, int k1,
+                                         int ks, int tb1, int c0, int cN) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  RsShared<kSplit> &S = *reinterpret_cast<RsShared<kSplit> *>(smem_raw);
+  RsStrip<kSplit> &Q = S.strip;
+  const int np = (cN + 1) / 2;
+  int k = ka, c = 2 * (int)threadIdx.x;
+  auto in_row = [&]() {                  // (k, c) of the pairs end to end
+    for (; c >= 2 * np; c -= 2 * np) k++;
+  };
+  auto keys = [&]() {
+    const double L = row_L(J, rb + k);
+    const double A = row_a(S.crg, L), B = row_b(S.crg, L);
+    return make_int2(rg_key_at(A, B, S.crg[5], col_P(J, c0 + c)),
+                     rg_key_at(A, B, S.crg[5], col_P(J, c0 + c + 1)));
+  };
+  in_row();
+  int2 next = keys();
+  while (k < k1) {
+    const int kx = next.x, ky = next.y, kr = k, cc = c;
+    c += 2 * RS_NT;
+    in_row();
+    next = keys();                       // the next pair's, while this one's loads run
+    keyed_pair<kSplit>(Q, J, kr, cc, cN, kx, ky, kr >= ks ? tb1 : 0, kr - k0,
+                       J.out + (long)(rb + kr - J.row0) * J.out_pitch + c0 + cc);
+  }
 }
 
 // The border pixels of a chunk's columns listed in Q.border (those off the
@@ -812,7 +928,7 @@ __device__ __forceinline__ void border_columns(const RsStrip<kSplit> &Q, const R
     int m = 0;
     while (k >= Q.run_rk[m][c].x) m++;
     const int key = Q.run_rk[m][c].y;
-    if (range_in(J, key)) continue;
+    if (range_in(J, key) || key == kKeyed) continue;
     const int4 M = Q.eM[e];
     obase[(long)k * J.out_pitch + c] = border_pixel(J, (M.y >> 12) & 3, M.x, key >> 12);
   }
@@ -836,8 +952,14 @@ __device__ __forceinline__ void slow_pixels(RsStrip<kSplit> &Q, const ResampleJo
     while (i-- > 0) m &= m - 1;
     const int uu = wq * 32 + __ffs(m) - 1;   // the pair's thread
     const int c = 2 * uu + (w & 1);
-    if (c < cN && ((Q.miss[uu] >> q) & 1))
-      pixel_shared(Q, J, k0 + q, k0 + q >= ks ? tb1 : 0, q, c, obase + (long)q * J.out_pitch + c);
+    if (c < cN && ((Q.miss[uu] >> q) & 1)) {
+      int m = 0;
+      while (k0 + q >= Q.run_rk[m][c].x) m++;
+      const int key = Q.run_rk[m][c].y;
+      if (key == kKeyed) continue;
+      pixel_shared(Q, J, k0 + q, k0 + q >= ks ? tb1 : 0, q, c, key, run_load(Q, J.lut, m, c, key),
+                   obase + (long)q * J.out_pitch + c);
+    }
   }
 }
 
@@ -992,38 +1114,14 @@ __device__ __forceinline__ void write_entry(RsStrip<kSplit> &Q, const ResampleJo
   Q.eM[e] = make_int4(E.x, E.y, __float_as_int(R0), ulo << 16 | uhi << 24);
 }
 
-// Residual-phase terms of a range-key run, (G2, G1, G0) with Gk = sum_i kRg[i]
-// gk(x_i) over the ring columns of its taps (0 when they leave the window).
+// The terms of a column's run.
 template <bool kSplit>
 __device__ __forceinline__ void run_terms(RsStrip<kSplit> &Q, const RsLut &lut, int m, int c,
                                           int key) {
-  const int p0 = key >> 12, bp = key & 4095;
-  const int xb = p0 - 5 - Q.xo;
-  float G2 = 0.f, G1 = 0.f, G0 = 0.f;
-  if (xb >= 0 && xb + kTaps <= RS_FW) {
-    const float *kp = lut.krg + bp * kTaps;
-#pragma unroll
-    for (int i = 0; i < kTaps; i++) {
-      const float w = __ldg(kp + i);
-      const int x = xb + i;
-      float3 g;
-      if constexpr (kSplit) {
-        g = make_float3(reinterpret_cast<const float *>(Q.ring.g2)[x],
-                        reinterpret_cast<const float *>(Q.ring.g1)[x],
-                        reinterpret_cast<const float *>(Q.ring.g0)[x]);
-      } else {
-        const double2 a = Q.ring.a21[x];
-        g = residual_phase(DerampQuad{Q.ring.a0[x], a.y, a.x},
-                           DerampQuad{Q.ref_a0, Q.ref_a1, Q.ref_a2}, Q.tm);
-      }
-      G2 = fmaf(w, g.x, G2);
-      G1 = fmaf(w, g.y, G1);
-      G0 = fmaf(w, g.z, G0);
-    }
-  }
-  Q.run_g[m][0][c] = G2;
-  Q.run_g[m][1][c] = G1;
-  Q.run_g[m][2][c] = G0;
+  const float3 G = key_terms<kSplit>(Q, lut, key);
+  Q.run_g[m][0][c] = G.x;
+  Q.run_g[m][1][c] = G.y;
+  Q.run_g[m][2][c] = G.z;
 }
 // [P6] The runs of column c's range key over chunk rows [0, n) (box rows rb
 // ...).  Most columns hold one key: when the position is monotone over the
@@ -1032,13 +1130,13 @@ __device__ __forceinline__ void run_terms(RsStrip<kSplit> &Q, const RsLut &lut, 
 // rows from the first change that does not fit the table on are left to the
 // next chunk (Q.cov).
 template <bool kSplit>
-__device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kSplit> &Q,
+__device__ __forceinline__ bool build_runs(const RsShared<kSplit> &S, RsStrip<kSplit> &Q,
                                            const ResampleJob &J, int rb, int n, int c0, int c,
                                            bool mono, int ka, int kz) {
   run_terms(Q, J.lut, 0, c, ka);
   if (mono && ka == kz) {
     Q.run_rk[0][c] = make_int2(INT32_MAX, ka);
-    return;
+    return false;
   }
   const double P = col_P(J, c0 + c);
   auto keyat = [&](int ri) { return rg_key(S.crg, J, rb + ri, P); };
@@ -1063,7 +1161,7 @@ __device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kS
         m++;
         if (m == RsStrip<kSplit>::kRuns) {
           atomicMin(&Q.cov, r);
-          return;
+          return true;
         }
         run_terms(Q, J.lut, m, c, k);
         key = k;
@@ -1086,6 +1184,7 @@ __device__ __forceinline__ void build_runs(const RsShared<kSplit> &S, RsStrip<kS
     from = bend + 1;
   }
   Q.run_rk[m][c] = make_int2(INT32_MAX, key);
+  return false;
 }
 
 // [P7] Half h of a chunk of n rows: its window's lines, the entries of each
@@ -1171,6 +1270,7 @@ template <bool kSplit>
 __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch &B, int item) {
   const int u = threadIdx.x;
   RsStrip<kSplit> &Q = S.strip;
+  constexpr int kRuns = RsStrip<kSplit>::kRuns;
 
   // ---- locate the work item (job, strip, segment)
   int jb = 0;
@@ -1256,18 +1356,15 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       const int x = xa + q;
       DerampQuad cq = refq;
       if (x >= J.sx0 && x <= J.sx1) cq = deramp_quad(J.kt[x], J.tref[x], J.fdc[x]);
-      if constexpr (kSplit) {
-        g[q] = residual_phase(cq, refq, Q.tm);
-      } else {
+      g[q] = residual_phase(cq, refq, Q.tm);
+      if constexpr (!kSplit) {
         Q.ring.a21[2 * u + q] = make_double2(cq.a2, cq.a1);
         Q.ring.a0[2 * u + q] = cq.a0;
       }
     }
-    if constexpr (kSplit) {
-      Q.ring.g2[u] = make_float2(g[0].x, g[1].x);
-      Q.ring.g1[u] = make_float2(g[0].y, g[1].y);
-      Q.ring.g0[u] = make_float2(g[0].z, g[1].z);
-    }
+    Q.ring.g2[u] = make_float2(g[0].x, g[1].x);
+    Q.ring.g1[u] = make_float2(g[0].y, g[1].y);
+    Q.ring.g0[u] = make_float2(g[0].z, g[1].z);
   }
 
   // range-pass columns
@@ -1290,6 +1387,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
     if (u == 0) {
       Q.nfit = nrc;
       Q.cov = nrc;
+      Q.kfrom = INT32_MAX;
       Q.n_border = 0;
     }
     __syncthreads();                     // also: the ring's terms are written
@@ -1330,6 +1428,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       for (int i = 0; i < re >> 16; i++)
         write_entry(Q, J, found[r * RS_MAXKEY + i], cN, e + i);
     }
+    int full = 0;                        // columns whose run table is full: 1 the first, 2 the second
     if (dval) {
       const double La = row_L(J, rb), Lz = row_L(J, rb + nfit - 1), c5 = S.crg[5];
       const double Aa = row_a(S.crg, La), Ba = row_b(S.crg, La);
@@ -1347,21 +1446,30 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       }
 #pragma unroll 1
       for (int i = 0; i < (dtwo ? 2 : 1); i++)
-        build_runs(S, Q, J, rb, nfit, c0, dc + i, i ? mono[1] : mono[0], i ? ka[1] : ka[0],
-                   i ? kz[1] : kz[0]);
+        full |= (int)build_runs(S, Q, J, rb, nfit, c0, dc + i, i ? mono[1] : mono[0],
+                                i ? ka[1] : ka[0], i ? kz[1] : kz[0])
+                << i;
     }
     __syncthreads();
     // ---- [P7] the halves; a chunk that does not end the item ends with a
     // pair of halves, so that the window carries over
-    int n = min(nfit, Q.cov);
+    int n = Q.cov >= kKeyedRows ? min(nfit, Q.cov) : nfit;
     if (n < nr - ch0 && n >= 2 * RS_H) n -= n % (2 * RS_H);
     const int nh = (n + RS_H - 1) / RS_H;
     if (dval) {
+      if (Q.cov < n) {
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+          if ((full >> i) & 1) {
+            Q.run_rk[kRuns - 1][dc + i] = make_int2(INT32_MAX, kKeyed);
+            atomicMin(&Q.kfrom, Q.run_rk[kRuns - 2][dc + i].x);
+          }
+      }
       for (int c = dc; c < min(dc + 2, cN); c++) {
         bool out = false;
         for (int m = 0;; m++) {
           const int2 rk = Q.run_rk[m][c];
-          out = out || !range_in(J, rk.y);
+          out = out || !(range_in(J, rk.y) || rk.y == kKeyed);
           if (rk.x >= n) break;
         }
         if (out) Q.border[atomicAdd(&Q.n_border, 1)] = (unsigned char)c;
@@ -1483,11 +1591,15 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       }
       __syncthreads();
 
-      // ---- [C] the pixels the pair path left, then per-pixel rows and the
-      // pixels left to the per-pixel path
+      // ---- [C] the pixels the pair path left and the keyed rows, then
+      // per-pixel rows and the pixels left to the per-pixel path
       if (Q.missb[0] | Q.missb[1]) {
         slow_pixels(Q, J, u, k0, k1 - k0, h * RS_H, H.tbase, cN,
                     J.out + (long)(rb + k0 - J.row0) * J.out_pitch + c0);
+        __syncthreads();
+      }
+      if (k1 > Q.kfrom) {
+        keyed_pairs<kSplit>(J, rb, k0, max(k0, Q.kfrom), k1, h * RS_H, H.tbase, c0, cN);
         __syncthreads();
       }
       if (Q.gen_any || (any & HG_PIX)) pixel_pass(S, Q, J, u, k0, rb + k0, k1 - k0, c0, cN);
