@@ -399,17 +399,20 @@ __device__ __forceinline__ float2 pixel_generic(const RsShared<kSplit> &S, const
 }
 
 // The per-pixel rows and the listed pixels of nrows tile rows (chunk rows from
-// cr0, box rows from r0 on), all threads.
+// cr0, box rows from r0 on), all threads; the rows end to end, so that no lane
+// idles at the end of each (1000 x 6000, all rows of more than 12 azimuth runs:
+// 4670 -> 4270 us).
 template <bool kSplit>
 __device__ __forceinline__ void pixel_pass(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
                                            const ResampleJob &J, int u, int cr0, int r0, int nrows,
                                            int c0, int cN) {
-  for (int k = 0; k < nrows; k++) {
-    const bool whole = (Q.rowe[cr0 + k] >> 16) == 0;
+  int k = 0;
+  for (int c = u;; c += RS_NT) {
+    for (; c >= cN; c -= cN) k++;
+    if (k >= nrows) break;
     const int r = r0 + k;
-    for (int c = u; c < cN; c += RS_NT)
-      if (whole || ((Q.gen[k][c >> 5] >> (c & 31)) & 1u))
-        J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] = pixel_generic(S, J, r, c0 + c);
+    if ((Q.rowe[cr0 + k] >> 16) == 0 || ((Q.gen[k][c >> 5] >> (c & 31)) & 1u))
+      J.out[(long)(r - J.row0) * J.out_pitch + c0 + c] = pixel_generic(S, J, r, c0 + c);
   }
 }
 

@@ -133,3 +133,16 @@ def test_cost_of_dense_range_keys(T):
         j.close()
     print(f"one key {one:.0f} us, a key per row {dense:.0f} us")
     assert dense < 3.0 * one, (one, dense)
+
+
+def test_cost_of_per_pixel_rows(T):
+    """Rows of more azimuth runs than a strip takes are computed pixel by pixel, a
+    thread per pixel and the rows end to end: 68 interior columns on 64 threads
+    cost little more than 60 (twice as much when every row starts anew).  Columns
+    0 to 3 and the last 8 are off the interior and cost next to nothing."""
+    jobs = [_Job(T, _inputs(T, 1200, w, az_tilt=0.5), "split") for w in (72, 80)]
+    a, b = _time(jobs)
+    for j in jobs:
+        j.close()
+    print(f"60 interior columns {a:.0f} us, 68 {b:.0f} us")
+    assert b < 1.5 * a, (a, b)
