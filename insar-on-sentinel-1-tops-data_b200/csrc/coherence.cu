@@ -334,9 +334,13 @@ __device__ __forceinline__ void coherence_item(const CoBatch &B, int item,
                          : 16 * (lane >> 2) + (lane & 2 ? CO_ODD : 512) + 8 * (lane & 1);
   unsigned char *const mine = stage + warp * (CO_D * CO_ROW);
   const unsigned base = (unsigned)__cvta_generic_to_shared(mine);
-  // copies left of the item before end here: no slot is written twice at a time
-  asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-  __syncwarp();
+  // The copies issued ahead of the last row, which nothing reads, end before the
+  // item does: the next item's are then the only ones on a slot, and none is in
+  // flight when a warp leaves the kernel.
+  auto drain = [&]() {
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();
+  };
   unsigned wr = 0;                         // the slot to write next (byte offset)
   auto after = [](unsigned slot) { return (slot + CO_ROW) & (CO_D * CO_ROW - 1); };
   int y = 0;                               // the next row to copy, and where it is
@@ -475,6 +479,7 @@ __device__ __forceinline__ void coherence_item(const CoBatch &B, int item,
         if (r + k < r_end) store(o, c[k]);
       }
     }
+    drain();
     return;
   }
 
@@ -526,6 +531,7 @@ __device__ __forceinline__ void coherence_item(const CoBatch &B, int item,
       }
     }
   }
+  drain();
 }
 
 // Warps per SM: 16 where up to two rows of products are kept, 12 for three and
