@@ -179,12 +179,13 @@ int tops_run_config(const char *config_path, tops_run_stats *stats);
  * tops_pair_download as usual. */
 typedef struct tops_batch tops_batch;
 
-/* Tile and scheduling of the resample and coherence launches. */
+/* Tile and scheduling of the resample and coherence launches.  The rows of a
+ * work item are chosen by the number of items, up to the limits here. */
 typedef struct {
-  int rs_seg_rows;      /* resample output rows per work item, 12..252 (0: chosen
-                           by the number of items) */
+  int rs_seg_rows;      /* most resample output rows per work item, 12..252
+                           (0: 252) */
   int rs_persistent;    /* 1: persistent kernel pulling items from a queue */
-  int coh_seg_rows;     /* coherence rows per work item, 8..512 (0: chosen) */
+  int coh_seg_rows;     /* most coherence rows per work item, 8..512 (0: 256) */
   int coh_persistent;
 } tops_tune;
 
@@ -197,8 +198,9 @@ int tops_batch_launches(const tops_batch *b);
 int tops_batch_set_tune(tops_batch *b, const tops_tune *t);
 int tops_batch_get_tune(const tops_batch *b, tops_tune *t);
 /* Times every candidate tile of the resample and coherence stages on this
- * batch (CUDA events on `stream`, synchronous) and keeps the fastest; best_ms
- * (optional, 2 doubles) receives the two stage times. */
+ * batch (CUDA events on `stream`, synchronous) and keeps the fastest (the
+ * default limits are among them); best_ms (optional, 2 doubles) receives the
+ * two stage times. */
 int tops_batch_autotune(tops_batch *b, void *stream, tops_tune *best, double *best_ms);
 
 #ifdef __cplusplus

@@ -590,13 +590,16 @@ static int launch_al(const CohJob *jobs, int njobs, int win_rg, int win_az, cons
   int nl, nr;
   window_lanes(win_rg, nl, nr);
   const int tw = CO_NW * CO_CPL * (32 - nl - nr);   // output columns of a CTA
-  // default segment rows: the fewest row times of the last CTA to finish, waves
-  // x (rows + the window's halo and the first loads, worth about 8 rows)
-  int seg_rows = (cfg.seg_rows + 3) & ~3;   // whole groups: a row's sums do not depend on the cut
-  if (!seg_rows) {
-    static const int kSegs[] = {256, 192, 128, 96, 64, 48, 32, 24, 16, 8};
+  // segment rows: the fewest row times of the last CTA to finish, waves x (rows
+  // + the window's halo and the first loads, worth about 8 rows), up to the
+  // caller's limit; whole groups, so that a row's sums do not depend on the cut
+  const int most = cfg.seg_rows ? (cfg.seg_rows + 3) & ~3 : 256;
+  int seg_rows = 0;
+  {
+    const int kSegs[] = {most, 256, 192, 128, 96, 64, 48, 32, 24, 16, 8};
     long best = 0;
     for (int sr : kSegs) {
+      if (sr > most) continue;
       long items = 0;
       for (int j = 0; j < njobs; j++)
         items += (long)((jobs[j].pixels + tw - 1) / tw) * ((jobs[j].lines + sr - 1) / sr);

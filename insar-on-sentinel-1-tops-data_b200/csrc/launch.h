@@ -2,10 +2,11 @@
 // kernels, used by the batched plans (host/pipeline.cpp): the work-item tile
 // (rows per item) and the scheduling mode.
 //
-//   seg_rows  output rows per work item; the resample kernel takes 12..252
-//             (0: of a few lengths, the one whose last CTA ends first by the
-//             count of items per CTA), the coherence kernel 8..512, rounded up
-//             to a multiple of 4 (0: chosen the same way)
+//   seg_rows  most output rows per work item; the resample kernel takes
+//             12..252 (0: 252), the coherence kernel 8..512, rounded up to a
+//             multiple of 4 (0: 256).  Of a few lengths up to that, a launch
+//             takes the one whose last CTA ends first by the count of items
+//             per CTA: a long item alone on an SM leaves the others idle
 //   counters  if non-null: persistent launch.  `grid` CTAs (0: as many as
 //             fit on the device at once) pull work items from a queue -- the
 //             device int counters[k], set to 0 on the stream before the k-th

@@ -1788,14 +1788,16 @@ static int launch_resample_t(const ResampleJob *jobs, int njobs, const TileCfg &
   if (s0 != TOPS_OK) return s0;
   if (cfg.seg_rows < 0 || cfg.seg_rows > RS_MAXSEG || (cfg.seg_rows && cfg.seg_rows < 2 * RS_H))
     return TOPS_E_INVALID;
-  // default segment rows: the fewest row times of the last CTA to finish,
-  // waves x (rows + the prologue and the window's fill, worth about 24 rows).
-  // Outputs do not depend on it.
-  int seg_rows = cfg.seg_rows;
-  if (!seg_rows) {
-    static const int kSegs[] = {252, 204, 168, 144, 120, 96, 84, 72, 60, 48, 36, 24, 12};
+  // segment rows: the fewest row times of the last CTA to finish, waves x (rows
+  // + the prologue and the window's fill, worth about 24 rows), up to the
+  // caller's limit.  Outputs do not depend on it.
+  const int most = cfg.seg_rows ? cfg.seg_rows : RS_MAXSEG;
+  int seg_rows = 0;
+  {
+    const int kSegs[] = {most, 252, 204, 168, 144, 120, 96, 84, 72, 60, 48, 36, 24, 12};
     long best = 0;
     for (int sr : kSegs) {
+      if (sr > most) continue;
       long items = 0;
       for (int j = 0; j < njobs; j++)
         items += (long)jobs[j].strips * ((jobs[j].nrows + sr - 1) / sr);

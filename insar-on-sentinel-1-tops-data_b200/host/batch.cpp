@@ -269,9 +269,10 @@ int tops_batch_run_graph(tops_batch *B, void *stream) {
 int tops_batch_launches(const tops_batch *B) { return B ? B->n_launches : -1; }
 
 // Autotuner: times the resample (ESD pass) and coherence stages of this
-// batch for every candidate tile -- rows per work item and grid-sized versus
-// persistent work-queue scheduling -- with CUDA events on `stream`, and keeps
-// the fastest of each.  Runs the whole batch once first so the stage inputs
+// batch for every candidate tile -- the most rows per work item and grid-sized
+// versus persistent work-queue scheduling -- with CUDA events on `stream`, and
+// keeps the fastest of each.  252 and 256 rows are the untuned launches' limits,
+// so a tuned batch is no slower than an untuned one.  Runs the whole batch once first so the stage inputs
 // (offsets, ESD shifts) are valid.
 int tops_batch_autotune(tops_batch *B, void *stream, tops_tune *best, double *best_ms) {
   if (!B) return TOPS_E_INVALID;
