@@ -695,8 +695,8 @@ constexpr int kKeyed = -(1 << 19) * 4096 + 4095;
 // Ring column of a key's first tap when its 14 samples are inside the ring,
 // else -1.
 __device__ __forceinline__ int ring_col(int xo, int key) {
-  const int xb = (key >> 12) - 5 - xo;
-  return xb >= 0 && xb + 13 < RS_FW ? xb : -1;
+  const unsigned xb = (unsigned)(key >> 12) - 5u - (unsigned)xo;
+  return xb < RS_FW - 13 ? (int)xb : -1;
 }
 __device__ __forceinline__ bool range_in(const ResampleJob &J, int key) {
   const int p0 = key >> 12;
@@ -734,8 +734,8 @@ __device__ __forceinline__ float3 taps_terms(const RsStrip<kSplit> &Q, const flo
 // Those of a range key (0 when its taps leave the ring).
 template <bool kSplit>
 __device__ __forceinline__ float3 key_terms(const RsStrip<kSplit> &Q, const RsLut &lut, int key) {
-  const int xb = (key >> 12) - 5 - Q.xo;
-  if (xb < 0 || xb + kTaps > RS_FW) return make_float3(0.f, 0.f, 0.f);
+  const unsigned xb = (unsigned)(key >> 12) - 5u - (unsigned)Q.xo;
+  if (xb > RS_FW - kTaps) return make_float3(0.f, 0.f, 0.f);
   float4 w[3];
   taps_even(w, lut, key & 4095);
   return taps_terms<0, kSplit>(Q, w, xb);
@@ -1050,12 +1050,14 @@ __device__ __forceinline__ void walk_row(const RsShared<kSplit> &S, const Resamp
 }
 
 // Ring units of output columns [c_lo, c_hi), from the strip's bounds of
-// (ring column - strip column).
+// (ring column - strip column); at least one, whatever the bounds are (those of
+// positions that spread over 2^31 samples overflow), so that the tile offsets of
+// a half's entries ascend from 0.
 template <bool kSplit>
 __device__ __forceinline__ void entry_units(const RsStrip<kSplit> &Q, int c_lo, int c_hi, int &ulo,
                                             int &uhi) {
   ulo = min(max(c_lo + Q.dlo, 0), RS_FW - 1) >> 1;
-  uhi = min(max(c_hi - 1 + Q.dhi + 13, 0), RS_FW - 1) >> 1;
+  uhi = max(min(max(c_hi - 1 + Q.dhi + 13, 0), RS_FW - 1) >> 1, ulo);
 }
 
 // [P4] A row's entries, to `out` (at most RS_MAXKEY): (line, bin | region << 12 |

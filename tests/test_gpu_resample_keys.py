@@ -107,6 +107,22 @@ def test_resample_keys(T, O, name, prec):
         assert np.array_equal(_run(T, kw, prec, rows=(r0, n)), gpu[r0:r0 + n]), (r0, n)
 
 
+@pytest.mark.parametrize("prec", ["split", "fp64"])
+def test_positions_spread_beyond_int(T, O, prec):
+    """Range positions from -2^31 + 48 to 2.1e9 across a strip, one column of them
+    inside the slave box, in rows of one and of several azimuth runs: the strip's
+    bounds and that column's ring position overflow, but no tile offset or ring
+    column follows them."""
+    kw = _inputs(T, 60, 96, az_tilt=0.001)
+    c = 48                                 # this column is at sample 40.3
+    slope = (40.3 + 2147483600.5) / c
+    kw["cpm_rg"][:] = [40.3 + (0.5 * 95 - c) * slope, 0, slope * 0.25 * 95, 0, 0, 0]
+    ref, _ = O.resample(**kw)
+    gpu = _run(T, kw, prec)
+    assert np.abs(ref[:, c]).max() > 100 and not np.delete(ref, c, 1).any()
+    assert rel_rms(gpu, ref) < TOL and np.all(gpu[np.abs(ref) == 0] == 0)
+
+
 def _time(jobs, reps=9):
     """Median time of each job (us), the jobs in turn."""
     import torch
