@@ -117,7 +117,10 @@ static_assert(RS_DT <= RS_NT && RS_CH <= 2 * RS_NT && RS_CH % (2 * RS_H) == 0 &&
 // same (300 x 6000, 0.34 keys per row: split chunks of 12 rows 83 us, keyed 85;
 // FP64, 4 runs per table, chunks of 9 rows 111 us, keyed 87), and beyond it the
 // chunks lose (310 x 25000, 1.3 keys per row: split 556 and 306, FP64 712 and
-// 308 us; the kernel before the run tables of a chunk took 337 and 341).
+// 308 us; the kernel before the run tables of a chunk took 337 and 341).  The
+// last rows of an item are cut where two chunks hold them: short items pay
+// one more prologue for it (300 x 300, 0.55 keys per row, items of 12 rows: 46
+// us, keyed 50).
 constexpr int kKeyedRows = 2 * RS_H;
 
 enum : int { REG_OUT = 0, REG_EDGE = 1, REG_IN = 2 };
@@ -1458,7 +1461,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
     __syncthreads();
     // ---- [P7] the halves; a chunk that does not end the item ends with a
     // pair of halves, so that the window carries over
-    int n = Q.cov >= kKeyedRows ? min(nfit, Q.cov) : nfit;
+    int n = Q.cov >= min(kKeyedRows, (nr - ch0 + 1) / 2) ? min(nfit, Q.cov) : nfit;
     if (n < nr - ch0 && n >= 2 * RS_H) n -= n % (2 * RS_H);
     const int nh = (n + RS_H - 1) / RS_H;
     if (dval) {
