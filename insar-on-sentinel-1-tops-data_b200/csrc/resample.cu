@@ -979,6 +979,7 @@ __device__ __forceinline__ void walk_row(const RsShared<kSplit> &S, const Resamp
   const double L = row_L(J, r);
   const double A = row_a(S.caz, L) + S.shift, B = row_b(S.caz, L), C = S.caz[5];
   const double pa = col_P(J, c0), pb = col_P(J, c0 + cN - 1);
+  int base;                              // the row's lowest line inside the box
   {
     // the whole strip in one run?
     double ylo, yhi;
@@ -992,16 +993,22 @@ __device__ __forceinline__ void walk_row(const RsShared<kSplit> &S, const Resamp
       emit(g0, l0, b0, 0, cN);
       return;
     }
+    base = max(l0, J.sy0);
+    if ((long)min(l1, J.sy1) - base >= 1 << 18) {   // more than a key holds: a per-pixel row
+      while (emit(REG_OUT, 0, 0, 0, cN)) {
+      }
+      return;
+    }
   }
   // key of column c, ascending with the position: before the box -1, edge
   // (line, 4095), interior (line, bin), past the box INT32_MAX; lines relative
-  // to the box
+  // to the row's lowest, since a box may have more than 2^19
   auto key = [&](int c) -> int {
     int l, b;
     split_pos(pix_pos(A, B, C, col_P(J, c0 + c)), l, b);
     const int g = region_1d(l, J.sy0, J.sy1);
     if (g == REG_OUT) return l < J.sy0 ? -1 : INT32_MAX;
-    return (l - J.sy0) * 4096 + (g == REG_EDGE ? 4095 : b);
+    return (l - base) * 4096 + (g == REG_EDGE ? 4095 : b);
   };
   // monotone pieces: split at the vertex
   const double s0 = fma(2.0 * C, pa, B), s1 = fma(2.0 * C, pb, B);
@@ -1016,7 +1023,7 @@ __device__ __forceinline__ void walk_row(const RsShared<kSplit> &S, const Resamp
   auto put = [&](int k, int i0, int i1) -> bool {   // run [i0, i1) of key k
     const int c_lo = rev ? cN - i1 : i0, c_hi = rev ? cN - i0 : i1;
     if (k == -1 || k == INT32_MAX) return emit(REG_OUT, 0, 0, c_lo, c_hi);
-    return emit((k & 4095) == 4095 ? REG_EDGE : REG_IN, J.sy0 + (k >> 12), k & 4095, c_lo, c_hi);
+    return emit((k & 4095) == 4095 ? REG_EDGE : REG_IN, base + (k >> 12), k & 4095, c_lo, c_hi);
   };
   const int split = rev ? cN - 2 - vert : vert;   // last index of the first piece
   int i = 0;

@@ -29,7 +29,8 @@ class _Job:
         self.T, self.prec, self.rows = T, T.PREC_SPLIT if prec == "split" else T.PREC_FP64, rows
         self.slave = torch.zeros(L, W + pad, 2, dtype=torch.int16, device="cuda")
         self.slave[:, :W] = torch.from_numpy(kw["slave"]).cuda()
-        self.out = torch.full((L, W, 2), 7.0, device="cuda")
+        box = [int(v) for v in kw["mbox"]]
+        self.out = torch.full((box[3] - box[2] + 1, W, 2), 7.0, device="cuda")
         self.par = [torch.from_numpy(np.ascontiguousarray(kw[k])).cuda() for k in ("kt", "tref", "fdc")]
         self.lut = C.c_void_p()
         T.check(T.lib.tops_lut_create(T.ptr(kw["kaz"], C.c_float), T.ptr(kw["krg"], C.c_float),
@@ -121,6 +122,30 @@ def test_positions_spread_beyond_int(T, O, prec):
     gpu = _run(T, kw, prec)
     assert np.abs(ref[:, c]).max() > 100 and not np.delete(ref, c, 1).any()
     assert rel_rms(gpu, ref) < TOL and np.all(gpu[np.abs(ref) == 0] == 0)
+
+
+@pytest.mark.parametrize("prec", ["split", "fp64"])
+def test_box_of_more_than_2_19_lines(T, O, prec):
+    """The last lines of a slave box of 2^19 + 600 lines, in rows of four or five
+    azimuth runs from its interior over its edge to the outside.  The burst's
+    time starts near them and its ramp is the same in all columns: FP32 phases
+    do not hold a ramp of 9 minutes."""
+    kw = _inputs(T, 60, 20)
+    n, W = 2 ** 19 + 600, 20
+    rng = np.random.default_rng(7)
+    slave = np.zeros((n, W, 2), np.int16)
+    slave[-200:] = rng.normal(0, 700, (200, W, 2)).round()
+    m0 = n - 55                            # the last 9 rows lie outside
+    kw.update(slave=slave, mbox=np.array([0, W - 1, m0, m0 + 59], np.int32),
+              sbox=np.array([0, W - 1, 0, n - 1], np.int32), s_burst_idx=1, lines_per_burst=n - 200)
+    for k in ("kt", "tref", "fdc"):
+        kw[k] = np.full(W, kw[k][0])
+    kw["cpm_az"][:] = [m0 + 29.5 + 0.3, 0.25 * 59, 0.0005, 0.0, 0.0, 0.0]
+    ref, cnt = O.resample(**kw)
+    gpu = _run(T, kw, prec)
+    assert cnt[2] > 0 and cnt[1] > 0 and not ref[-4:].any()
+    assert rel_rms(gpu, ref) < TOL, rel_rms(gpu, ref)
+    assert np.all(gpu[np.abs(ref) == 0] == 0)
 
 
 def _time(jobs, reps=9):
