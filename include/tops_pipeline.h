@@ -42,8 +42,9 @@ typedef struct {
                                or TOPS_PREC_FP64 */
   int compensated;          /* 1: ESD phasor sums with Kahan compensation and
                                coherence with its reciprocal square roots
-                               refined (its window sums are trees in both
-                               modes); 0 (default): plain fixed-order FP32 */
+                               refined (its window sums are the same in both
+                               modes: trees for heights of up to 6 rows); 0
+                               (default): plain fixed-order FP32 */
   int coh_overlap;          /* 1: the ReSlaveESD resample in up to 3 chunks of
                                bursts, the coherence of each chunk on a second
                                stream as soon as it is resampled, overlapping

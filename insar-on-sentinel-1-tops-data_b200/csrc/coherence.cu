@@ -17,16 +17,20 @@
 // row is read once; output rows go in pairs whose common rows are summed once.
 // The horizontal sums come from prefix, suffix and whole sums of the lanes' four
 // columns that the lanes exchange with shuffles.  No sum is updated by
-// subtraction, so the rounding error does not grow along a row or with the
-// window (7.8e-8 relative RMS at 10 x 3, 8.0e-8 at 24 x 6).
+// subtraction, so the rounding error does not grow along a row, and a sample
+// that is not finite spoils its own windows only.  For heights of up to 6 the
+// sums are trees, whose error hardly grows with the window (7.8e-8 relative RMS
+// at 10 x 3, 8.0e-8 at 24 x 6); taller windows add the rows that 4 output rows
+// share one after another, an error of up to win_az roundings.
 //
 // What bounds it: instruction issue (10 x 3: 64 per output pixel, 11 of them
 // packed adds and 9 shuffles; two thirds of the issue slots) and the L1 data pipe
 // (the shuffles) at 16 warps per SM by registers, then the 16 bytes per pixel of
 // memory traffic.  Measured, in us, against a kernel that staged the products of
 // a block in shared memory and summed windows by sliding updates behind block
-// barriers:
-//   1500 x 21000, 10 x 3   154 -> 97 (5.2 TB/s)      24 x 6   243 -> 156
+// barriers (a single burst with a cold L2 takes a few more than these, which
+// found part of it there: 10 x 3 104 to 108, 4.7 to 4.8 TB/s):
+//   1500 x 21000, 10 x 3   154 -> 97                 24 x 6   243 -> 156
 //   1523 x 8193, 5 x 5     147 -> 48                 1200 x 7000, 30 x 9  180 -> 133
 //   1200 x 7000, 17 x 2    129 -> 47                 300 x 512, 10 x 3    66 -> 9
 //   800 x 9000, 2 x 1      111 -> 24                 33 x 7               152 -> 78
@@ -653,9 +657,11 @@ static int launch_t(const CohJob *jobs, int njobs, int win_rg, int win_az, const
 }
 
 // Compiled windows: 10 and the reference driver's 24 samples
-// (Func.cpp:2583-2584), with 3 and 6 rows, and every height up to 6 rows with
-// range windows of up to 6 samples (one compiled case each) and of 7 or more
-// (5 x 5 took 133 us with the lane sums picked at run time, 49 this way).
+// (Func.cpp:2583-2584), with 3 and 6 rows (1500 x 21000, us, as any window of 7
+// or more and so: 10 x 3 125 and 104, 10 x 6 209 and 144, 24 x 3 143 and 119,
+// 24 x 6 238 and 162), and every height up to 6 rows with range windows of up to
+// 6 samples (one compiled case each) and of 7 or more (5 x 5 took 133 us with
+// the lane sums picked at run time, 49 this way).
 // Taller windows sum the rows that 4 output rows share once.
 int launch_coherence(const CohJob *jobs, int njobs, int win_rg, int win_az, const TileCfg &cfg,
                      cudaStream_t st) {
