@@ -114,10 +114,10 @@ static_assert(RS_DT <= RS_NT && RS_CH <= 2 * RS_NT && RS_CH % (2 * RS_H) == 0 &&
 // A chunk whose run tables end before this many rows is not cut there: columns
 // with a full table are keyed behind it.  A shorter chunk prepares and refills
 // for each tile what it needs only once per 96 rows; at the line both cost the
-// same (300 x 6000, 0.34 keys per row: split chunks of 12 rows 83 us, keyed 85;
+// same (300 x 6000, 0.34 keys per row: split chunks of 12 rows 83 us, keyed 86;
 // FP64, 4 runs per table, chunks of 9 rows 111 us, keyed 87), and beyond it the
-// chunks lose (310 x 25000, 1.3 keys per row: split 556 and 306, FP64 712 and
-// 308 us; the kernel before the run tables of a chunk took 337 and 341).  The
+// chunks lose (310 x 25000, 0.55 keys per row: split 417 and 304, FP64 519 and
+// 304 us; the kernel before the run tables of a chunk took 333 and 341).  The
 // last rows of an item are cut where two chunks hold them: short items pay
 // one more prologue for it (300 x 300, 0.55 keys per row, items of 12 rows: 46
 // us, keyed 50).
@@ -126,9 +126,10 @@ constexpr int kKeyedRows = 2 * RS_H;
 enum : int { REG_OUT = 0, REG_EDGE = 1, REG_IN = 2 };
 // A half: has interior entries; fills its window anew; has entries off its
 // window; shares its tile with the next half; has per-pixel rows; every row is
-// one interior entry; and, besides, 6 rows with the window's lines and one bin.
+// one interior entry; and, besides, 6 rows with the window's lines and one bin;
+// has keyed rows.
 enum : int { HG_ON = 1, HG_FILL = 2, HG_DIRECT = 4, HG_JOIN = 8, HG_PIX = 16, HG_ONE = 32,
-             HG_PLAIN = 64 };
+             HG_PLAIN = 64, HG_KEY = 128 };
 constexpr int E_DIRECT = 4;                // entry flag beside its region
 
 using RsLut = LutPtrs;
@@ -404,9 +405,10 @@ __device__ __forceinline__ float2 pixel_generic(const RsShared<kSplit> &S, const
 // The per-pixel rows and the listed pixels of nrows tile rows (chunk rows from
 // cr0, box rows from r0 on), all threads; the rows end to end, so that no lane
 // idles at the end of each (1000 x 6000, all rows of more than 12 azimuth runs:
-// 4670 -> 4270 us).
+// 4670 -> 4270 us).  Out of line: rare, and the other chunks run faster with less
+// text (a 9-burst pair 6.92 -> 6.77 ms).
 template <bool kSplit>
-__device__ __forceinline__ void pixel_pass(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
+__device__ __noinline__ void pixel_pass(const RsShared<kSplit> &S, const RsStrip<kSplit> &Q,
                                            const ResampleJob &J, int u, int cr0, int r0, int nrows,
                                            int c0, int cN) {
   int k = 0;
@@ -887,7 +889,7 @@ __device__ __forceinline__ void keyed_pair(RsStrip<kSplit> &Q, const ResampleJob
 // each pixel's key found anew, all threads.  From row ks on the entries' tile
 // starts at tb1.
 template <bool kSplit>
-__device__ __noinline__ void keyed_pairs(const ResampleJob &J, int rb, int k0, int ka, int k1,
+__device__ __forceinline__ void keyed_pairs(const ResampleJob &J, int rb, int k0, int ka, int k1,
                                          int ks, int tb1, int c0, int cN) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RsShared<kSplit> &S = *reinterpret_cast<RsShared<kSplit> *>(smem_raw);
@@ -1499,6 +1501,7 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
       const int expect = u == 0 ? Q.prev_line
                          : (Q.half[u - 1].flags & HG_ON) ? Q.half[u - 1].lb + RS_H : INT32_MIN;
       if ((fl & HG_ON) && H.lb != expect) fl |= HG_FILL;
+      if (min((u + 1) * RS_H, n) > Q.kfrom) fl |= HG_KEY;
       const int h0 = u & ~1;
       if (h0 + 1 < nh && Q.half[h0].units + Q.half[h0 + 1].units <= RS_TU) {
         if (u & 1)
@@ -1613,11 +1616,13 @@ __device__ __forceinline__ void resample_item(RsShared<kSplit> &S, const RsBatch
                     J.out + (long)(rb + k0 - J.row0) * J.out_pitch + c0);
         __syncthreads();
       }
-      if (k1 > Q.kfrom) {
-        keyed_pairs<kSplit>(J, rb, k0, max(k0, Q.kfrom), k1, h * RS_H, H.tbase, c0, cN);
-        __syncthreads();
+      if (Q.gen_any || (any & (HG_PIX | HG_KEY))) {
+        if (any & HG_KEY) {
+          keyed_pairs<kSplit>(J, rb, k0, max(k0, Q.kfrom), k1, h * RS_H, H.tbase, c0, cN);
+          __syncthreads();
+        }
+        if (Q.gen_any || (any & HG_PIX)) pixel_pass(S, Q, J, u, k0, rb + k0, k1 - k0, c0, cN);
       }
-      if (Q.gen_any || (any & HG_PIX)) pixel_pass(S, Q, J, u, k0, rb + k0, k1 - k0, c0, cN);
       if (Q.gen_any) {
         __syncthreads();
         if (u < 2 * RS_H * 4) (&Q.gen[0][0])[u] = 0u;
