@@ -181,7 +181,8 @@ int tops_run_config(const char *config_path, tops_run_stats *stats);
 typedef struct tops_batch tops_batch;
 
 /* Tile and scheduling of the resample and coherence launches.  The rows of a
- * work item are chosen by the number of items, up to the limits here. */
+ * work item are chosen by the number of items, up to the limits here; a launch
+ * of 8 items and more per resident CTA takes a given limit as it is. */
 typedef struct {
   int rs_seg_rows;      /* most resample output rows per work item, 12..252
                            (0: 252) */

@@ -596,7 +596,8 @@ static int launch_al(const CohJob *jobs, int njobs, int win_rg, int win_az, cons
   const int tw = CO_NW * CO_CPL * (32 - nl - nr);   // output columns of a CTA
   // segment rows: the fewest row times of the last CTA to finish, waves x (rows
   // + the window's halo and the first loads, worth about 8 rows), up to the
-  // caller's limit; whole groups, so that a row's sums do not depend on the cut
+  // caller's limit, which 8 waves and more take as it is; whole groups, so that
+  // a row's sums do not depend on the cut
   const int most = cfg.seg_rows ? (cfg.seg_rows + 3) & ~3 : 256;
   int seg_rows = 0;
   {
@@ -612,6 +613,7 @@ static int launch_al(const CohJob *jobs, int njobs, int win_rg, int win_az, cons
         best = cost;
         seg_rows = sr;
       }
+      if (cfg.seg_rows && sr == most && items >= 8L * resident) break;
     }
   }
   for (int j0 = 0, k = 0; j0 < njobs; j0 += CO_MAXJOBS, k++) {

@@ -6,7 +6,8 @@
 //             12..252 (0: 252), the coherence kernel 8..512, rounded up to a
 //             multiple of 4 (0: 256).  Of a few lengths up to that, a launch
 //             takes the one whose last CTA ends first by the count of items
-//             per CTA: a long item alone on an SM leaves the others idle
+//             per CTA: a long item alone on an SM leaves the others idle.  With
+//             8 items and more per resident CTA a given length is taken as it is
 //   counters  if non-null: persistent launch.  `grid` CTAs (0: as many as
 //             fit on the device at once) pull work items from a queue -- the
 //             device int counters[k], set to 0 on the stream before the k-th

@@ -1807,7 +1807,9 @@ static int launch_resample_t(const ResampleJob *jobs, int njobs, const TileCfg &
     return TOPS_E_INVALID;
   // segment rows: the fewest row times of the last CTA to finish, waves x (rows
   // + the prologue and the window's fill, worth about 24 rows), up to the
-  // caller's limit.  Outputs do not depend on it.
+  // caller's limit; 8 waves and more at the limit take it as it is, since their
+  // CTAs are out of step (27 bursts of three sub-swaths: limit 252 8.47 ms,
+  // the choice up to it 8.83).  Outputs do not depend on it.
   const int most = cfg.seg_rows ? cfg.seg_rows : RS_MAXSEG;
   int seg_rows = 0;
   {
@@ -1823,6 +1825,7 @@ static int launch_resample_t(const ResampleJob *jobs, int njobs, const TileCfg &
         best = cost;
         seg_rows = sr;
       }
+      if (cfg.seg_rows && sr == most && items >= 8L * resident) break;
     }
   }
   for (int j0 = 0, k = 0; j0 < njobs; j0 += RS_MAXJOBS, k++) {
