@@ -56,13 +56,14 @@
 // What bounds it: the latency of each warp's instruction stream (about 7 cycles
 // per instruction) with 12 warps per SM: the window, the taps of two columns and
 // a row's samples need 168 registers.  Two columns per thread share a line's
-// terms, a row's taps and the bookkeeping, and fill the FP32x2 lanes: 105
-// instead of 158 thread instructions per pixel.  A burst of 1500 x 21000 (one
-// entry per row) 0.463 -> 0.300 ms (816 -> 1260 GB/s of 12 bytes per pixel); a
-// burst of 300 x 512 70 -> 23 us (short segments: a row costs a lone CTA 0.7
-// us).  Rows whose strip spans several azimuth keys took a per-pixel path from
-// HBM before, columns with many range keys a keyed one: a burst of 1539 x 10867
-// of crossing orbits 3.92 -> 0.62 ms.
+// terms, a row's taps and the bookkeeping, and fill the FP32x2 lanes: 110
+// thread instructions per pixel, the uniform ones included, where one column
+// per thread took 158.  A burst of 1500 x 21000 (one entry per row) 0.462 ->
+// 0.292 ms (818 -> 1295 GB/s of 12 bytes per pixel); a burst of 300 x 512 70 ->
+// 23 us (short segments: a row costs a lone CTA 0.7 us).  Rows whose strip
+// spans several azimuth keys took a per-pixel path from HBM before, columns
+// with many range keys a keyed one: a burst of 1539 x 10867 of crossing orbits
+// 3.89 -> 0.58 ms.
 //
 // Which path a pixel takes, and the order of its sums, depend on its row, its
 // column and its strip only, never on the work item, so a job that produces a
